@@ -150,6 +150,10 @@ struct m2_ctx {
     uint2* d_aux = nullptr;    // per-element unweighting rotations and digit widths (m2k::LargeBufs::aux)
     bool fused = false;        // inverse and next forward column pass as one cooperative launch
     bool gf61 = false;         // GF(P61^2)-only transform (M2_FIELDS_GF61)
+    bool flow = false;         // squarings run in the one-launch kernel (m2_flow.cu)
+    bool flow_dirty = false;   // a three-pass stage ran since: element tags to be set again
+    m2k::FlowArgs fargs{};
+    char* d_flow = nullptr;    // its tagged carries, then its parity words
     // GRAPH_ITERS[i] iterations of the three-pass path captured once and replayed
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     bool graph_failed = false;
@@ -211,14 +215,38 @@ bool ensure_graph(m2_ctx* c, int i) {
     return false;
 }
 
+// Squarings per launch of the one-launch kernel: long enough that a launch's
+// start is nothing (20 ms at n = 2^18), short enough that other contexts'
+// launches get their turn.
+constexpr uint32_t FLOW_ITERS = 1000;
+
+// the one-launch kernel's tags as every launch expects them: all element tags
+// 1, carries of parity 0
+cudaError_t flow_reset(m2_ctx* c) {
+    cudaError_t e = cudaMemsetAsync(c->d_za, 0xff, sizeof(ulonglong2) * c->L.h, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_zb, 0xff, sizeof(uint2) * c->L.h, c->stream);
+    const int lh = c->L.ln - 1;
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flow, 0, 8 * m2k::flow_carry_words(lh) + 4 * m2k::flow_groups(lh), c->stream);
+    if (e == cudaSuccess) c->flow_dirty = false;
+    return e;
+}
+
+// what a new state needs beside its digits: no pending carries, epoch flags
+// and tags as at creation
+cudaError_t reset_sync_words(m2_ctx* c) {
+    cudaError_t e = cudaSuccess;
+    if (c->path == M2_PATH_LARGE) e = cudaMemsetAsync(c->d_carries, 0, sizeof(i64) * (size_t)c->plan.R * c->plan.G, c->stream);
+    if (e == cudaSuccess && c->d_flags) e = cudaMemsetAsync(c->d_flags, 0, flags_bytes(c->plan), c->stream);
+    if (e == cudaSuccess && c->flow) e = flow_reset(c);
+    return e;
+}
+
 int cuda_err(cudaError_t e) { return e == cudaSuccess ? M2_OK : (e == cudaErrorMemoryAllocation ? M2_ENOMEM : M2_ECUDA); }
 
 int upload_state(m2_ctx* c, const std::vector<u64>& canon) {
     std::vector<i64> bal = m2::balanced_digits(c->L, canon);
     cudaError_t e = cudaMemcpyAsync(c->d_digits, bal.data(), bal.size() * sizeof(i64), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess && c->path == M2_PATH_LARGE)
-        e = cudaMemsetAsync(c->d_carries, 0, sizeof(i64) * (size_t)c->plan.R * c->plan.G, c->stream);
-    if (e == cudaSuccess && c->d_flags) e = cudaMemsetAsync(c->d_flags, 0, flags_bytes(c->plan), c->stream);
+    if (e == cudaSuccess) e = reset_sync_words(c);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     return cuda_err(e);
 }
@@ -315,9 +343,7 @@ int canon_buffer(m2_ctx* c, unsigned long long** buf) {
 int load_canon(m2_ctx* c, uint32_t iteration) {
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     cudaError_t e = m2k::launch_balance(c->d_canon, c->d_digits, c->L.p, c->L.ln, c->L.n, nullptr, c->stream);
-    if (e == cudaSuccess && c->path == M2_PATH_LARGE)
-        e = cudaMemsetAsync(c->d_carries, 0, sizeof(i64) * (size_t)c->plan.R * c->plan.G, c->stream);
-    if (e == cudaSuccess && c->d_flags) e = cudaMemsetAsync(c->d_flags, 0, flags_bytes(c->plan), c->stream);
+    if (e == cudaSuccess) e = reset_sync_words(c);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
     if (e != cudaSuccess) return fail_cuda("state load", e);
     c->iteration = iteration;
@@ -437,22 +463,15 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         }
         raw->bufs = m2k::LargeBufs{raw->d_digits, raw->d_carries, raw->d_za, raw->d_zb, raw->d_w61, raw->d_w31,
                                    raw->tw.tw4, raw->tw.tc, raw->d_status, raw->d_flags};
-        if (m2k::cols_q_supported(P)) {
-            // the inverse column passes' per-element table: the rotation by
-            // 2^-(s + ln + 1) that unweights a digit of shift s (mod 61 and mod
-            // 31) and the digit widths
-            std::vector<uint2> aux(h);
-            const uint32_t ln1 = (uint32_t)raw->L.ln + 1;
-            auto un = [ln1](uint32_t s, uint32_t m) { const uint32_t t = (s + ln1) % m; return t ? m - t : 0u; };
-            for (u64 k = 0; k < h; ++k) {
-                const u64 j = 2 * k;
-                aux[k].x = un(raw->L.w61[j], 61) | (un(raw->L.w61[j + 1], 61) << 8) | (un(raw->L.w31[j], 31) << 16) |
-                           (un(raw->L.w31[j + 1], 31) << 24);
-                aux[k].y = (uint32_t)raw->L.width[j] | ((uint32_t)raw->L.width[j + 1] << 8);
-            }
+        const int lh = raw->L.ln - 1;
+        // one launch for all squarings of a call where a shape of that kernel
+        // serves the size; M2_PATH_LARGE and a -B hint ask for the three-pass kernels
+        raw->flow = o.path == M2_PATH_AUTO && o.carry_pairs == 0 && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 && m2k::flow_setup(lh, gf61) == cudaSuccess;
+        cudaGetLastError();
+        if (m2k::cols_q_supported(P) || raw->flow) {
+            // the inverse column passes' per-element table, built on the device
             if ((rc = dalloc(raw, &raw->d_aux, sizeof(uint2) * h))) { m2_destroy(c.release()); return rc; }
-            if (cudaMemcpyAsync(raw->d_aux, aux.data(), sizeof(uint2) * h, cudaMemcpyHostToDevice, raw->stream) != cudaSuccess ||
-                cudaStreamSynchronize(raw->stream) != cudaSuccess) {
+            if (m2k::launch_aux(raw->d_aux, raw->d_w61, raw->d_w31, p, raw->L.ln, raw->stream) != cudaSuccess) {
                 m2_destroy(c.release());
                 return M2_ECUDA;
             }
@@ -463,6 +482,13 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         raw->plan.mid_tickets = (raw->fused && !m2k::cols_mid_cooperative(P)) ? 1u : 0u;
         // the phase barrier measured faster with R = 1024 rows only (n = 2^21)
         raw->plan.mid_barrier = (raw->fused && !P.mid_tickets && P.R == 1024u) ? 1u : 0u;
+        if (raw->flow) {
+            const size_t cw = m2k::flow_carry_words(lh);
+            if ((rc = dalloc(raw, &raw->d_flow, 8 * cw + 4 * m2k::flow_groups(lh)))) { m2_destroy(c.release()); return rc; }
+            raw->fargs = m2k::FlowArgs{raw->d_digits, raw->d_carries, raw->d_za, raw->d_zb, raw->d_w61, raw->d_w31, raw->d_aux,
+                                       raw->tw.tw4, raw->tw.tc, reinterpret_cast<unsigned long long*>(raw->d_flow),
+                                       reinterpret_cast<unsigned*>(raw->d_flow + 8 * cw), raw->d_status, 0u, 2u * P.C, raw->span, mode};
+        }
         raw->bufs.ticket = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G);
         raw->bufs.phase = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G + 2);
     }
@@ -479,6 +505,12 @@ int m2_iterate(m2_ctx* c, uint32_t k) {
     cudaError_t e = cudaSuccess;
     if (c->path == M2_PATH_SMALL) {
         e = m2k::launch_small(c->d_test, 1, (unsigned)c->L.h, c->threads, k, c->stream, c->h_test.fuse_middle != 0, c->gf61);
+    } else if (c->flow) {
+        if (c->flow_dirty) e = flow_reset(c);
+        for (uint32_t left = k; left > 0 && e == cudaSuccess; left -= c->fargs.k) {
+            c->fargs.k = std::min(left, FLOW_ITERS);
+            e = m2k::launch_flow(c->L.ln - 1, c->gf61, c->fargs, c->stream);
+        }
     } else {
         uint32_t left = k;
         for (int i = 0; i < 2; ++i)
@@ -525,9 +557,7 @@ int m2_set_digits(m2_ctx* c, const uint64_t* digits, uint32_t iteration) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_canon, digits, c->L.n * sizeof(u64), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = m2k::launch_balance(c->d_canon, c->d_digits, c->L.p, c->L.ln, c->L.n, d_bad, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, d_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && c->path == M2_PATH_LARGE)
-        e = cudaMemsetAsync(c->d_carries, 0, sizeof(i64) * (size_t)c->plan.R * c->plan.G, c->stream);
-    if (e == cudaSuccess && c->d_flags) e = cudaMemsetAsync(c->d_flags, 0, flags_bytes(c->plan), c->stream);
+    if (e == cudaSuccess) e = reset_sync_words(c);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return fail_cuda("state upload", e);
@@ -611,8 +641,15 @@ int m2_carry_normalize(uint32_t p, const int64_t* digits, const int64_t* seg_car
 
 int m2_test_stall_fused(m2_ctx* c) {
     if (!c) return M2_EINVAL;
-    if (!c->fused || !c->d_flags) return M2_EUNSUPPORTED;
+    if (!c->flow && (!c->fused || !c->d_flags)) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
+    if (c->flow) {
+        // column group 0 expects a tag that no carry word has
+        const unsigned never = 2u;
+        cudaError_t e = cudaMemcpyAsync(c->fargs.parity, &never, sizeof(never), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        return e == cudaSuccess ? M2_OK : fail_cuda("m2_test_stall_fused", e);
+    }
     unsigned f0 = 0;
     cudaError_t e = cudaMemcpyAsync(&f0, c->d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -626,6 +663,7 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
     if (!c || stage < 0 || stage > 2) return M2_EINVAL;
     if (c->path != M2_PATH_LARGE) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
+    c->flow_dirty = c->flow;
     cudaError_t e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
     const size_t h = c->L.h;
     if (e == cudaSuccess && za_out) e = cudaMemcpyAsync(za_out, c->d_za, 16 * h, cudaMemcpyDeviceToHost, c->stream);
@@ -658,7 +696,7 @@ void m2_destroy(m2_ctx* c) {
     // stream-ordered frees: they follow the context's queued work and do not
     // wait for other streams; its stream is released once that work is done
     void* bufs[] = {c->d_w61, c->d_w31, c->d_status, c->d_digits, c->d_test, c->d_carries, c->d_za, c->d_zb,
-                    c->d_canon, c->d_norm, c->d_flags, c->d_aux};
+                    c->d_canon, c->d_norm, c->d_flags, c->d_aux, c->d_flow};
     if (c->stream)
         for (void* b : bufs) if (b) cudaFreeAsync(b, c->stream);
     for (cudaGraphExec_t g : c->graph)
@@ -680,6 +718,7 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
     } else {
         for (uint32_t i = 0; i < iters; ++i) for (int st = 0; st < m2k::LARGE_STAGES; ++st) seq.push_back(st);
     }
+    c->flow_dirty = c->flow;
     std::vector<cudaEvent_t> ev(seq.size() + 1);
     for (auto& e : ev) if (cudaEventCreate(&e) != cudaSuccess) return M2_ECUDA;
     cudaError_t err = cudaEventRecord(ev[0], c->stream);
@@ -724,6 +763,7 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
 uint64_t m2_launches_for(m2_ctx* c, uint32_t k) {
     if (!c || k == 0) return 0;
     if (c->path == M2_PATH_SMALL) return 1ull;
+    if (c->flow) return ((uint64_t)k + FLOW_ITERS - 1) / FLOW_ITERS;
     if (!c->fused) return (uint64_t)m2k::LARGE_STAGES * k;
     // graph replays of GRAPH_ITERS[0] then GRAPH_ITERS[1] squarings, then the
     // rest in one sequence

@@ -61,6 +61,26 @@ struct LargeBufs {
     const uint2* aux;
 };
 
+// Arguments of the one-launch kernel of mid-size transforms (m2_flow.cu).
+struct FlowArgs {
+    long long* digits;         // n digits of the state; left with no pending carries
+    long long* carries;        // pending segment carries of the three-pass kernels, applied and cleared
+    ulonglong2* za;            // h tagged GF(P61^2) elements, every tag 1 between launches
+    uint2* zb;                 // h tagged GF(P31^2) elements
+    const unsigned char* w61;
+    const unsigned char* w31;
+    const uint2* aux;          // per element: LargeBufs::aux
+    const DTw* tw4;
+    const DTw* tc;
+    unsigned long long* fcar;  // flow_carry_words tagged segment carries
+    unsigned int* parity;      // flow_groups words: squarings done, modulo 2
+    int* status;
+    unsigned int k;            // squarings of this launch (>= 1)
+    unsigned int seg;          // digits per pending carry segment
+    int span;                  // at most 3
+    int mode;
+};
+
 constexpr int LARGE_STAGES = 3;
 constexpr int STAGE_MID = 3;   // the fused inverse + forward column pass (k_cols_mid_q)
 
