@@ -140,6 +140,7 @@ struct m2_ctx {
     m2k::SmallTest h_test{};   // host copy of the descriptor (the serving engine batches these)
     int threads = 0;
     int carry_threads = 0;
+    bool lane = false;         // squarings run in the one-element-per-thread kernel (m2_lane.cu)
     // large path
     m2k::LargePlan plan{};
     m2k::LargeBufs bufs{};
@@ -213,6 +214,12 @@ bool ensure_graph(m2_ctx* c, int i) {
     c->graph[i] = nullptr;
     c->graph_failed = true;
     return false;
+}
+
+// k squarings of a one-CTA context
+cudaError_t launch_one_cta(m2_ctx* c, uint32_t k) {
+    if (c->lane) return m2k::launch_lane(c->d_test, 1, (unsigned)c->L.h, k, c->stream, c->gf61);
+    return m2k::launch_small(c->d_test, 1, (unsigned)c->L.h, c->threads, k, c->stream, c->h_test.fuse_middle != 0, c->gf61);
 }
 
 // Squarings per launch of the one-launch kernel: long enough that a launch's
@@ -447,6 +454,11 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         t.fuse_middle = o.fused_middle ? 1 : 0;
         t.gf61_only = gf61 ? 1 : 0;
         raw->h_test = t;
+        // a lone small test: one element per thread (M2_PATH_SMALL and the
+        // hints speak of the one-CTA kernel, which the shared launches of
+        // batches and the server run too)
+        raw->lane = o.path == M2_PATH_AUTO && !o.wg && !o.carry_pairs && !o.fused_middle &&
+                    m2k::lane_supported((unsigned)h, raw->span, raw->carry_threads);
         if (cudaMemcpyAsync(raw->d_test, &raw->h_test, sizeof(t), cudaMemcpyHostToDevice, raw->stream) != cudaSuccess) {
             m2_destroy(c.release());
             return M2_ECUDA;
@@ -504,7 +516,7 @@ int m2_iterate(m2_ctx* c, uint32_t k) {
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     cudaError_t e = cudaSuccess;
     if (c->path == M2_PATH_SMALL) {
-        e = m2k::launch_small(c->d_test, 1, (unsigned)c->L.h, c->threads, k, c->stream, c->h_test.fuse_middle != 0, c->gf61);
+        e = launch_one_cta(c, k);
     } else if (c->flow) {
         if (c->flow_dirty) e = flow_reset(c);
         for (uint32_t left = k; left > 0 && e == cudaSuccess; left -= c->fargs.k) {
@@ -724,7 +736,7 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
     cudaError_t err = cudaEventRecord(ev[0], c->stream);
     for (size_t i = 0; i < seq.size() && err == cudaSuccess; ++i) {
         if (seq[i] < 0)
-            err = m2k::launch_small(c->d_test, 1, (unsigned)c->L.h, c->threads, iters, c->stream, c->h_test.fuse_middle != 0, c->gf61);
+            err = launch_one_cta(c, iters);
         else err = m2k::launch_large_stage(c->plan, c->bufs, seq[i], c->stream);
         if (err == cudaSuccess) err = cudaEventRecord(ev[i + 1], c->stream);
     }

@@ -30,103 +30,11 @@
 // 2^13 18.5 -> 6.7, 2^14 19.5 -> 7.7, 2^15 21.7 -> 8.8, 2^16 27.5 -> 9.6,
 // 2^17 31.9 -> 10.0, 2^18 37.3 -> 16.3.  The three passes paid three launches
 // per squaring, each with cold L1 tables, and ran rows on as few as 32 SMs.
-#include "m2_field.cuh"
-#include "m2_kernels.cuh"
-
-using namespace M2D_NS;
+#include "m2_split.cuh"
 
 namespace M2K_NS {
 
 namespace {
-
-// ---------------- one field at a time ----------------
-struct __align__(16) X61 { u64 a, b; };
-struct __align__(8) X31 { u32 c, d; };
-
-__device__ __forceinline__ X61 xmul(const X61& x, const X61& w) { X61 r; cmul61(x.a, x.b, w.a, w.b, r.a, r.b); return r; }
-__device__ __forceinline__ X31 xmul(const X31& x, const X31& w) { X31 r; cmul31(x.c, x.d, w.c, w.d, r.c, r.d); return r; }
-__device__ __forceinline__ X61 xmulc(const X61& x, const X61& w) { X61 r; cmulconj61(x.a, x.b, w.a, w.b, r.a, r.b); return r; }
-__device__ __forceinline__ X31 xmulc(const X31& x, const X31& w) { X31 r; cmulconj31(x.c, x.d, w.c, w.d, r.c, r.d); return r; }
-__device__ __forceinline__ X61 xsqr(const X61& x) { X61 r; csqr61(x.a, x.b, r.a, r.b); return r; }
-__device__ __forceinline__ X31 xsqr(const X31& x) { X31 r; csqr31(x.c, x.d, r.c, r.d); return r; }
-__device__ __forceinline__ X61 xadd(const X61& x, const X61& y) { return X61{add61(x.a, y.a), add61(x.b, y.b)}; }
-__device__ __forceinline__ X31 xadd(const X31& x, const X31& y) { return X31{add31(x.c, y.c), add31(x.d, y.d)}; }
-__device__ __forceinline__ X61 xsub(const X61& x, const X61& y) { return X61{sub61(x.a, y.a), sub61(x.b, y.b)}; }
-__device__ __forceinline__ X31 xsub(const X31& x, const X31& y) { return X31{sub31(x.c, y.c), sub31(x.d, y.d)}; }
-__device__ __forceinline__ X61 xaddconj(const X61& x, const X61& y) { return X61{add61(x.a, y.a), sub61(x.b, y.b)}; }
-__device__ __forceinline__ X31 xaddconj(const X31& x, const X31& y) { return X31{add31(x.c, y.c), sub31(x.d, y.d)}; }
-__device__ __forceinline__ X61 xsubconj(const X61& x, const X61& y) { return X61{sub61(x.a, y.a), add61(x.b, y.b)}; }
-__device__ __forceinline__ X31 xsubconj(const X31& x, const X31& y) { return X31{sub31(x.c, y.c), add31(x.d, y.d)}; }
-__device__ __forceinline__ X61 xconjsub(const X61& x, const X61& y) { return X61{sub61(x.a, y.a), sub61(y.b, x.b)}; }
-__device__ __forceinline__ X31 xconjsub(const X31& x, const X31& y) { return X31{sub31(x.c, y.c), sub31(y.d, x.d)}; }
-__device__ __forceinline__ X61 xtimes_i(const X61& r) { return X61{P61 - r.b, r.a}; }
-__device__ __forceinline__ X31 xtimes_i(const X31& r) { return X31{P31 - r.d, r.c}; }
-__device__ __forceinline__ X61 xone(const X61&) { return X61{1, 0}; }
-__device__ __forceinline__ X31 xone(const X31&) { return X31{1, 0}; }
-
-// the add layers of dif4 / dit4 (m2_field.cuh) in one field
-__device__ __forceinline__ void dif_adds(X61 (&x)[4], const X61& u1, const X61& u2, const X61& u3) {
-    const L61 v0 = ladd(x[0].a, x[0].b, u2.a, u2.b), v1 = ladd(u1.a, u1.b, u3.a, u3.b);
-    const L61 v2 = lsub(x[0].a, x[0].b, u2.a, u2.b), v3 = lsub(u1.a, u1.b, u3.a, u3.b);
-    x[0] = X61{fadd(v0.a, v1.a), fadd(v0.b, v1.b)};
-    x[1] = X61{fsub(v0.a, v1.a), fsub(v0.b, v1.b)};
-    x[2] = X61{fsub(v2.a, v3.b), fadd(v2.b, v3.a)};   // v2 + i v3
-    x[3] = X61{fadd(v2.a, v3.b), fsub(v2.b, v3.a)};   // v2 - i v3
-}
-__device__ __forceinline__ void dif_adds(X31 (&x)[4], const X31& u1, const X31& u2, const X31& u3) {
-    const X31 v0 = xadd(x[0], u2), v1 = xadd(u1, u3), v2 = xsub(x[0], u2), v3 = xsub(u1, u3);
-    x[0] = xadd(v0, v1);
-    x[1] = xsub(v0, v1);
-    x[2] = X31{sub31(v2.c, v3.d), add31(v2.d, v3.c)};
-    x[3] = X31{add31(v2.c, v3.d), sub31(v2.d, v3.c)};
-}
-__device__ __forceinline__ void dit_adds(X61 (&x)[4]) {
-    const L61 v0 = ladd(x[0].a, x[0].b, x[1].a, x[1].b), v1 = lsub(x[0].a, x[0].b, x[1].a, x[1].b);
-    const L61 v2 = ladd(x[2].a, x[2].b, x[3].a, x[3].b), v3 = lsub(x[3].a, x[3].b, x[2].a, x[2].b);
-    x[0] = X61{fadd(v0.a, v2.a), fadd(v0.b, v2.b)};
-    x[2] = X61{fsub(v0.a, v2.a), fsub(v0.b, v2.b)};
-    x[1] = X61{fsub(v1.a, v3.b), fadd(v1.b, v3.a)};   // v1 + i v3
-    x[3] = X61{fadd(v1.a, v3.b), fsub(v1.b, v3.a)};   // v1 - i v3
-}
-__device__ __forceinline__ void dit_adds(X31 (&x)[4]) {
-    const X31 v0 = xadd(x[0], x[1]), v1 = xsub(x[0], x[1]), v2 = xadd(x[2], x[3]), v3 = xsub(x[3], x[2]);
-    x[0] = xadd(v0, v2);
-    x[2] = xsub(v0, v2);
-    x[1] = X31{sub31(v1.c, v3.d), add31(v1.d, v3.c)};
-    x[3] = X31{add31(v1.c, v3.d), sub31(v1.d, v3.c)};
-}
-template <class X> struct Tri { X r1, r2, r3; };
-template <class X> __device__ __forceinline__ void xdif4(X (&x)[4], const Tri<X>& t) {
-    dif_adds(x, xmul(x[1], t.r1), xmul(x[2], t.r2), xmul(x[3], t.r3));
-}
-template <class X> __device__ __forceinline__ void xdif4_1(X (&x)[4]) { const X a = x[1], b = x[2], c = x[3]; dif_adds(x, a, b, c); }
-template <class X> __device__ __forceinline__ void xdit4(X (&x)[4], const Tri<X>& t) {
-    dit_adds(x);
-    x[1] = xmulc(x[1], t.r1); x[2] = xmulc(x[2], t.r2); x[3] = xmulc(x[3], t.r3);
-}
-// centre_pair (m2_field.cuh) in one field
-template <class X> __device__ __forceinline__ void xcentre(X& zk, X& zm, const X& zeta) {
-    const X u0 = xaddconj(zk, zm), u1 = xsubconj(zk, zm);
-    const X v0 = xsub(xsqr(u0), xmul(xsqr(u1), zeta));
-    const X v1 = xmul(u0, xadd(u1, u1));
-    zk = xadd(v0, v1);
-    zm = xconjsub(v0, v1);
-}
-
-// twiddle of the table in one field
-__device__ __forceinline__ void ldtw(X61& w, const DTw* t, u32 i) {
-    const u64* q = reinterpret_cast<const u64*>(t + i);
-    w.a = __ldg(q); w.b = __ldg(q + 1);
-}
-__device__ __forceinline__ void ldtw(X31& w, const DTw* t, u32 i) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(t + i) + 2);
-    w.c = v.x; w.d = v.y;
-}
-template <class X> __device__ __forceinline__ Tri<X> ldtri(const DTw* tw4, u32 blk) {   // blk = S + J
-    Tri<X> t;
-    ldtw(t.r1, tw4, 3 * blk); ldtw(t.r2, tw4, 3 * blk + 1); ldtw(t.r3, tw4, 3 * blk + 2);
-    return t;
-}
 
 __device__ __forceinline__ X61 xshfl(const X61& v, int src) {
     return X61{__shfl_sync(0xffffffffu, v.a, src), __shfl_sync(0xffffffffu, v.b, src)};
@@ -436,9 +344,6 @@ template <class S, class X> struct Unit {
         for (int m = 0; m < 4; ++m) z[s0 ^ sw(m)] = x[m];
     }
 };
-
-__device__ __forceinline__ X61 weigh61(i64 d0, i64 d1, u32 s) { return X61{rotl61(digit_to61(d0), s & 0xffu), rotl61(digit_to61(d1), (s >> 8) & 0xffu)}; }
-__device__ __forceinline__ X31 weigh31(i64 d0, i64 d1, u32 s) { return X31{rotl31(digit_to31(d0), s & 0xffu), rotl31(digit_to31(d1), (s >> 8) & 0xffu)}; }
 
 template <class S>
 __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
