@@ -223,7 +223,7 @@ cudaError_t launch_one_cta(m2_ctx* c, uint32_t k) {
 }
 
 // Squarings per launch of the one-launch kernel: long enough that a launch's
-// start is nothing (20 ms at n = 2^18), short enough that other contexts'
+// start is nothing (62 ms at n = 2^20), short enough that other contexts'
 // launches get their turn.
 constexpr uint32_t FLOW_ITERS = 1000;
 

@@ -1,4 +1,4 @@
-// m2_flow.cu -- k squarings of one mid-size test (n = 2^12 ... 2^18) in one
+// m2_flow.cu -- k squarings of one mid-size test (n = 2^12 ... 2^20) in one
 // cooperative launch.
 //
 // h = R x B elements as in the three-pass path, with the same roots, tables
@@ -26,10 +26,11 @@
 // What bounds it: up to n = 2^16 latency -- the serial chain of butterfly levels
 // on a few warps per SM, and three L2 round trips (two hand-overs and the
 // carry) -- and from n = 2^17 on the integer pipes of the SMs that have a unit.
-// Measured, us per squaring, three-pass launches -> here: n = 2^12 16.2 -> 7.0,
-// 2^13 18.5 -> 6.7, 2^14 19.5 -> 7.7, 2^15 21.7 -> 8.8, 2^16 27.5 -> 9.6,
-// 2^17 31.9 -> 10.0, 2^18 37.3 -> 16.3.  The three passes paid three launches
-// per squaring, each with cold L1 tables, and ran rows on as few as 32 SMs.
+// Measured, us per squaring, three-pass launches -> here: n = 2^12 16.2 -> 6.5,
+// 2^13 18.5 -> 6.6, 2^14 19.5 -> 7.6, 2^15 21.7 -> 8.2, 2^16 27.5 -> 9.6,
+// 2^17 31.9 -> 10.0, 2^18 37.3 -> 15.7, 2^19 44.9 -> 30.4, 2^20 79.6 -> 62.3.
+// The three passes paid three launches per squaring, each with cold L1 tables,
+// and ran rows on as few as 32 SMs.
 #include "m2_split.cuh"
 
 namespace M2K_NS {
@@ -121,10 +122,11 @@ template <int LR_, int LB_, int C_> struct Shape {
     static constexpr u32 UC = R * C, UR = 2 * B;             // elements of a column group and of a row pair
     static constexpr u32 NBC = UC / 4, NBR = UR / 4;         // radix-4 butterflies of a level
     static constexpr u32 NB0 = NBC > NBR ? NBC : NBR;
-    static constexpr u32 NF = NB0 < 32 ? 32 : NB0;           // threads per field
+    static constexpr u32 NF = NB0 < 32 ? 32 : NB0 > 512 ? 512 : NB0;   // threads per field
     static constexpr u32 NT = kDual ? 2 * NF : NF;
     static constexpr u32 SEGS = UC / 2;                      // carry segments (2 elements, 4 digits) of a column group
     static constexpr u32 SI = (SEGS + NT - 1) / NT;          // segments per thread
+    static constexpr u32 SR = C / 2;                         // segments per row
     static constexpr u32 CTAS = G > R / 2 ? G : R / 2;
     static constexpr u32 SLOTS = UC > UR ? UC : UR;
     static constexpr u32 SMEM = 24 * SLOTS;
@@ -132,76 +134,97 @@ template <int LR_, int LB_, int C_> struct Shape {
 
 template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
-// the levels of one CTA's units in one field
+// the levels of one CTA's units in one field: each thread runs the butterflies
+// fb, fb + NF, ... of a level
 template <class S, class X> struct Unit {
     X* z;              // shared slots
     X* g;              // global elements
     const DTw* tw4;
     const DTw* tc;
-    u32 b;             // butterfly index of this thread
+    u32 fb;            // thread of the field
     u32 bar;           // barrier of the field's warps
 
+    static constexpr u32 IC = (S::NBC + S::NF - 1) / S::NF, IR = (S::NBR + S::NF - 1) / S::NF;
     __device__ __forceinline__ void sync() const { bar_field<S::NF>(bar); }
+
+    // One level: the butterflies' twiddles of a thread's first butterfly are
+    // fetched before the barrier.  op(x, t): the level's arithmetic; ld/st by
+    // butterfly index and slot offset.
+    template <u32 ITERS, u32 NB, class TW, class LD, class OP, class ST>
+    __device__ __forceinline__ void level(bool barrier, TW&& tw, LD&& ld, OP&& op, ST&& st) const {
+        Tri<X> t;
+        const bool on = NB % S::NF == 0 || fb < NB;
+        if (on) tw(fb, t);
+        if (barrier) sync();
+        if (!on) return;
+        if (ITERS == 1) {
+            X x[4];
+            ld(fb, x);
+            op(x, t);
+            st(fb, x);
+        } else {
+#pragma unroll 1
+            for (u32 b = fb; b < NB; b += S::NF) {
+                X x[4];
+                if (b != fb) tw(b, t);
+                ld(b, x);
+                op(x, t);
+                st(b, x);
+            }
+        }
+    }
 
     // ---- column group cg ----
     // the forward levels: shared slots in, global out
     __device__ __forceinline__ void cols_fwd(u32 cg) const {
         constexpr int NL = S::LR / 2;
-        const bool on = S::NBC == S::NF || b < S::NBC;
-        const u32 cc = b % S::C, rho = b / S::C;
 #pragma unroll
         for (int l = 0; l < NL; ++l) {
-            const u32 M = S::R >> (2 * l), Q = M / 4, j = rho / Q, i = rho % Q;
-            Tri<X> t;
-            if (l > 0 && on) t = ldtri<X>(tw4, (1u << (2 * l)) + j);
-            if (l > 0) sync();
-            if (!on) continue;
-            const u32 s0 = sw((j * M + i) * S::C + cc);
-            X x[4];
+            const u32 M = S::R >> (2 * l), Q = M / 4;
+            level<IC, S::NBC>(l > 0, [&](u32 b, Tri<X>& t) { if (l > 0) t = ldtri<X>(tw4, (1u << (2 * l)) + b / S::C / Q); },
+                  [&](u32 b, X (&x)[4]) {
+                      const u32 rho = b / S::C, s0 = sw((rho / Q * M + rho % Q) * S::C + b % S::C);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q * S::C)];
-            if (l == 0) xdif4_1(x);
-            else xdif4(x, t);
-            if (l < NL - 1) {
+                      for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q * S::C)];
+                  },
+                  [&](X (&x)[4], const Tri<X>& t) { if (l == 0) xdif4_1(x); else xdif4(x, t); },
+                  [&](u32 b, const X (&x)[4]) {
+                      const u32 rho = b / S::C, cc = b % S::C;
+                      if (l < NL - 1) {
+                          const u32 s0 = sw((rho / Q * M + rho % Q) * S::C + cc);
 #pragma unroll
-                for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q * S::C)] = x[m];
-            } else {
-                X* p = g + (u64)(4 * j) * S::B + cg * S::C + cc;
+                          for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q * S::C)] = x[m];
+                      } else {
+                          X* p = g + (u64)(4 * rho) * S::B + cg * S::C + cc;
 #pragma unroll
-                for (int m = 0; m < 4; ++m) st_tagged<0>(p + m * S::B, x[m]);
-            }
+                          for (int m = 0; m < 4; ++m) st_tagged<0>(p + m * S::B, x[m]);
+                      }
+                  });
         }
     }
     // the inverse levels: global in, shared slots out
     __device__ __forceinline__ void cols_inv(u32 cg, Wait& w) const {
         constexpr int NL = S::LR / 2;
-        const bool on = S::NBC == S::NF || b < S::NBC;
-        const u32 cc = b % S::C, rho = b / S::C;
 #pragma unroll
         for (int l = NL - 1; l >= 0; --l) {
-            const u32 M = S::R >> (2 * l), Q = M / 4, j = rho / Q, i = rho % Q;
-            Tri<X> t;
-            if (l > 0 && on) t = ldtri<X>(tw4, (1u << (2 * l)) + j);
-            X x[4];
-            const u32 s0 = sw((j * M + i) * S::C + cc);
-            if (l == NL - 1) {
-                if (on) take4<1>(x, g + (u64)(4 * j) * S::B + cg * S::C + cc, S::B, w);
-            } else {
-                sync();
-                if (on) {
+            const u32 M = S::R >> (2 * l), Q = M / 4;
+            level<IC, S::NBC>(true, [&](u32 b, Tri<X>& t) { if (l > 0) t = ldtri<X>(tw4, (1u << (2 * l)) + b / S::C / Q); },
+                  [&](u32 b, X (&x)[4]) {
+                      const u32 rho = b / S::C, cc = b % S::C;
+                      if (l == NL - 1) {
+                          take4<1>(x, g + (u64)(4 * rho) * S::B + cg * S::C + cc, S::B, w);
+                      } else {
+                          const u32 s0 = sw((rho / Q * M + rho % Q) * S::C + cc);
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q * S::C)];
-                }
-            }
-            if (on) {
-                if (l > 0) xdit4(x, t);
-                else dit_adds(x);
-            }
-            if (l == NL - 1) sync();   // the row phase's last reads of the slots are done
-            if (on) {
+                          for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q * S::C)];
+                      }
+                  },
+                  [&](X (&x)[4], const Tri<X>& t) { if (l == 0) dit_adds(x); else xdit4(x, t); },
+                  [&](u32 b, const X (&x)[4]) {
+                      const u32 rho = b / S::C, s0 = sw((rho / Q * M + rho % Q) * S::C + b % S::C);
 #pragma unroll
-                for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q * S::C)] = x[m];
-            }
+                      for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q * S::C)] = x[m];
+                  });
         }
     }
 
@@ -210,59 +233,67 @@ template <class S, class X> struct Unit {
         constexpr int NL = S::LB / 2;                        // radix-4 levels
         constexpr bool ODD = (S::LB & 1) != 0;
         constexpr int NF4 = ODD ? NL : NL - 1;               // those outside the tail
-        const bool on = S::NBR == S::NF || b < S::NBR;
         u32 t0 = 0, t1 = 1;
         if (pi) {
             const u32 e = 32u - __clz(pi), a = pi - (1u << (e - 1));
             t0 = (1u << e) + a;
             t1 = (2u << e) - 1u - a;
         }
-        const u32 sl = b / (S::B / 4), rho = b % (S::B / 4), trow = sl ? t1 : t0;
 #pragma unroll
         for (int l = 0; l < NF4; ++l) {
-            const u32 M = S::B >> (2 * l), Q = M / 4, j = rho / Q, i = rho % Q;
-            Tri<X> t;
-            if (on) t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + j);
-            const u32 s0 = sw(sl * S::B + j * M + i);
-            X x[4];
-            if (l == 0) {
-                if (on) take4<0>(x, g + (u64)trow * S::B + i, Q, w);
-            } else {
-                sync();
-                if (on) {
+            const u32 M = S::B >> (2 * l), Q = M / 4;
+            level<IR, S::NBR>(true, [&](u32 b, Tri<X>& t) {
+                      const u32 rho = b % (S::B / 4), trow = b / (S::B / 4) ? t1 : t0;
+                      t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + rho / Q);
+                  },
+                  [&](u32 b, X (&x)[4]) {
+                      const u32 rho = b % (S::B / 4), sl = b / (S::B / 4);
+                      if (l == 0) {
+                          take4<0>(x, g + (u64)(sl ? t1 : t0) * S::B + rho, Q, w);
+                      } else {
+                          const u32 s0 = sw(sl * S::B + rho / Q * M + rho % Q);
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q)];
-                }
-            }
-            if (on) xdif4(x, t);
-            if (l == 0) sync();   // the column phase's last reads of the slots are done
-            if (on) {
+                          for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q)];
+                      }
+                  },
+                  [&](X (&x)[4], const Tri<X>& t) { xdif4(x, t); },
+                  [&](u32 b, const X (&x)[4]) {
+                      const u32 rho = b % (S::B / 4), sl = b / (S::B / 4), s0 = sw(sl * S::B + rho / Q * M + rho % Q);
 #pragma unroll
-                for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q)] = x[m];
-            }
+                      for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q)] = x[m];
+                  });
         }
-        if (ODD) tail2(pi, t0, t1, on);
-        else tail4(pi, t0, t1, on);
+        sync();
+#pragma unroll 1
+        for (u32 b = fb; b < S::NBR; b += S::NF) {
+            if (ODD) tail2(pi, t0, t1, b);
+            else tail4(pi, t0, t1, b);
+        }
 #pragma unroll
         for (int l = NF4 - 1; l >= 0; --l) {
-            const u32 M = S::B >> (2 * l), Q = M / 4, j = rho / Q, i = rho % Q;
-            Tri<X> t;
-            if (on) t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + j);
-            sync();
-            if (!on) continue;
-            const u32 s0 = sw(sl * S::B + j * M + i);
-            X x[4];
+            const u32 M = S::B >> (2 * l), Q = M / 4;
+            level<IR, S::NBR>(true, [&](u32 b, Tri<X>& t) {
+                      const u32 rho = b % (S::B / 4), trow = b / (S::B / 4) ? t1 : t0;
+                      t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + rho / Q);
+                  },
+                  [&](u32 b, X (&x)[4]) {
+                      const u32 rho = b % (S::B / 4), sl = b / (S::B / 4), s0 = sw(sl * S::B + rho / Q * M + rho % Q);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q)];
-            xdit4(x, t);
-            if (l > 0) {
+                      for (int m = 0; m < 4; ++m) x[m] = z[s0 ^ sw(m * Q)];
+                  },
+                  [&](X (&x)[4], const Tri<X>& t) { xdit4(x, t); },
+                  [&](u32 b, const X (&x)[4]) {
+                      const u32 rho = b % (S::B / 4), sl = b / (S::B / 4);
+                      if (l > 0) {
+                          const u32 s0 = sw(sl * S::B + rho / Q * M + rho % Q);
 #pragma unroll
-                for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q)] = x[m];
-            } else {
-                X* p = g + (u64)trow * S::B + i;
+                          for (int m = 0; m < 4; ++m) z[s0 ^ sw(m * Q)] = x[m];
+                      } else {
+                          X* p = g + (u64)(sl ? t1 : t0) * S::B + rho;
 #pragma unroll
-                for (int m = 0; m < 4; ++m) st_tagged<1>(p + m * Q, x[m]);
-            }
+                          for (int m = 0; m < 4; ++m) st_tagged<1>(p + m * Q, x[m]);
+                      }
+                  });
         }
     }
     // blocks j (row t0) and j' (row t1) of `per` consecutive positions that
@@ -285,13 +316,12 @@ template <class S, class X> struct Unit {
     }
     // log2 B odd: the radix-2 level, the centre square and the inverse level
     // on two mirror blocks of 2 positions per thread
-    __device__ __forceinline__ void tail2(u32 pi, u32 t0, u32 t1, bool on) const {
+    __device__ __forceinline__ void tail2(u32 pi, u32 t0, u32 t1, u32 b) const {
         u32 j, jm;
         blocks(pi, b, 2, j, jm);
         X cx, cy;
-        if (on) { ldtw(cx, tc, gblock(t0, t1, 2, j)); ldtw(cy, tc, gblock(t0, t1, 2, jm)); }
-        sync();
-        if (!on) return;
+        ldtw(cx, tc, gblock(t0, t1, 2, j));
+        ldtw(cy, tc, gblock(t0, t1, 2, jm));
         const u32 sx = sw(2 * j), sy = sw(2 * jm);
         X x0 = z[sx], x1 = z[sx ^ sw(1)], y0 = z[sy], y1 = z[sy ^ sw(1)];
         const X ux = xmul(x1, cx), uy = xmul(y1, cy);
@@ -313,16 +343,13 @@ template <class S, class X> struct Unit {
     }
     // log2 B even: the last radix-4 level, the centre square and its inverse
     // level; neighbouring lanes hold mirror blocks and swap odd positions
-    __device__ __forceinline__ void tail4(u32 pi, u32 t0, u32 t1, bool on) const {
+    __device__ __forceinline__ void tail4(u32 pi, u32 t0, u32 t1, u32 b) const {
+        static_assert((S::LB & 1) || S::NBR % 32 == 0, "whole warps take part");
         const u32 item = b >> 1, s = b & 1u;
         u32 j, jm;
-        blocks(pi, on ? item : 0, 4, j, jm);
+        blocks(pi, item, 4, j, jm);
         if (s) j = jm;
-        Tri<X> t;
-        t = ldtri<X>(tw4, S::H / 4 + gblock(t0, t1, 4, j));
-        sync();
-        static_assert((S::LB & 1) || S::NBR >= 32, "whole warps take part");
-        if (!on) return;
+        const Tri<X> t = ldtri<X>(tw4, S::H / 4 + gblock(t0, t1, 4, j));
         const u32 s0 = sw(4 * j);
         X x[4];
 #pragma unroll
@@ -432,7 +459,7 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
         for (u32 q = 0; q < S::SI; ++q) {
             const u32 s = tid + q * S::NT;
             if (s >= S::SEGS) continue;
-            const u32 p = sw(2 * s), r = 2 * s / S::C;
+            const u32 p = sw(2 * s), r = s / S::SR;
             i64 c = 0;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -445,7 +472,7 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
                 d[q][2 * k] = crt_digit(x0, y0, wd & 0xffu, mul, sub, c, bad, !kDual);
                 d[q][2 * k + 1] = crt_digit(x1, y1, (wd >> 8) & 0xffu, mul, 0, c, bad, !kDual);
             }
-            if (S::C == 2 || (s & 1u)) st_relaxed(A.fcar + x * S::R + r, ((u64)c << 1) | par);
+            if (s % S::SR == S::SR - 1) st_relaxed(A.fcar + x * S::R + r, ((u64)c << 1) | par);
             cin[q] = c;
         }
         if (bad) atomicOr(A.status, ST_CARRY_RANGE);
@@ -453,10 +480,10 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
         for (u32 q = 0; q < S::SI; ++q) {
             const u32 s = tid + q * S::NT;
             if (s >= S::SEGS) continue;
-            const u32 r = 2 * s / S::C;
+            const u32 r = s / S::SR;
             i64 c = cin[q];
-            if (S::C == 4) c = __shfl_up_sync(0xffffffffu, c, 1);
-            if (S::C == 2 || !(s & 1u)) {
+            if (S::SR > 1) c = __shfl_up_sync(0xffffffffu, c, 1);
+            if (s % S::SR == 0) {
                 // the segment before this row's first one
                 const u64* from = x ? A.fcar + (x - 1) * S::R + r : A.fcar + (S::G - 1) * S::R + ((r - 1) & (S::R - 1));
                 u32 n = 0;
@@ -514,13 +541,21 @@ template <class S> cudaError_t flow_launch(const FlowArgs& A, cudaStream_t s) {
     return cudaLaunchKernelEx(&cfg, k_flow<S>, A);
 }
 
-// the shapes by log2 h
-#define M2_FLOW_SHAPES(X) X(11, 6, 5, 2) X(12, 6, 6, 2) X(13, 6, 7, 2) X(14, 6, 8, 4) X(15, 8, 7, 2) X(16, 8, 8, 2) X(17, 8, 9, 4)
+// The shapes by log2 h: log2 rows, log2 row length, columns per group.  R and C
+// put the two phases' units on about as many CTAs as SMs where the size allows
+// (128 of each from h = 2^16), with segments of at least 4 digits; from h = 2^18
+// the SM count fixes the units (2048 and 4096 elements, 84% of the SMs) and a
+// CTA fills its SM with 512 threads per field, 64 registers each (h = 2^18:
+// 256 threads per field 34.0 us a squaring, 512 30.4; h = 2^19: 256 68.4, 512
+// 62.3).  Larger sizes keep the three-pass kernels: at h = 2^20 a unit of 8192
+// elements per SM would take as long as those, which use all 152 SMs.
+#define M2_FLOW_SHAPES(X) \
+    X(11, 6, 5, 2) X(12, 6, 6, 2) X(13, 6, 7, 2) X(14, 6, 8, 4) X(15, 8, 7, 2) X(16, 8, 8, 2) X(17, 8, 9, 4) X(18, 8, 10, 8) X(19, 8, 11, 16)
 
 }  // namespace
 
 size_t flow_carry_words(int lh) {
-#define M2_FLOW_W(LH, LR, LB, C) if (lh == LH) return (size_t)1 << (LR + LB) >> (C == 4 ? 2 : 1);
+#define M2_FLOW_W(LH, LR, LB, C) if (lh == LH) return ((size_t)1 << (LR + LB)) / C;
     M2_FLOW_SHAPES(M2_FLOW_W)
 #undef M2_FLOW_W
     return 0;

@@ -7,10 +7,10 @@ pytestmark = pytest.mark.gpu
 
 # (log2 n, smallest and largest exponent of that transform)
 DUAL = [(12, 81929, 159739), (13, 159763, 319483), (14, 319489, 622577), (15, 622603, 1245169), (16, 1245187, 2424827),
-        (17, 2424833, 4849651), (18, 4849681, 9437179)]
+        (17, 2424833, 4849651), (18, 4849681, 9437179), (19, 9437185, 18874367), (20, 18874369, 36700159)]
 
 GF61 = [(12, 49153, 98303), (13, 98305, 188415), (14, 188417, 376831), (15, 376833, 720895), (16, 720897, 1441791),
-        (17, 1441793, 2752511), (18, 2752513, 5505023)]
+        (17, 1441793, 2752511), (18, 2752513, 5505023), (19, 5505025, 10485759), (20, 10485761, 20971519)]
 
 
 def _random_state(m2, p, fields, seed):
@@ -26,7 +26,7 @@ def _compare(m2, p, mode, fields, ln):
     with m2.Engine(p, mode, fields=fields) as a, m2.Engine(p, mode, fields=fields, path=m2.PATH_LARGE) as b:
         assert a.info().ln == ln and a.info().path == m2.PATH_LARGE
         # the kernel under test is the one that runs, but for a carry span beyond its segments of 4 digits
-        # (the smallest GF(P61^2)-only exponents of n = 2^18, which keep the three-pass kernels)
+        # (the smallest GF(P61^2)-only exponents of n = 2^18 and up, which keep the three-pass kernels)
         assert (a.launches_for(7) == 1) == (a.info().span <= 3)
         for state in (start, extreme):
             a.set_digits(state, 0)
@@ -98,9 +98,9 @@ def test_flow_wait_runs_out_and_reports_timeout(m2, oracle_mod, p):
 
 
 def test_flow_contexts_share_the_gpu(m2):
-    """Three contexts whose launches are in flight together on streams of their
-    own end where each ends alone."""
-    ps = (216091, 1257787, 6972593)
+    """Contexts whose launches are in flight together on streams of their own
+    (more CTAs than the GPU holds at once) end where each ends alone."""
+    ps = (216091, 1257787, 6972593, 13466917, 24036583, 13466917)
     alone = []
     for p in ps:
         with m2.Engine(p, 1) as e:
