@@ -147,26 +147,29 @@ template <class S, class X> struct Unit {
     static constexpr u32 IC = (S::NBC + S::NF - 1) / S::NF, IR = (S::NBR + S::NF - 1) / S::NF;
     __device__ __forceinline__ void sync() const { bar_field<S::NF>(bar); }
 
-    // One level: the butterflies' twiddles of a thread's first butterfly are
-    // fetched before the barrier.  op(x, t): the level's arithmetic; ld/st by
-    // butterfly index and slot offset.
+    // One level.  tw, ld, st: twiddles, operands and results of a butterfly by
+    // its index; op: the level's arithmetic.  With registers to spare the
+    // twiddles are fetched before the barrier; with 1024 threads of 64
+    // registers the other warps hide them (h = 2^19: 62.3 -> 60.1 us).
     template <u32 ITERS, u32 NB, class TW, class LD, class OP, class ST>
     __device__ __forceinline__ void level(bool barrier, TW&& tw, LD&& ld, OP&& op, ST&& st) const {
+        constexpr bool EARLY = S::NT <= 512;
         Tri<X> t;
         const bool on = NB % S::NF == 0 || fb < NB;
-        if (on) tw(fb, t);
+        if (EARLY && on) tw(fb, t);
         if (barrier) sync();
         if (!on) return;
         if (ITERS == 1) {
             X x[4];
             ld(fb, x);
+            if (!EARLY) tw(fb, t);
             op(x, t);
             st(fb, x);
         } else {
 #pragma unroll 1
             for (u32 b = fb; b < NB; b += S::NF) {
                 X x[4];
-                if (b != fb) tw(b, t);
+                if (!EARLY || b != fb) tw(b, t);
                 ld(b, x);
                 op(x, t);
                 st(b, x);
@@ -380,8 +383,8 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
     const u32 tid = threadIdx.x, x = blockIdx.x;
     const bool second = kDual && tid >= S::NF;     // the GF(P31^2) half's warps
     const u32 fb = second ? tid - S::NF : tid;
-    const Unit<S, X61> ua{za, reinterpret_cast<X61*>(A.za), A.tw4, A.tc, fb, 1};
-    const Unit<S, X31> ub{zb, reinterpret_cast<X31*>(A.zb), A.tw4, A.tc, fb, 2};
+    Unit<S, X61> ua{za, reinterpret_cast<X61*>(A.za), A.tw4, A.tc, fb, 1};
+    Unit<S, X31> ub{zb, reinterpret_cast<X31*>(A.zb), A.tw4, A.tc, fb, 2};
     const bool has_cols = S::G == S::CTAS || x < S::G, has_rows = S::R / 2 == S::CTAS || x < S::R / 2;
     Wait w{A.status, false};
     const u32 base = has_cols ? A.parity[x] : 0u;  // squarings handed over so far (bit 0); bit 1 never matches a word's tag
@@ -420,6 +423,9 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
     const u32 mul = (A.mode == PRP3) ? 3u : 1u;
 
     for (u32 it = 0;; ++it) {
+        // full registers: the levels' addresses and twiddles are made anew in
+        // every squaring (kept over the loop they were spilled)
+        if (S::NT > 512) asm volatile("" : "+r"(ua.fb), "+r"(ub.fb));
         if (has_cols) {
             // weigh this thread's digits into the slots, then the forward levels
 #pragma unroll
