@@ -37,23 +37,22 @@ std::map<std::pair<int, u64>, TwTables> g_tw;
 
 cudaMemPool_t ctx_pool(int device);
 
-// Tables of a new transform size come from the stream-ordered pool on a stream
-// of their own, so building them waits for nothing else running on the device
-// (a cudaMalloc may synchronise the whole device).  Kept until the process ends.
+// Tables of a new transform size come from the stream-ordered pool and are
+// built on a stream of their own, so making them waits for nothing else running
+// on the device (a cudaMalloc may synchronise the whole device).  Kept until
+// the process ends.
 int get_twiddles(int device, u64 h, TwTables& out) {
     std::lock_guard<std::mutex> lk(g_tw_mu);
     auto it = g_tw.find({device, h});
     if (it != g_tw.end()) { out = it->second; return M2_OK; }
-    m2::Twiddles T = m2::make_twiddles(h);
     TwTables t;
-    const size_t b4 = T.tw4.size() * sizeof(m2::Dual), bc = T.tc.size() * sizeof(m2::Dual);
+    const size_t b4 = m2k::twiddle_entries(h) * sizeof(m2k::DTw), bc = std::max<u64>(h / 2, 1) * sizeof(m2k::DTw);
     cudaMemPool_t mp = ctx_pool(device);
     cudaStream_t s = nullptr;
     if (!mp || cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); return M2_ECUDA; }
     cudaError_t e = cudaMallocFromPoolAsync((void**)&t.tw4, b4, mp, s);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void**)&t.tc, bc, mp, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(t.tw4, T.tw4.data(), b4, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(t.tc, T.tc.data(), bc, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = m2k::launch_twiddles(t.tw4, t.tc, (unsigned)h, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaStreamDestroy(s);
     if (e != cudaSuccess) {
@@ -97,6 +96,10 @@ int fail_cuda(const char* where, cudaError_t e) {
     std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s", where, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? M2_ENOMEM : M2_ECUDA;
 }
+
+// Digits that the host keeps the layout of: enough for 64 bits and for small
+// values wherever digits have a bit at all (n > 64 has q >= 10).
+constexpr u64 HEAD = 72;
 
 u32 total_iters_for(u32 p, int mode) {
     if (mode == M2_MODE_LL) return p >= 2 ? p - 2 : 0;
@@ -158,19 +161,46 @@ struct m2_ctx {
     // GRAPH_ITERS[i] iterations of the three-pass path captured once and replayed
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     bool graph_failed = false;
-    // canonical digits and carry-propagation scratch (allocated on first read)
+    void* d_slab = nullptr;    // the allocation that holds the buffers above
+    // canonical digits and carry-propagation scratch (allocated on first read, in d_read)
+    void* d_read = nullptr;
     unsigned long long* d_canon = nullptr;
     void* d_norm = nullptr;
 };
 
 namespace {
 
-template <class T> int dalloc(m2_ctx* c, T** p, size_t bytes) {
-    cudaMemPool_t mp = ctx_pool(c->device);
-    if (!mp) return M2_ECUDA;
-    if (cudaMallocFromPoolAsync((void**)p, bytes, mp, c->stream) != cudaSuccess) { cudaGetLastError(); *p = nullptr; return M2_ENOMEM; }
-    c->bytes += bytes;
-    return M2_OK;
+// One allocation for a set of buffers (256-byte aligned parts).  An allocation
+// from the stream-ordered pool costs about 5 us per stream that has used the
+// pool (it looks for blocks freed on each), so a context of ten buffers made
+// beside 60 others took 2 ms when it asked for each.
+struct Slab {
+    struct Part { void** p; size_t bytes; };
+    std::vector<Part> parts;
+    template <class T> void add(T** p, size_t bytes) { parts.push_back(Part{(void**)p, bytes}); }
+    int alloc(m2_ctx* c, void** base) {
+        cudaMemPool_t mp = ctx_pool(c->device);
+        if (!mp) return M2_ECUDA;
+        size_t total = 0;
+        for (const Part& q : parts) total += (q.bytes + 255) & ~size_t(255);
+        if (cudaMallocFromPoolAsync(base, total, mp, c->stream) != cudaSuccess) { cudaGetLastError(); *base = nullptr; return M2_ENOMEM; }
+        char* at = static_cast<char*>(*base);
+        for (const Part& q : parts) {
+            *q.p = at;
+            at += (q.bytes + 255) & ~size_t(255);
+            c->bytes += q.bytes;
+        }
+        return M2_OK;
+    }
+};
+
+// canonical digits and the carry propagation's scratch, on the first read
+int canon_alloc(m2_ctx* c) {
+    if (c->d_canon) return M2_OK;
+    Slab m;
+    m.add(&c->d_canon, c->L.n * sizeof(u64));
+    m.add(&c->d_norm, m2k::norm_scratch_bytes(c->L.n));
+    return m.alloc(c, &c->d_read);
 }
 
 // the fused column kernel's G epoch flags followed by its 64-bit ticket and
@@ -250,8 +280,8 @@ cudaError_t reset_sync_words(m2_ctx* c) {
 
 int cuda_err(cudaError_t e) { return e == cudaSuccess ? M2_OK : (e == cudaErrorMemoryAllocation ? M2_ENOMEM : M2_ECUDA); }
 
-int upload_state(m2_ctx* c, const std::vector<u64>& canon) {
-    std::vector<i64> bal = m2::balanced_digits(c->L, canon);
+int upload_state(m2_ctx* c, const m2::Layout& L, const std::vector<u64>& canon) {
+    std::vector<i64> bal = m2::balanced_digits(L, canon);
     cudaError_t e = cudaMemcpyAsync(c->d_digits, bal.data(), bal.size() * sizeof(i64), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = reset_sync_words(c);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -262,8 +292,7 @@ int upload_state(m2_ctx* c, const std::vector<u64>& canon) {
 // canonical digits land in d_canon, the summary flags in the scratch.
 int device_canonical(m2_ctx* c, m2k::NormArgs& a) {
     int rc;
-    if (!c->d_canon && (rc = dalloc(c, &c->d_canon, c->L.n * sizeof(u64)))) return rc;
-    if (!c->d_norm && (rc = dalloc(c, (char**)&c->d_norm, m2k::norm_scratch_bytes(c->L.n)))) return rc;
+    if ((rc = canon_alloc(c))) return rc;
     a = m2k::NormArgs{};
     a.digits = c->d_digits;
     a.carries = (c->path == M2_PATH_LARGE) ? c->d_carries : nullptr;
@@ -281,7 +310,7 @@ int read_head(m2_ctx* c, std::vector<u64>& head, unsigned& flags) {
     m2k::NormArgs a;
     int rc = device_canonical(c, a);
     if (rc) return rc;
-    head.assign(std::min<u64>(c->L.n, 72), 0);
+    head.assign(std::min<u64>(c->L.n, HEAD), 0);
     cudaError_t e = cudaMemcpyAsync(head.data(), c->d_canon, head.size() * sizeof(u64), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, a.flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
     if (e != cudaSuccess) return fail_cuda("digits read", e);
@@ -341,8 +370,7 @@ int raw_state(m2_ctx* c, long long** digits) {
 
 int canon_buffer(m2_ctx* c, unsigned long long** buf) {
     int rc;
-    if (!c->d_canon && (rc = dalloc(c, &c->d_canon, c->L.n * sizeof(u64)))) return rc;
-    if (!c->d_norm && (rc = dalloc(c, (char**)&c->d_norm, m2k::norm_scratch_bytes(c->L.n)))) return rc;
+    if ((rc = canon_alloc(c))) return rc;
     *buf = c->d_canon;
     return M2_OK;
 }
@@ -399,7 +427,7 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
     if (m2::transform_log2(p, gf61 ? 61 : 92) > 30) return M2_EUNSUPPORTED;
     std::unique_ptr<m2_ctx> c(new (std::nothrow) m2_ctx());
     if (!c) return M2_ENOMEM;
-    c->L = m2::make_layout(p, gf61 ? 61 : 92);
+    c->L = m2::make_layout(p, gf61 ? 61 : 92, HEAD);
     c->gf61 = gf61;
     c->mode = mode;
     c->device = o.device;
@@ -424,14 +452,35 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
     const u64 n = c->L.n;
     if ((rc = get_twiddles(c->device, h, c->tw))) { m2_destroy(c.release()); return rc; }
     m2_ctx* raw = c.get();
-    if ((rc = dalloc(raw, &raw->d_w61, n)) || (rc = dalloc(raw, &raw->d_w31, n)) ||
-        (rc = dalloc(raw, &raw->d_status, sizeof(int))) || (rc = dalloc(raw, &raw->d_digits, n * sizeof(i64)))) {
-        m2_destroy(c.release());
-        return rc;
+    Slab mem;
+    mem.add(&raw->d_w61, n);
+    mem.add(&raw->d_w31, n);
+    mem.add(&raw->d_status, sizeof(int));
+    mem.add(&raw->d_digits, n * sizeof(i64));
+    const int lh = raw->L.ln - 1;
+    size_t cw = 0;
+    if (path == M2_PATH_SMALL) {
+        mem.add(&raw->d_test, sizeof(m2k::SmallTest));
+    } else {
+        const m2k::LargePlan& P = raw->plan;
+        mem.add(&raw->d_carries, sizeof(i64) * (size_t)P.R * P.G);
+        mem.add(&raw->d_za, sizeof(ulonglong2) * h);
+        mem.add(&raw->d_zb, sizeof(uint2) * h);
+        mem.add(&raw->d_flags, flags_bytes(P));
+        // one launch for all squarings of a call where a shape of that kernel
+        // serves the size; M2_PATH_LARGE and a -B hint ask for the three-pass kernels
+        raw->flow = o.path == M2_PATH_AUTO && o.carry_pairs == 0 && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 &&
+                    m2k::flow_setup(lh, gf61) == cudaSuccess;
+        cudaGetLastError();
+        // the inverse column passes' per-element table
+        if (m2k::cols_q_supported(P) || raw->flow) mem.add(&raw->d_aux, sizeof(uint2) * h);
+        if (raw->flow) {
+            cw = m2k::flow_carry_words(lh);
+            mem.add(&raw->d_flow, 8 * cw + 4 * m2k::flow_groups(lh));
+        }
     }
-    cudaError_t e = cudaMemcpyAsync(raw->d_w61, raw->L.w61.data(), n, cudaMemcpyHostToDevice, raw->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(raw->d_w31, raw->L.w31.data(), n, cudaMemcpyHostToDevice, raw->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(raw->d_status, 0, sizeof(int), raw->stream);
+    if ((rc = mem.alloc(raw, &raw->d_slab))) { m2_destroy(c.release()); return rc; }
+    cudaError_t e = cudaMemsetAsync(raw->d_status, 0, sizeof(int), raw->stream);
     if (e != cudaSuccess) { m2_destroy(c.release()); return M2_ECUDA; }
     if (path == M2_PATH_SMALL) {
         raw->threads = m2k::small_threads_for((unsigned)h);
@@ -445,7 +494,6 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
                 ++shift;
             raw->carry_threads = small_carry_threads(raw->L, raw->span, raw->threads, shift);
         }
-        if ((rc = dalloc(raw, &raw->d_test, sizeof(m2k::SmallTest)))) { m2_destroy(c.release()); return rc; }
         m2k::SmallTest t{};
         t.digits = raw->d_digits; t.w61 = raw->d_w61; t.w31 = raw->d_w31;
         t.tw4 = raw->tw.tw4; t.tc = raw->tw.tc; t.status = raw->d_status;
@@ -467,36 +515,15 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         const m2k::LargePlan& P = raw->plan;
         raw->plan.mode = mode;
         raw->plan.gf61 = gf61 ? 1u : 0u;
-        if ((rc = dalloc(raw, &raw->d_carries, sizeof(i64) * (size_t)P.R * P.G)) ||
-            (rc = dalloc(raw, &raw->d_za, sizeof(ulonglong2) * h)) || (rc = dalloc(raw, &raw->d_zb, sizeof(uint2) * h)) ||
-            (rc = dalloc(raw, &raw->d_flags, flags_bytes(P)))) {
-            m2_destroy(c.release());
-            return rc;
-        }
         raw->bufs = m2k::LargeBufs{raw->d_digits, raw->d_carries, raw->d_za, raw->d_zb, raw->d_w61, raw->d_w31,
                                    raw->tw.tw4, raw->tw.tc, raw->d_status, raw->d_flags};
-        const int lh = raw->L.ln - 1;
-        // one launch for all squarings of a call where a shape of that kernel
-        // serves the size; M2_PATH_LARGE and a -B hint ask for the three-pass kernels
-        raw->flow = o.path == M2_PATH_AUTO && o.carry_pairs == 0 && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 && m2k::flow_setup(lh, gf61) == cudaSuccess;
-        cudaGetLastError();
-        if (m2k::cols_q_supported(P) || raw->flow) {
-            // the inverse column passes' per-element table, built on the device
-            if ((rc = dalloc(raw, &raw->d_aux, sizeof(uint2) * h))) { m2_destroy(c.release()); return rc; }
-            if (m2k::launch_aux(raw->d_aux, raw->d_w61, raw->d_w31, p, raw->L.ln, raw->stream) != cudaSuccess) {
-                m2_destroy(c.release());
-                return M2_ECUDA;
-            }
-            raw->bufs.aux = raw->d_aux;
-        }
+        raw->bufs.aux = raw->d_aux;
         if (m2k::large_setup(P) != cudaSuccess) { m2_destroy(c.release()); return M2_EUNSUPPORTED; }
         raw->fused = m2k::cols_mid_supported(P);
         raw->plan.mid_tickets = (raw->fused && !m2k::cols_mid_cooperative(P)) ? 1u : 0u;
         // the phase barrier measured faster with R = 1024 rows only (n = 2^21)
         raw->plan.mid_barrier = (raw->fused && !P.mid_tickets && P.R == 1024u) ? 1u : 0u;
         if (raw->flow) {
-            const size_t cw = m2k::flow_carry_words(lh);
-            if ((rc = dalloc(raw, &raw->d_flow, 8 * cw + 4 * m2k::flow_groups(lh)))) { m2_destroy(c.release()); return rc; }
             raw->fargs = m2k::FlowArgs{raw->d_digits, raw->d_carries, raw->d_za, raw->d_zb, raw->d_w61, raw->d_w31, raw->d_aux,
                                        raw->tw.tw4, raw->tw.tc, reinterpret_cast<unsigned long long*>(raw->d_flow),
                                        reinterpret_cast<unsigned*>(raw->d_flow + 8 * cw), raw->d_status, 0u, 2u * P.C, raw->span, mode};
@@ -505,7 +532,18 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         raw->bufs.phase = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G + 2);
     }
     raw->bytes += raw->tw.bytes;
-    if ((rc = upload_state(raw, m2::digits_of_small(raw->L, mode == M2_MODE_LL ? 4 : 3)))) { m2_destroy(c.release()); return rc; }
+    // shifts, unweighting records and the start state x0, built on the device
+    // (tiny exponents, whose first digit may not hold x0, take it from the host)
+    const long long x0 = mode == M2_MODE_LL ? 4 : 3;
+    const bool host_state = raw->L.q < 4;
+    e = m2k::launch_test_init(m2k::TestInit{raw->d_w61, raw->d_w31, raw->d_aux, host_state ? nullptr : raw->d_digits, x0, p, raw->L.ln},
+                              raw->stream);
+    if (e == cudaSuccess) e = reset_sync_words(raw);
+    if (e != cudaSuccess) { rc = fail_cuda("test setup", e); m2_destroy(c.release()); return rc; }
+    if (host_state) {
+        const m2::Layout L = m2::make_layout(p, gf61 ? 61 : 92);
+        if ((rc = upload_state(raw, L, m2::digits_of_small(L, (u64)x0)))) { m2_destroy(c.release()); return rc; }
+    }
     *out = c.release();
     return M2_OK;
 }
@@ -561,8 +599,7 @@ int m2_set_digits(m2_ctx* c, const uint64_t* digits, uint32_t iteration) {
     // balanced on the device, which also checks that it is canonical; anything
     // else is reduced on the host first
     int rc;
-    if (!c->d_canon && (rc = dalloc(c, &c->d_canon, c->L.n * sizeof(u64)))) return rc;
-    if (!c->d_norm && (rc = dalloc(c, (char**)&c->d_norm, m2k::norm_scratch_bytes(c->L.n)))) return rc;
+    if ((rc = canon_alloc(c))) return rc;
     unsigned* d_bad = reinterpret_cast<unsigned*>(c->d_norm);   // scratch word, free between reads
     unsigned bad = 0;
     cudaError_t e = cudaMemsetAsync(d_bad, 0, sizeof(unsigned), c->stream);
@@ -575,12 +612,13 @@ int m2_set_digits(m2_ctx* c, const uint64_t* digits, uint32_t iteration) {
     if (e != cudaSuccess) return fail_cuda("state upload", e);
     if (bad) {
         std::vector<u64> canon;
+        const m2::Layout L = m2::make_layout(c->L.p, c->gf61 ? 61 : 92);
         try {
-            canon = m2::canonical_from_unsigned(c->L, digits);
+            canon = m2::canonical_from_unsigned(L, digits);
         } catch (const std::exception&) {
             return M2_EINVAL;
         }
-        if ((rc = upload_state(c, canon))) return rc;
+        if ((rc = upload_state(c, L, canon))) return rc;
         cudaMemset(c->d_status, 0, sizeof(int));
     }
     c->iteration = iteration;
@@ -607,12 +645,13 @@ int m2_verdict(m2_ctx* c, int* is_prime) {
     if (rc) return rc;
     u64 want = c->mode == M2_MODE_LL ? 0 : (c->mode == M2_MODE_PRP ? 9 : 3);
     if (c->L.p < 64) want %= (u64(1) << c->L.p) - 1;
-    const std::vector<u64> w = m2::digits_of_small(c->L, want);
     // digits from index 8 on are zero when the result was all ones (written as
     // zero) or when no digit there is nonzero
     bool same = (flags & 1u) || !(flags & 2u);
-    for (u64 j = 0; j < head.size() && same; ++j) same = (head[j] == w[j]);
-    for (u64 j = head.size(); j < w.size() && same; ++j) same = (w[j] == 0);
+    for (u64 j = 0; j < head.size() && same; ++j) {
+        const u64 pos = c->L.bitpos[j], w = c->L.width[j];
+        same = head[j] == (pos < 64 ? (want >> pos) & ((u64(1) << w) - 1) : 0);
+    }
     *is_prime = same ? 1 : 0;
     return M2_OK;
 }
@@ -707,10 +746,8 @@ void m2_destroy(m2_ctx* c) {
     cudaSetDevice(c->device);
     // stream-ordered frees: they follow the context's queued work and do not
     // wait for other streams; its stream is released once that work is done
-    void* bufs[] = {c->d_w61, c->d_w31, c->d_status, c->d_digits, c->d_test, c->d_carries, c->d_za, c->d_zb,
-                    c->d_canon, c->d_norm, c->d_flags, c->d_aux, c->d_flow};
     if (c->stream)
-        for (void* b : bufs) if (b) cudaFreeAsync(b, c->stream);
+        for (void* b : {c->d_slab, c->d_read}) if (b) cudaFreeAsync(b, c->stream);
     for (cudaGraphExec_t g : c->graph)
         if (g) cudaGraphExecDestroy(g);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -935,13 +972,17 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         if (p[i] < 3 || mode < M2_MODE_LL || mode > M2_MODE_PRP3) return M2_EINVAL;
         if (m2::transform_log2(p[i]) > 14) return M2_EUNSUPPORTED;   // h <= 8192
         Item it;
-        it.idx = i; it.L = m2::make_layout(p[i]); it.mode = mode;
+        it.idx = i; it.L = m2::make_layout(p[i], 92, 0); it.mode = mode;
         it.iters = iters ? iters[i] : total_iters_for(p[i], mode);
         it.span = m2::carry_span(it.L);
         buckets[it.L.h].push_back(std::move(it));
     }
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // device memory from the stream-ordered pool: a call neither waits for nor
+    // holds up other work on the device
+    cudaMemPool_t mp = ctx_pool(device);
+    if (!mp) return M2_ECUDA;
     struct Dev {
         std::vector<void*> allocs;
         std::vector<cudaStream_t> streams;
@@ -949,81 +990,97 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         ~Dev() {
+            if (!streams.empty() && streams[0])
+                for (auto a : allocs) cudaFreeAsync(a, streams[0]);
             if (exec) cudaGraphExecDestroy(exec);
             if (graph) cudaGraphDestroy(graph);
-            for (auto e : events) cudaEventDestroy(e);
-            for (auto s : streams) cudaStreamDestroy(s);
-            for (auto a : allocs) cudaFree(a);
+            for (auto e : events) if (e) cudaEventDestroy(e);
+            for (auto s : streams) if (s) cudaStreamDestroy(s);
         }
     } dv;
+    const size_t nb = buckets.size();
+    dv.streams.resize(nb + 1, nullptr);
+    for (auto& s : dv.streams) if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return M2_ECUDA;
+    dv.events.resize(nb + 3, nullptr);
+    for (size_t i = 0; i < dv.events.size(); ++i)
+        if (cudaEventCreateWithFlags(&dv.events[i], i == 1 || i == 2 ? cudaEventDefault : cudaEventDisableTiming) != cudaSuccess) return M2_ECUDA;
+    cudaStream_t s0 = dv.streams[0];
     auto dmal = [&](void** ptr, size_t bytes) -> int {
-        if (cudaMalloc(ptr, bytes) != cudaSuccess) { cudaGetLastError(); return M2_ENOMEM; }
+        if (cudaMallocFromPoolAsync(ptr, bytes, mp, s0) != cudaSuccess) { cudaGetLastError(); return M2_ENOMEM; }
         dv.allocs.push_back(*ptr);
         return M2_OK;
     };
-    struct Launch { u64 h; int threads; int ntests; int grid; m2k::SmallTest* d_tests; int* d_queue; long long* d_dig; std::vector<Item>* items; bool fuse; };
+    // test descriptors, results and one {queue, status} pair per bucket, in bucket order
+    int rc;
+    m2k::SmallTest* d_all = nullptr; m2k::TestInit* d_init = nullptr; unsigned long long* d_res = nullptr; int *d_prime = nullptr, *d_q = nullptr;
+    if ((rc = dmal((void**)&d_all, count * sizeof(m2k::SmallTest))) || (rc = dmal((void**)&d_init, count * sizeof(m2k::TestInit))) ||
+        (rc = dmal((void**)&d_res, count * sizeof(u64))) || (rc = dmal((void**)&d_prime, count * sizeof(int))) ||
+        (rc = dmal((void**)&d_q, 2 * nb * sizeof(int))))
+        return rc;
+    struct Launch { u64 h; int ln, threads, ntests, grid; size_t first; long long* d_dig; std::vector<Item>* items; bool fuse; };
     std::vector<Launch> launches;
+    std::vector<m2k::SmallTest> tests(count);
+    std::vector<m2k::TestInit> init(count);
     uint64_t squarings = 0;
+    size_t first = 0;
     for (auto& kv : buckets) {
-        const u64 h = kv.first;
+        const u64 h = kv.first, n = 2 * h;
         std::vector<Item>& items = kv.second;
         std::sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.iters > b.iters; });
-        const u64 n = 2 * h;
         const size_t nt = items.size();
         TwTables tw;
-        int rc = get_twiddles(device, h, tw);
-        if (rc) return rc;
-        long long* d_dig = nullptr; unsigned char* d_w = nullptr; m2k::SmallTest* d_tests = nullptr; int* d_q = nullptr;
-        if ((rc = dmal((void**)&d_dig, nt * n * sizeof(i64))) || (rc = dmal((void**)&d_w, nt * n * 2)) ||
-            (rc = dmal((void**)&d_tests, nt * sizeof(m2k::SmallTest))) || (rc = dmal((void**)&d_q, 2 * sizeof(int))))
-            return rc;
-        int threads = m2k::small_threads_for((unsigned)h);
-        std::vector<i64> dig(nt * n);
-        std::vector<unsigned char> w(nt * n * 2);
-        std::vector<m2k::SmallTest> tests(nt);
+        if ((rc = get_twiddles(device, h, tw))) return rc;
+        long long* d_dig = nullptr; unsigned char* d_w = nullptr;
+        if ((rc = dmal((void**)&d_dig, nt * n * sizeof(i64))) || (rc = dmal((void**)&d_w, nt * n * 2))) return rc;
         for (size_t t = 0; t < nt; ++t) {
             const Item& it = items[t];
-            std::vector<i64> b = m2::balanced_digits(it.L, m2::digits_of_small(it.L, it.mode == M2_MODE_LL ? 4 : 3));
-            std::copy(b.begin(), b.end(), dig.begin() + t * n);
-            std::copy(it.L.w61.begin(), it.L.w61.end(), w.begin() + t * 2 * n);
-            std::copy(it.L.w31.begin(), it.L.w31.end(), w.begin() + t * 2 * n + n);
-            m2k::SmallTest& T = tests[t];
+            m2k::SmallTest& T = tests[first + t];
             T.digits = d_dig + t * n; T.w61 = d_w + t * 2 * n; T.w31 = d_w + t * 2 * n + n;
-            T.tw4 = tw.tw4; T.tc = tw.tc; T.status = d_q + 1;
+            T.tw4 = tw.tw4; T.tc = tw.tc; T.status = d_q + 2 * launches.size() + 1;
             T.p = it.L.p; T.iters = it.iters; T.ln = it.L.ln; T.mode = it.mode; T.span = it.span;
-            T.carry_threads = small_carry_threads(it.L, it.span, threads);
+            T.carry_threads = small_carry_threads(it.L, it.span, m2k::small_threads_for((unsigned)h));
+            T.gf61_only = 0; T.fuse_middle = 0;
+            const u64 x0 = it.mode == M2_MODE_LL ? 4 : 3;
+            const bool host_state = it.L.q < 4;   // tiny: the first digit may not hold x0
+            init[first + t] = m2k::TestInit{d_w + t * 2 * n, d_w + t * 2 * n + n, nullptr, host_state ? nullptr : T.digits, (long long)x0, it.L.p, it.L.ln};
+            if (host_state) {
+                const m2::Layout L = m2::make_layout(it.L.p);
+                const std::vector<i64> b = m2::balanced_digits(L, m2::digits_of_small(L, x0));
+                if (cudaMemcpyAsync(T.digits, b.data(), n * sizeof(i64), cudaMemcpyHostToDevice, s0) != cudaSuccess) return M2_ECUDA;
+            }
             squarings += it.iters;
         }
-        if (cudaMemcpy(d_dig, dig.data(), dig.size() * sizeof(i64), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(d_w, w.data(), w.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            return M2_ECUDA;
-        Tuned tn;
-        if ((rc = tune_bucket(device, h, items, tests, d_dig, sms, tn))) return rc;
-        threads = tn.threads;
-        for (size_t t = 0; t < nt; ++t) {
-            tests[t].carry_threads = small_carry_threads(items[t].L, items[t].span, threads, tn.carry_shift);
-            tests[t].fuse_middle = tn.fuse;
-        }
-        if (cudaMemcpy(d_tests, tests.data(), tests.size() * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemset(d_q, 0, 2 * sizeof(int)) != cudaSuccess)
-            return M2_ECUDA;
-        const int per_sm = m2k::small_ctas_per_sm((unsigned)h, threads, tn.fuse != 0);
-        const int grid = (int)std::min<size_t>(nt, (size_t)per_sm * (size_t)std::max(sms, 1));
-        launches.push_back(Launch{h, threads, (int)nt, grid, d_tests, d_q, d_dig, &items, tn.fuse != 0});
+        launches.push_back(Launch{h, items[0].L.ln, 0, (int)nt, 0, first, d_dig, &items, false});
+        first += nt;
     }
+    cudaError_t e = cudaMemsetAsync(d_q, 0, 2 * nb * sizeof(int), s0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_init, init.data(), count * sizeof(m2k::TestInit), cudaMemcpyHostToDevice, s0);
+    if (e == cudaSuccess) e = m2k::launch_test_init(d_init, (int)count, s0);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s0);   // the tuner reads the start states on a stream of its own
+    if (e != cudaSuccess) return fail_cuda("batch setup", e);
+    for (Launch& l : launches) {
+        std::vector<Item>& items = *l.items;
+        Tuned tn;
+        const std::vector<m2k::SmallTest> mine(tests.begin() + l.first, tests.begin() + l.first + l.ntests);
+        if ((rc = tune_bucket(device, l.h, items, mine, l.d_dig, sms, tn))) return rc;
+        l.threads = tn.threads;
+        l.fuse = tn.fuse != 0;
+        for (int t = 0; t < l.ntests; ++t) {
+            tests[l.first + t].carry_threads = small_carry_threads(items[t].L, items[t].span, tn.threads, tn.carry_shift);
+            tests[l.first + t].fuse_middle = tn.fuse;
+        }
+        const int per_sm = m2k::small_ctas_per_sm((unsigned)l.h, l.threads, l.fuse);
+        l.grid = (int)std::min<size_t>((size_t)l.ntests, (size_t)per_sm * (size_t)std::max(sms, 1));
+    }
+    if (cudaMemcpyAsync(d_all, tests.data(), count * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, s0) != cudaSuccess) return M2_ECUDA;
     // capture: fork from stream 0 to one stream per bucket, join back
-    dv.streams.resize(launches.size() + 1);
-    for (auto& s : dv.streams) if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return M2_ECUDA;
-    dv.events.resize(launches.size() + 3);
-    for (auto& e : dv.events) if (cudaEventCreate(&e) != cudaSuccess) return M2_ECUDA;
-    cudaStream_t s0 = dv.streams[0];
     if (cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return M2_ECUDA;
     cudaEventRecord(dv.events[0], s0);
     for (size_t b = 0; b < launches.size(); ++b) {
         cudaStream_t sb = dv.streams[b + 1];
         cudaStreamWaitEvent(sb, dv.events[0], 0);
         const Launch& l = launches[b];
-        m2k::launch_small_persistent(l.d_tests, l.ntests, (unsigned)l.h, l.threads, l.d_queue, l.grid, sb, l.fuse);
+        m2k::launch_small_persistent(d_all + l.first, l.ntests, (unsigned)l.h, l.threads, d_q + 2 * b, l.grid, sb, l.fuse);
         cudaEventRecord(dv.events[b + 3], sb);
         cudaStreamWaitEvent(s0, dv.events[b + 3], 0);
     }
@@ -1033,27 +1090,25 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
     cudaEventRecord(t0, s0);
     if (cudaGraphLaunch(dv.exec, s0) != cudaSuccess) return M2_ECUDA;
     cudaEventRecord(t1, s0);
-    if (cudaStreamSynchronize(s0) != cudaSuccess) return M2_ECUDA;
+    for (const Launch& l : launches)
+        if (e == cudaSuccess) e = m2k::launch_results(d_all + l.first, l.ntests, l.ln, d_res + l.first, d_prime + l.first, s0);
+    std::vector<u64> res(count);
+    std::vector<int> prime(count), q(2 * nb);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(res.data(), d_res, count * sizeof(u64), cudaMemcpyDeviceToHost, s0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(prime.data(), d_prime, count * sizeof(int), cudaMemcpyDeviceToHost, s0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(q.data(), d_q, 2 * nb * sizeof(int), cudaMemcpyDeviceToHost, s0);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
+    if (e != cudaSuccess) return fail_cuda("batch run", e);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, t0, t1);
     int status_any = 0;
-    for (const Launch& l : launches) {
-        int st = 0;
-        if (cudaMemcpy(&st, l.d_queue + 1, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return M2_ECUDA;
-        status_any |= st;
-        const u64 n = 2 * l.h;
-        std::vector<i64> dig((size_t)l.ntests * n);
-        if (cudaMemcpy(dig.data(), l.d_dig, dig.size() * sizeof(i64), cudaMemcpyDeviceToHost) != cudaSuccess) return M2_ECUDA;
+    for (size_t b = 0; b < launches.size(); ++b) {
+        status_any |= q[2 * b + 1];
+        const Launch& l = launches[b];
         for (int t = 0; t < l.ntests; ++t) {
             const Item& it = (*l.items)[t];
-            std::vector<i64> d(dig.begin() + (size_t)t * n, dig.begin() + (size_t)(t + 1) * n);
-            std::vector<u64> canon;
-            try { canon = m2::canonical_digits(it.L, d, {}, 0); } catch (const std::exception&) { return M2_ESTATE; }
-            if (res64_out) res64_out[it.idx] = m2::res64_of(it.L, canon);
-            if (is_prime_out) {
-                const u64 want = it.mode == M2_MODE_LL ? 0 : (it.mode == M2_MODE_PRP ? 9 : 3);
-                is_prime_out[it.idx] = m2::equals_small(it.L, canon, want) ? 1 : 0;
-            }
+            if (res64_out) res64_out[it.idx] = res[l.first + t];
+            if (is_prime_out) is_prime_out[it.idx] = prime[l.first + t];
         }
     }
     if (stats) {
@@ -1124,6 +1179,11 @@ struct m2_server {
     uint64_t next_key = 0;
     std::deque<m2_srv_result> finished;
     std::map<u64, SrvBucket> buckets;
+    // the one-CTA tests' contexts share a stream (they only set up and read
+    // back on it; their squarings run in the buckets' launches, which wait for
+    // small_ready): a stream per test makes every allocation slower
+    cudaStream_t small_stream = nullptr;
+    cudaEvent_t small_ready = nullptr;
     uint64_t resident = 0, squarings = 0, completed = 0;
     uint32_t steps = 0, launches = 0;
     std::chrono::steady_clock::time_point t0;
@@ -1222,7 +1282,8 @@ int srv_launch(m2_server* s) {
             t.status = b.d_status + j;
             b.h_tests[j] = t;
         }
-        cudaError_t e = cudaMemsetAsync(b.d_status, 0, cnt * sizeof(int), b.stream);
+        cudaError_t e = cudaStreamWaitEvent(b.stream, s->small_ready, 0);
+        if (e == cudaSuccess) e = cudaMemsetAsync(b.d_status, 0, cnt * sizeof(int), b.stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b.d_tests, b.h_tests, cnt * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, b.stream);
         if (e != cudaSuccess) return fail_cuda("server descriptor upload", e);
         if ((e = m2k::launch_small(b.d_tests, (int)cnt, (unsigned)kv.first, threads, 0u, b.stream, fuse)) != cudaSuccess)
@@ -1291,6 +1352,11 @@ int m2_srv_create(m2_server** out, int device, uint64_t budget_bytes, uint32_t q
     s->device = device;
     s->budget = budget_bytes;
     s->quantum = quantum ? quantum : 1000;
+    if (cudaStreamCreateWithFlags(&s->small_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->small_ready, cudaEventDisableTiming) != cudaSuccess) {
+        m2_srv_destroy(s);
+        return M2_ECUDA;
+    }
     s->t0 = std::chrono::steady_clock::now();
     *out = s;
     return M2_OK;
@@ -1321,6 +1387,7 @@ int m2_srv_step(m2_server* s) {
         o.device = s->device;
         // up to h = 8192 a test joins its size's shared one-CTA launch
         o.path = (m2::transform_log2(it.p) <= 14) ? M2_PATH_SMALL : M2_PATH_LARGE;
+        if (o.path == M2_PATH_SMALL) o.stream = s->small_stream;
         const int rc = m2_create(&it.ctx, it.p, it.mode, &o);
         it.t_admit = s->now();
         s->resident += it.bytes;
@@ -1338,6 +1405,8 @@ int m2_srv_step(m2_server* s) {
     }
     if (s->active.empty()) return M2_OK;
     s->steps++;
+    const cudaError_t er = cudaEventRecord(s->small_ready, s->small_stream);
+    if (er != cudaSuccess) return fail_cuda("server setup event", er);
     int rc = srv_launch(s);
     if (rc) return rc;
     // wait until a lane finishes (polling; bounded)
@@ -1407,6 +1476,8 @@ void m2_srv_destroy(m2_server* s) {
         if (b.ev) cudaEventDestroy(b.ev);
         if (b.stream) cudaStreamDestroy(b.stream);
     }
+    if (s->small_ready) cudaEventDestroy(s->small_ready);
+    if (s->small_stream) cudaStreamDestroy(s->small_stream);
     delete s;
 }
 

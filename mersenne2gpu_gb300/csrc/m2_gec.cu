@@ -13,7 +13,7 @@
 // and the relation d_t = x_k0 d_(t-1)^(2^B) becomes
 //   D_t = Z 4^((t-1)(1 - 2^B)),  Z = 4 x_k0 D_(t-1)^(2^B),
 // where Z is formed by the same product and the power of two is a rotation of
-// the p-bit residue (2^p == 1), applied on the host once per verification.
+// the p-bit residue (2^p == 1), applied once per verification (k_gec_rotate).
 // The block products are enqueued without a host wait: the context's stream
 // hands the boundary state to the second context's stream through an event,
 // and waits for the product through another before its next squaring.
@@ -24,7 +24,7 @@
 #include <algorithm>
 #include <chrono>
 #include <new>
-#include <vector>
+#include <utility>
 
 namespace {
 
@@ -50,42 +50,29 @@ __global__ void k_gec_diff(const ull* __restrict__ a, const ull* __restrict__ b,
     if (c) atomicAdd(count, c);
 }
 
-inline u32 grid_for(ull n) { return (u32)std::min<ull>((n + 255) / 256, 152ull * 8); }
-
-inline ull mask_of(u32 w) { return w >= 64 ? ~0ull : (1ull << w) - 1; }
-
-// v <- v * 2^e mod 2^p - 1 for canonical v (host): bit i of the result is bit
-// (i - e) mod p of v
-void rotate_up(const m2::Layout& L, std::vector<uint64_t>& v, uint64_t e) {
-    const uint64_t p = L.p;
-    e %= p;
-    if (e == 0) return;
-    const uint64_t r = p - e;   // source bit of result bit i: (i + r) mod p
-    std::vector<uint64_t> bits(p / 64 + 2, 0);
-    for (uint64_t j = 0; j < L.n; ++j) {
-        const uint64_t pos = L.bitpos[j], w = L.width[j];
-        if (w == 0 || v[j] == 0) continue;
-        const uint64_t k = pos >> 6, off = pos & 63;
-        bits[k] |= v[j] << off;
-        if (off + w > 64) bits[k + 1] |= v[j] >> (64 - off);
-    }
-    auto get = [&](uint64_t pos, uint64_t len) -> uint64_t {   // len <= 64, pos + len <= p
-        if (len == 0) return 0;
-        const uint64_t k = pos >> 6, off = pos & 63;
-        uint64_t x = bits[k] >> off;
-        if (off + len > 64) x |= bits[k + 1] << (64 - off);
-        return x & mask_of((u32)len);
-    };
-    for (uint64_t j = 0; j < L.n; ++j) {
-        const uint64_t w = L.width[j], pos = (L.bitpos[j] + r) % p;
-        if (pos + w <= p) {
-            v[j] = get(pos, w);
-        } else {
-            const uint64_t lo = p - pos;
-            v[j] = get(pos, lo) | (get(0, w - lo) << lo);
+// out = v * 2^e mod 2^p - 1 for canonical v, as a rotation of the p-bit
+// residue: bit i of the result is bit (i + r) mod p of v, r = p - e mod p.
+// Digit j gathers its bits from the one to three digits of v they lie in.
+__global__ void k_gec_rotate(const ull* __restrict__ v, ull* __restrict__ out, ull r, ull p, int ln, ull n) {
+    for (ull j = blockIdx.x * (ull)blockDim.x + threadIdx.x; j < n; j += (ull)gridDim.x * blockDim.x) {
+        const ull pos = bitpos_at(p, ln, j);
+        const u32 w = (u32)(bitpos_at(p, ln, j + 1) - pos);
+        ull s = pos + r, x = 0;
+        if (s >= p) s -= p;
+        for (u32 got = 0; got < w;) {
+            const ull i = (s << ln) / p;                  // the digit of bit s: bitpos(i) <= s < bitpos(i + 1)
+            const ull b0 = bitpos_at(p, ln, i);
+            const u32 avail = (u32)(bitpos_at(p, ln, i + 1) - s), take = min(avail, w - got);
+            x |= ((v[i] >> (s - b0)) & ((1ull << take) - 1)) << got;
+            got += take;
+            s += take;
+            if (s == p) s = 0;
         }
+        out[j] = x;
     }
 }
+
+inline u32 grid_for(ull n) { return (u32)std::min<ull>((n + 255) / 256, 152ull * 8); }
 
 uint64_t pow2_mod(uint64_t e, uint64_t m) {
     uint64_t r = 1 % m, b = 2 % m;
@@ -108,6 +95,7 @@ struct m2_gec {
     u32 t = 0;                      // products taken since k0
     cudaStream_t cs = nullptr, as = nullptr;     // ctx's and aux's streams
     cudaEvent_t to_aux = nullptr, to_ctx = nullptr;
+    ull* mem = nullptr;             // the allocation that holds them
     // device vectors of n canonical digits
     ull* x0 = nullptr;              // x_k0
     ull* D = nullptr;               // D_t
@@ -198,9 +186,7 @@ int restart(m2_gec* g) {
 int set_device(const m2_gec* g) { return cuda_rc(cudaSetDevice(m2i::creation_opts(g->ctx).device)); }
 
 void release(m2_gec* g) {
-    ull* bufs[] = {g->x0, g->D, g->Dprev, g->xb, g->sq, g->tmp};
-    for (ull* b : bufs) if (b) cudaFree(b);
-    if (g->count) cudaFree(g->count);
+    if (g->mem) cudaFree(g->mem);
     if (g->to_aux) cudaEventDestroy(g->to_aux);
     if (g->to_ctx) cudaEventDestroy(g->to_ctx);
     m2_destroy(g->aux);
@@ -229,11 +215,14 @@ int m2_gec_create(m2_gec** out, m2_ctx* ctx, uint32_t block) {
     if ((rc = m2_create(&g->aux, info.p, M2_MODE_PRP, &o))) { delete g; return rc; }
     g->as = m2i::stream(g->aux);
     const size_t bytes = g->L->n * sizeof(ull);
-    ull** bufs[] = {&g->x0, &g->D, &g->Dprev, &g->xb, &g->sq, &g->tmp};
+    // one allocation: the six vectors, then the counter
     rc = set_device(g);
-    for (ull** b : bufs)
-        if (!rc) rc = cuda_rc(cudaMalloc(b, bytes));
-    if (!rc) rc = cuda_rc(cudaMalloc(&g->count, sizeof(unsigned)));
+    if (!rc) rc = cuda_rc(cudaMalloc((void**)&g->mem, 6 * bytes + sizeof(unsigned)));
+    ull** bufs[] = {&g->x0, &g->D, &g->Dprev, &g->xb, &g->sq, &g->tmp};
+    if (!rc) {
+        for (int i = 0; i < 6; ++i) *bufs[i] = g->mem + i * g->L->n;
+        g->count = reinterpret_cast<unsigned*>(g->mem + 6 * g->L->n);
+    }
     if (!rc) rc = cuda_rc(cudaEventCreateWithFlags(&g->to_aux, cudaEventDisableTiming));
     if (!rc) rc = cuda_rc(cudaEventCreateWithFlags(&g->to_ctx, cudaEventDisableTiming));
     if (!rc) rc = ctx_state(g, g->x0);
@@ -302,22 +291,16 @@ int m2_gec_check(m2_gec* g, uint32_t* verified_iter) {
             rc = square_k(g, g->Dprev, g->block, &c);
             if (!rc) rc = cuda_rc(cudaMemcpyAsync(g->tmp, c, bytes, cudaMemcpyDeviceToDevice, g->as));
             if (!rc) rc = mul4(g, g->tmp, g->x0, g->Dprev);   // D_(t-1) is not needed afterwards
-            std::vector<uint64_t> z, d;
-            try {
-                z.resize(L.n);
-                d.resize(L.n);
-            } catch (const std::bad_alloc&) {
-                rc = M2_ENOMEM;
-            }
-            if (!rc) rc = cuda_rc(cudaMemcpyAsync(z.data(), g->Dprev, bytes, cudaMemcpyDeviceToHost, g->as));
-            if (!rc) rc = cuda_rc(cudaMemcpyAsync(d.data(), g->D, bytes, cudaMemcpyDeviceToHost, g->as));
-            if (!rc) rc = cuda_rc(cudaStreamSynchronize(g->as));
             if (!rc) {
                 const uint64_t p = L.p;
-                const uint64_t f = (1 + p - pow2_mod(g->block, p)) % p;          // 1 - 2^B mod p
-                rotate_up(L, z, 2 * ((uint64_t)(g->t - 1) % p * f % p) % p);     // 4^((t-1)(1 - 2^B))
-                ok = (z == d);
+                const uint64_t f = (1 + p - pow2_mod(g->block, p)) % p;                // 1 - 2^B mod p
+                const uint64_t e = 2 * ((uint64_t)(g->t - 1) % p * f % p) % p;         // 4^((t-1)(1 - 2^B))
+                k_gec_rotate<<<grid_for(L.n), 256, 0, g->as>>>(g->Dprev, g->sq, e ? p - e : 0, p, L.ln, L.n);
+                rc = cuda_rc(cudaGetLastError());
             }
+            unsigned diff = 0;
+            if (!rc) rc = count_diff(g, g->D, g->sq, &diff);
+            if (!rc) ok = diff == 0;
         }
         if (!rc && ok) {
             // the current state: the last boundary's, or the squarings after

@@ -85,18 +85,6 @@ Dual root_of_unity(u64 order) {
     return Dual{x.a, x.b, y.a, y.b};
 }
 
-static inline Dual dmul(const Dual& x, const Dual& y) {
-    G61 a = mul(G61{x.a, x.b}, G61{y.a, y.b});
-    G31 b = mul(G31{x.c, x.d}, G31{y.c, y.d});
-    return Dual{a.a, a.b, b.a, b.b};
-}
-
-static inline u64 bitrev(u64 i, int bits) {
-    u64 r = 0;
-    for (int k = 0; k < bits; ++k, i >>= 1) r = (r << 1) | (i & 1);
-    return r;
-}
-
 // ---------------- layout ----------------
 int transform_log2(u64 p, int bound) {
     int ln = 2;
@@ -105,68 +93,22 @@ int transform_log2(u64 p, int bound) {
     return ln;
 }
 
-Layout make_layout(u32 p, int bound) {
+Layout make_layout(u32 p, int bound, u64 head) {
     Layout L;
     L.p = p;
     L.ln = transform_log2(p, bound);
     L.n = u64(1) << L.ln;
     L.h = L.n / 2;
     L.q = u32(p >> L.ln);
-    L.width.assign(L.n, 0);
-    L.w61.assign(L.n, 0);
-    L.w31.assign(L.n, 0);
-    L.bitpos.assign(L.n + 1, 0);
-    const u64 n = L.n;
-    // lr = n^-1 mod 61 (resp. 31); 2^60 == 1 mod 61 and 2^30 == 1 mod 31
-    const u64 lr61 = ((u64(1) << 60) / n) % 61, lr31 = ((u64(1) << 30) / n) % 31;
-    for (u64 j = 0; j <= n; ++j) {
+    const u64 n = L.n, m = std::min(n, head);
+    L.width.assign(m, 0);
+    L.bitpos.assign(m + 1, 0);
+    for (u64 j = 0; j <= m; ++j) {
         u64 pj = u64(p) * j;
         L.bitpos[j] = j ? ((pj - 1) >> L.ln) + 1 : 0;         // ceil(p j / n)
         if (j > 0) L.width[j - 1] = uint8_t(L.bitpos[j] - L.bitpos[j - 1]);
-        if (j > 0 && j < n) {
-            u64 r = pj & (n - 1);
-            L.w61[j] = uint8_t((lr61 * (n - r)) % 61);
-            L.w31[j] = uint8_t((lr31 * (n - r)) % 31);
-        }
     }
     return L;
-}
-
-// ---------------- twiddles ----------------
-Twiddles make_twiddles(u64 h) {
-    Twiddles T;
-    int lh = 0;
-    while ((u64(1) << lh) < h) ++lh;
-    // radix-4 steps: S = 1, 4, 16, ... while 4S <= h
-    u64 smax = 0;
-    for (u64 S = 1; 4 * S <= h; S *= 4) smax = S;
-    T.tw4.assign(smax ? 3 * 2 * smax : 3, Dual{0, 0, 0, 0});
-    for (u64 S = 1; 4 * S <= h; S *= 4) {
-        int bits = 0;
-        while ((u64(1) << bits) < S) ++bits;
-        Dual w = root_of_unity(4 * S);
-        std::vector<Dual> pw(S);
-        pw[0] = Dual{1, 0, 1, 0};
-        for (u64 e = 1; e < S; ++e) pw[e] = dmul(pw[e - 1], w);
-        for (u64 j = 0; j < S; ++j) {
-            Dual r = pw[bitrev(j, bits)];
-            Dual r2 = dmul(r, r), r3 = dmul(r2, r);
-            T.tw4[3 * (S + j) + 0] = r;
-            T.tw4[3 * (S + j) + 1] = r2;
-            T.tw4[3 * (S + j) + 2] = r3;
-        }
-    }
-    // centre / radix-2 twiddles: tc[j] = w_h^{br_{h/2}(j)}
-    const u64 hh = std::max<u64>(h / 2, 1);
-    T.tc.assign(hh, Dual{1, 0, 1, 0});
-    if (h >= 2) {
-        Dual w = root_of_unity(h);
-        std::vector<Dual> pw(hh);
-        pw[0] = Dual{1, 0, 1, 0};
-        for (u64 e = 1; e < hh; ++e) pw[e] = dmul(pw[e - 1], w);
-        for (u64 j = 0; j < hh; ++j) T.tc[j] = pw[bitrev(j, lh - 1)];
-    }
-    return T;
 }
 
 int carry_span(const Layout& L) {
@@ -183,17 +125,6 @@ int carry_span(const Layout& L) {
 
 // ---------------- state conversion ----------------
 static std::vector<u64> normalize(const Layout& L, const std::vector<i128>& t);
-
-std::vector<u64> canonical_digits(const Layout& L, const std::vector<i64>& d,
-                                  const std::vector<i64>& carry, u64 seg_digits) {
-    const u64 n = L.n;
-    std::vector<i128> t(n);
-    for (u64 j = 0; j < n; ++j) t[j] = d[j];
-    if (seg_digits) {
-        for (u64 s = 0; s < carry.size(); ++s) t[((s + 1) * seg_digits) % n] += carry[s];
-    }
-    return normalize(L, t);
-}
 
 std::vector<u64> canonical_from_unsigned(const Layout& L, const u64* d) {
     std::vector<i128> t(L.n);
@@ -257,17 +188,6 @@ std::vector<u64> digits_of_small(const Layout& L, u64 x) {
         x = (w >= 64) ? 0 : (x >> w);
     }
     return out;
-}
-
-u64 res64_of(const Layout& L, const std::vector<u64>& canon) {
-    u64 r = 0;
-    for (u64 j = 0; j < L.n && L.bitpos[j] < 64; ++j) r |= canon[j] << L.bitpos[j];
-    return r;
-}
-
-bool equals_small(const Layout& L, const std::vector<u64>& canon, u64 v) {
-    if (L.p < 64) v %= (u64(1) << L.p) - 1;   // canonical residue of v
-    return digits_of_small(L, v) == canon;
 }
 
 }  // namespace m2

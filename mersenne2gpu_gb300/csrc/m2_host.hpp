@@ -4,7 +4,7 @@
 // reference definitions (mersenne2_gpu.cpp:286-293, 3921-3944) because they
 // define the residue's digit layout, which must be identical for the state to
 // be a drop-in.  The transform itself (generator, twiddle tables, step plan)
-// is this engine's own.
+// is this engine's own; its tables are built on the device (m2_tables.cu).
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -37,48 +37,25 @@ struct Layout {
     int ln = 0;            // log2 n
     u64 n = 0, h = 0;      // real digits, complex elements
     u32 q = 0;             // narrow digit width p >> ln
+    // the first min(n, head) digits of these (make_layout):
     std::vector<uint8_t> width;   // n digit widths, q or q+1
-    std::vector<uint8_t> w61;     // n shifts mod 61
-    std::vector<uint8_t> w31;     // n shifts mod 31
     std::vector<u64> bitpos;      // n+1 bit positions ceil(p j / n)
 };
-Layout make_layout(u32 p, int bound = 92);
+Layout make_layout(u32 p, int bound = 92, u64 head = ~u64(0));
 
 // Roots of unity of this engine: g61 of order 2^62 in GF(P61^2) and g31 of
 // order 2^32 in GF(P31^2), chosen so that the order-4 root is +i.
 Dual root_of_unity(u64 order);       // primitive root of the given power-of-two order
-
-// Twiddle tables for the in-place decimation-in-frequency transform of
-// length h with per-block twiddles (natural order in, bit-reversed out):
-//   tw4[3*(S+j) + a-1] = r^a, r = w_{4S}^{br_S(j)}, for every radix-4 step with
-//                        S blocks before the step (S = 1, 4, 16, ...)
-//   tc[j]              = w_h^{br_{h/2}(j)}, j < h/2: the centre twiddle of
-//                        position 2j; also the radix-2 step's twiddle when
-//                        log2 h is odd.
-struct Twiddles {
-    std::vector<Dual> tw4;   // 3 * (max S of a radix-4 step) * 2 entries
-    std::vector<Dual> tc;    // h/2 entries
-};
-Twiddles make_twiddles(u64 h);
 
 // Bound-driven number of digits through which an incoming segment carry is
 // propagated before its remainder is added to the next digit (see the .cpp).
 int carry_span(const Layout& L);
 
 // ---- state conversion (exact, host side) ----
-// Balanced device state: digits d_j (|d_j| <~ 2^(w_j-1)) and optional pending
-// carries carry[s] that belong at bit position bitpos[seg_start[s+1]] (cyclic).
-// Returns canonical digits in [0, 2^w_j), all-ones (== M_p) mapped to zero.
-std::vector<u64> canonical_digits(const Layout& L, const std::vector<i64>& d,
-                                  const std::vector<i64>& carry, u64 seg_digits);
 // Any n unsigned digit words -> canonical digits of the residue they denote.
 std::vector<u64> canonical_from_unsigned(const Layout& L, const u64* d);
 // Canonical (or any non-negative) digits -> balanced digits of the same residue.
 std::vector<i64> balanced_digits(const Layout& L, const std::vector<u64>& canon);
 // Small integer -> canonical digits.
 std::vector<u64> digits_of_small(const Layout& L, u64 x);
-u64 res64_of(const Layout& L, const std::vector<u64>& canon);
-// Value of canonical digits is exactly `v` (a small integer)?
-bool equals_small(const Layout& L, const std::vector<u64>& canon, u64 v);
-
 }  // namespace m2

@@ -421,19 +421,6 @@ int small_ctas_per_sm(unsigned int h, int threads, bool fuse) {
     return nb > 0 ? nb : 1;
 }
 
-// LargeBufs::aux from the shift tables: the rotations by 2^-(s + ln + 1) that
-// unweight an element's two digits, and the digits' widths
-__global__ void __launch_bounds__(256) k_aux(uint2* aux, const unsigned char* w61, const unsigned char* w31, u32 p, int ln) {
-    const u32 k = blockIdx.x * 256u + threadIdx.x, j = 2 * k;
-    if (j >= (1u << ln)) return;
-    aux[k] = make_uint2(unrot61(w61[j], ln) | (unrot61(w61[j + 1], ln) << 8) | (unrot31(w31[j], ln) << 16) | (unrot31(w31[j + 1], ln) << 24),
-                        width_of(p, ln, j) | (width_of(p, ln, j + 1) << 8));
-}
-cudaError_t launch_aux(uint2* aux, const unsigned char* w61, const unsigned char* w31, u32 p, int ln, cudaStream_t s) {
-    k_aux<<<(unsigned)(((1ull << ln) / 2 + 255) / 256), 256, 0, s>>>(aux, w61, w31, p, ln);
-    return cudaGetLastError();
-}
-
 // =====================================================================
 // three-pass path
 // =====================================================================

@@ -84,6 +84,23 @@ struct FlowArgs {
 constexpr int LARGE_STAGES = 3;
 constexpr int STAGE_MID = 3;   // the fused inverse + forward column pass (k_cols_mid_q)
 
+// ---- tables, start states and batch results (m2_tables.cu) ----
+struct TestInit {
+    unsigned char* w61;
+    unsigned char* w31;
+    uint2* aux;                // LargeBufs::aux, or null
+    long long* digits;         // the start state x0 (a value below 2^(w_0 - 1)), or null
+    long long x0;
+    unsigned int p;
+    int ln;                    // at most 30
+};
+size_t twiddle_entries(unsigned long long h);   // DTw entries of tw4; tc has h / 2
+cudaError_t launch_twiddles(DTw* tw4, DTw* tc, unsigned int h, cudaStream_t s);   // h >= 4
+cudaError_t launch_test_init(const TestInit& T, cudaStream_t s);
+cudaError_t launch_test_init(const TestInit* d_tests, int ntests, cudaStream_t s);
+// low 64 bits and verdict of each test's state (n = 2^ln <= 16384 digits)
+cudaError_t launch_results(const SmallTest* d_tests, int ntests, int ln, unsigned long long* res64, int* prime, cudaStream_t s);
+
 // Throughput of 32x32->64-bit integer multiplies (mul.wide.u32 / mad.wide.u32)
 // on every SM: independent chains, returns products per second.
 double measure_wide_mul_rate(int device);

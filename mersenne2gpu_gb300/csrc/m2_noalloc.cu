@@ -52,44 +52,6 @@ void* g_addr[kMaxDevices] = {};
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 
-__device__ __forceinline__ E dpow(E x, unsigned long long e) {
-    E r{1, 0, 1, 0};
-    while (e) {
-        if (e & 1) r = emul(r, x);
-        x = esqr(x);
-        e >>= 1;
-    }
-    return r;
-}
-__device__ __forceinline__ unsigned brev(unsigned i, int bits) { return bits ? (__brev(i) >> (32 - bits)) : 0u; }
-// tables hold canonical coordinates (products leave up to P61 + 5)
-__device__ __forceinline__ void put_tw(m2k::DTw* t, unsigned i, const E& v) { t[i] = m2k::DTw{fold61(v.a), fold61(v.b), v.c, v.d}; }
-
-// Twiddle and weight tables of this engine, rebuilt on the device:
-//   tw4[3(S+j)+a-1] = r^a with r = w_{4S}^{br_S(j)}, tc[j] = w_h^{br_{h/2}(j)},
-//   w61/w31[j] = n^-1 (n - p j mod n) mod 61 / 31 (shift 0 for j = 0).
-__global__ void k_noalloc_tables(m2k::DTw* tw4, m2k::DTw* tc, unsigned char* w61, unsigned char* w31,
-                                 unsigned h, int lh, unsigned p, int ln, E wh, unsigned lr61, unsigned lr31) {
-    const unsigned n = 2u * h;
-    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const unsigned r = (unsigned)(((unsigned long long)p * t) & (n - 1));
-        w61[t] = t ? (unsigned char)((lr61 * (n - r)) % 61u) : 0;
-        w31[t] = t ? (unsigned char)((lr31 * (n - r)) % 31u) : 0;
-        if (t < h / 2) put_tw(tc, t, dpow(wh, brev(t, lh - 1)));
-        // radix-4 step S owns entries S..2S-1; t in [S, 2S) for exactly one power of two S
-        if (t >= 1 && t < h / 2) {
-            const int sb = 31 - __clz(t);
-            const unsigned S = 1u << sb;
-            if ((sb & 1) == 0 && 4u * S <= h) {
-                const unsigned j = t - S;
-                const E r = dpow(wh, (unsigned long long)(h / (4u * S)) * brev(j, sb));
-                const E r2 = esqr(r), r3 = emul(r2, r);
-                put_tw(tw4, 3u * t, r); put_tw(tw4, 3u * t + 1, r2); put_tw(tw4, 3u * t + 2, r3);
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ unsigned long long bitpos_of(unsigned p, int ln, unsigned long long j) {
     return j ? ((((unsigned long long)p * j) - 1) >> ln) + 1 : 0;
 }
@@ -173,8 +135,6 @@ extern "C" int m2_square_noalloc(uint32_t p, int mode, int64_t* digits, uint32_t
     if (!m2i::plan_large(L, span, 0, P)) return M2_EUNSUPPORTED;
     P.mode = mode;
     const unsigned h = (unsigned)L.h, n = (unsigned)L.n;
-    unsigned smax = 0;
-    for (unsigned S = 1; 4 * S <= h; S *= 4) smax = S;
 
     // carve the scratch
     unsigned char* s = static_cast<unsigned char*>(base);
@@ -183,7 +143,7 @@ extern "C" int m2_square_noalloc(uint32_t p, int mode, int64_t* digits, uint32_t
     auto* za = reinterpret_cast<ulonglong2*>(take(16ull * h));
     auto* zb = reinterpret_cast<uint2*>(take(8ull * h));
     auto* car = reinterpret_cast<long long*>(take(8ull * P.R * P.G));
-    auto* tw4 = reinterpret_cast<m2k::DTw*>(take(sizeof(m2k::DTw) * 3ull * 2 * (smax ? smax : 1)));
+    auto* tw4 = reinterpret_cast<m2k::DTw*>(take(sizeof(m2k::DTw) * m2k::twiddle_entries(h)));
     auto* tc = reinterpret_cast<m2k::DTw*>(take(sizeof(m2k::DTw) * (h / 2)));
     auto* w61 = take(n);
     auto* w31 = take(n);
@@ -191,13 +151,11 @@ extern "C" int m2_square_noalloc(uint32_t p, int mode, int64_t* digits, uint32_t
     if (off > kScratchBytes) return M2_EUNSUPPORTED;
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const m2::Dual wh = m2::root_of_unity(h);
-    const unsigned lr61 = (unsigned)(((1ull << 60) / n) % 61), lr31 = (unsigned)(((1ull << 30) / n) % 31);
-    int lh = 0;
-    while ((1u << lh) < h) ++lh;
     const int threads = 256, blocks = (int)((n + threads - 1) / threads);
-    k_noalloc_tables<<<blocks, threads, 0, st>>>(tw4, tc, w61, w31, h, lh, p, ln, E{wh.a, wh.b, wh.c, wh.d}, lr61, lr31);
-    cudaError_t e = cudaMemsetAsync(car, 0, 8ull * P.R * P.G, st);
+    cudaError_t e = m2k::launch_twiddles(tw4, tc, h, st);
+    if (e == cudaSuccess) e = m2k::launch_test_init(m2k::TestInit{w61, w31, nullptr, nullptr, 0, p, ln}, st);
+    if (e != cudaSuccess) return M2_ECUDA;
+    e = cudaMemsetAsync(car, 0, 8ull * P.R * P.G, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, sizeof(int), st);
     if (e != cudaSuccess) return M2_ECUDA;
     // za is free until the first squaring: it holds the copy the rebalance step reads (8n bytes)
