@@ -130,9 +130,24 @@ template <int LR_, int LB_, int C_> struct Shape {
     static constexpr u32 CTAS = G > R / 2 ? G : R / 2;
     static constexpr u32 SLOTS = UC > UR ? UC : UR;
     static constexpr u32 SMEM = 24 * SLOTS;
+    // barriers of only the warps that share a block: n = 2^18 15.6 -> 15.1 us,
+    // 2^19 30.0 -> 29.0, 2^20 60.9 -> 59.8; with 64 rows (at most four warps a
+    // field, n up to 2^15) one barrier for all was faster (n = 2^12 6.6 against 9.4)
+    static constexpr bool NARROW = R >= 256;
 };
 
 template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+
+// Barrier of the aligned group of at least `d` threads of the field (threads
+// fb, NF in all) that this thread is in: a warp, a quarter, half or all of the
+// field's threads.  bar: the first of the field's seven barriers.
+template <class S> __device__ __forceinline__ void sync_group(u32 d, u32 fb, u32 bar) {
+    constexpr u32 NF = S::NF;
+    if (S::NARROW && d <= 32) __syncwarp();
+    else if (S::NARROW && d <= NF / 4) bar_field<NF / 4>(bar + 3 + fb / (NF / 4));
+    else if (S::NARROW && d <= NF / 2) bar_field<NF / 2>(bar + 1 + fb / (NF / 2));
+    else bar_field<NF>(bar);
+}
 
 // the levels of one CTA's units in one field: each thread runs the butterflies
 // fb, fb + NF, ... of a level
@@ -142,22 +157,24 @@ template <class S, class X> struct Unit {
     const DTw* tw4;
     const DTw* tc;
     u32 fb;            // thread of the field
-    u32 bar;           // barrier of the field's warps
+    u32 bar;           // first barrier of the field's warps
 
     static constexpr u32 IC = (S::NBC + S::NF - 1) / S::NF, IR = (S::NBR + S::NF - 1) / S::NF;
-    __device__ __forceinline__ void sync() const { bar_field<S::NF>(bar); }
+    __device__ __forceinline__ void sync() const { sync_group<S>(S::NF, fb, bar); }
 
-    // One level.  tw, ld, st: twiddles, operands and results of a butterfly by
+    // One level.  group: the threads that wrote what this level reads (the
+    // butterflies of one block of the level above, which are consecutive): the
+    // size of the barrier before it, 0 for none.  tw, ld, st: twiddles, operands and results of a butterfly by
     // its index; op: the level's arithmetic.  With registers to spare the
     // twiddles are fetched before the barrier; with 1024 threads of 64
     // registers the other warps hide them (h = 2^19: 62.3 -> 60.1 us).
     template <u32 ITERS, u32 NB, class TW, class LD, class OP, class ST>
-    __device__ __forceinline__ void level(bool barrier, TW&& tw, LD&& ld, OP&& op, ST&& st) const {
+    __device__ __forceinline__ void level(u32 group, TW&& tw, LD&& ld, OP&& op, ST&& st) const {
         constexpr bool EARLY = S::NT <= 512;
         Tri<X> t;
         const bool on = NB % S::NF == 0 || fb < NB;
         if (EARLY && on) tw(fb, t);
-        if (barrier) sync();
+        if (group) sync_group<S>(group, fb, bar);
         if (!on) return;
         if (ITERS == 1) {
             X x[4];
@@ -184,7 +201,7 @@ template <class S, class X> struct Unit {
 #pragma unroll
         for (int l = 0; l < NL; ++l) {
             const u32 M = S::R >> (2 * l), Q = M / 4;
-            level<IC, S::NBC>(l > 0, [&](u32 b, Tri<X>& t) { if (l > 0) t = ldtri<X>(tw4, (1u << (2 * l)) + b / S::C / Q); },
+            level<IC, S::NBC>(l > 0 ? M * S::C : 0, [&](u32 b, Tri<X>& t) { if (l > 0) t = ldtri<X>(tw4, (1u << (2 * l)) + b / S::C / Q); },
                   [&](u32 b, X (&x)[4]) {
                       const u32 rho = b / S::C, s0 = sw((rho / Q * M + rho % Q) * S::C + b % S::C);
 #pragma unroll
@@ -211,7 +228,7 @@ template <class S, class X> struct Unit {
 #pragma unroll
         for (int l = NL - 1; l >= 0; --l) {
             const u32 M = S::R >> (2 * l), Q = M / 4;
-            level<IC, S::NBC>(true, [&](u32 b, Tri<X>& t) { if (l > 0) t = ldtri<X>(tw4, (1u << (2 * l)) + b / S::C / Q); },
+            level<IC, S::NBC>(l == NL - 1 ? S::NF : Q * S::C, [&](u32 b, Tri<X>& t) { if (l > 0) t = ldtri<X>(tw4, (1u << (2 * l)) + b / S::C / Q); },
                   [&](u32 b, X (&x)[4]) {
                       const u32 rho = b / S::C, cc = b % S::C;
                       if (l == NL - 1) {
@@ -245,7 +262,7 @@ template <class S, class X> struct Unit {
 #pragma unroll
         for (int l = 0; l < NF4; ++l) {
             const u32 M = S::B >> (2 * l), Q = M / 4;
-            level<IR, S::NBR>(true, [&](u32 b, Tri<X>& t) {
+            level<IR, S::NBR>(l > 0 ? M : S::NF, [&](u32 b, Tri<X>& t) {
                       const u32 rho = b % (S::B / 4), trow = b / (S::B / 4) ? t1 : t0;
                       t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + rho / Q);
                   },
@@ -275,7 +292,7 @@ template <class S, class X> struct Unit {
 #pragma unroll
         for (int l = NF4 - 1; l >= 0; --l) {
             const u32 M = S::B >> (2 * l), Q = M / 4;
-            level<IR, S::NBR>(true, [&](u32 b, Tri<X>& t) {
+            level<IR, S::NBR>(l == NF4 - 1 ? S::NF : Q, [&](u32 b, Tri<X>& t) {
                       const u32 rho = b % (S::B / 4), trow = b / (S::B / 4) ? t1 : t0;
                       t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + rho / Q);
                   },
@@ -384,7 +401,7 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
     const bool second = kDual && tid >= S::NF;     // the GF(P31^2) half's warps
     const u32 fb = second ? tid - S::NF : tid;
     Unit<S, X61> ua{za, reinterpret_cast<X61*>(A.za), A.tw4, A.tc, fb, 1};
-    Unit<S, X31> ub{zb, reinterpret_cast<X31*>(A.zb), A.tw4, A.tc, fb, 2};
+    Unit<S, X31> ub{zb, reinterpret_cast<X31*>(A.zb), A.tw4, A.tc, fb, 8};
     const bool has_cols = S::G == S::CTAS || x < S::G, has_rows = S::R / 2 == S::CTAS || x < S::R / 2;
     Wait w{A.status, false};
     const u32 base = has_cols ? A.parity[x] : 0u;  // squarings handed over so far (bit 0); bit 1 never matches a word's tag
