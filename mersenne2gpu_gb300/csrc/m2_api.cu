@@ -155,7 +155,9 @@ struct m2_ctx {
     bool fused = false;        // inverse and next forward column pass as one cooperative launch
     bool gf61 = false;         // GF(P61^2)-only transform (M2_FIELDS_GF61)
     bool flow = false;         // squarings run in the one-launch kernel (m2_flow.cu)
-    bool flow_dirty = false;   // a three-pass stage ran since: element tags to be set again
+    bool cluster = false;      // squarings run in one thread-block cluster (m2_cluster.cu)
+    bool stall = false;        // its next launch waits for a carry that never comes (m2_test_stall_fused)
+    bool staged = false;       // a three-pass stage ran since: pending carries, untagged elements
     m2k::FlowArgs fargs{};
     char* d_flow = nullptr;    // its tagged carries, then its parity words
     // GRAPH_ITERS[i] iterations of the three-pass path captured once and replayed
@@ -246,8 +248,13 @@ bool ensure_graph(m2_ctx* c, int i) {
     return false;
 }
 
-// k squarings of a one-CTA context
-cudaError_t launch_one_cta(m2_ctx* c, uint32_t k) {
+// k squarings of a context whose test one CTA or one cluster runs
+cudaError_t launch_one(m2_ctx* c, uint32_t k) {
+    if (c->cluster) {
+        const bool stall = c->stall;
+        c->stall = false;
+        return m2k::launch_cluster(c->d_test, c->L.ln - 1, k, stall, c->gf61, c->stream);
+    }
     if (c->lane) return m2k::launch_lane(c->d_test, 1, (unsigned)c->L.h, k, c->stream, c->gf61);
     return m2k::launch_small(c->d_test, 1, (unsigned)c->L.h, c->threads, k, c->stream, c->h_test.fuse_middle != 0, c->gf61);
 }
@@ -264,7 +271,6 @@ cudaError_t flow_reset(m2_ctx* c) {
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_zb, 0xff, sizeof(uint2) * c->L.h, c->stream);
     const int lh = c->L.ln - 1;
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flow, 0, 8 * m2k::flow_carry_words(lh) + 4 * m2k::flow_groups(lh), c->stream);
-    if (e == cudaSuccess) c->flow_dirty = false;
     return e;
 }
 
@@ -275,6 +281,7 @@ cudaError_t reset_sync_words(m2_ctx* c) {
     if (c->path == M2_PATH_LARGE) e = cudaMemsetAsync(c->d_carries, 0, sizeof(i64) * (size_t)c->plan.R * c->plan.G, c->stream);
     if (e == cudaSuccess && c->d_flags) e = cudaMemsetAsync(c->d_flags, 0, flags_bytes(c->plan), c->stream);
     if (e == cudaSuccess && c->flow) e = flow_reset(c);
+    if (e == cudaSuccess) c->staged = false;
     return e;
 }
 
@@ -459,9 +466,8 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
     mem.add(&raw->d_digits, n * sizeof(i64));
     const int lh = raw->L.ln - 1;
     size_t cw = 0;
-    if (path == M2_PATH_SMALL) {
-        mem.add(&raw->d_test, sizeof(m2k::SmallTest));
-    } else {
+    mem.add(&raw->d_test, sizeof(m2k::SmallTest));
+    if (path == M2_PATH_LARGE) {
         const m2k::LargePlan& P = raw->plan;
         mem.add(&raw->d_carries, sizeof(i64) * (size_t)P.R * P.G);
         mem.add(&raw->d_za, sizeof(ulonglong2) * h);
@@ -469,7 +475,9 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         mem.add(&raw->d_flags, flags_bytes(P));
         // one launch for all squarings of a call where a shape of that kernel
         // serves the size; M2_PATH_LARGE and a -B hint ask for the three-pass kernels
-        raw->flow = o.path == M2_PATH_AUTO && o.carry_pairs == 0 && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 &&
+        const bool lone = o.path == M2_PATH_AUTO && o.carry_pairs == 0;
+        raw->cluster = lone && m2k::cluster_supported(lh, raw->span, gf61);
+        raw->flow = lone && !raw->cluster && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 &&
                     m2k::flow_setup(lh, gf61) == cudaSuccess;
         cudaGetLastError();
         // the inverse column passes' per-element table
@@ -494,23 +502,12 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
                 ++shift;
             raw->carry_threads = small_carry_threads(raw->L, raw->span, raw->threads, shift);
         }
-        m2k::SmallTest t{};
-        t.digits = raw->d_digits; t.w61 = raw->d_w61; t.w31 = raw->d_w31;
-        t.tw4 = raw->tw.tw4; t.tc = raw->tw.tc; t.status = raw->d_status;
-        t.p = p; t.iters = 0; t.ln = raw->L.ln; t.mode = mode; t.span = raw->span;
-        t.carry_threads = raw->carry_threads;
-        t.fuse_middle = o.fused_middle ? 1 : 0;
-        t.gf61_only = gf61 ? 1 : 0;
-        raw->h_test = t;
-        // a lone small test: one element per thread (M2_PATH_SMALL and the
-        // hints speak of the one-CTA kernel, which the shared launches of
-        // batches and the server run too)
-        raw->lane = o.path == M2_PATH_AUTO && !o.wg && !o.carry_pairs && !o.fused_middle &&
-                    m2k::lane_supported((unsigned)h, raw->span, raw->carry_threads);
-        if (cudaMemcpyAsync(raw->d_test, &raw->h_test, sizeof(t), cudaMemcpyHostToDevice, raw->stream) != cudaSuccess) {
-            m2_destroy(c.release());
-            return M2_ECUDA;
-        }
+        // a lone small test: one element per thread, in a cluster from n = 2^9
+        // on (M2_PATH_SMALL and the hints speak of the one-CTA kernel, which the
+        // shared launches of batches and the server run too)
+        const bool lone = o.path == M2_PATH_AUTO && !o.wg && !o.carry_pairs && !o.fused_middle && raw->carry_threads > 0;
+        raw->cluster = lone && m2k::cluster_supported(lh, raw->span, gf61);
+        raw->lane = lone && !raw->cluster && m2k::lane_supported((unsigned)h, raw->span, raw->carry_threads);
     } else {
         const m2k::LargePlan& P = raw->plan;
         raw->plan.mode = mode;
@@ -530,6 +527,18 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         }
         raw->bufs.ticket = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G);
         raw->bufs.phase = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G + 2);
+    }
+    m2k::SmallTest t{};
+    t.digits = raw->d_digits; t.w61 = raw->d_w61; t.w31 = raw->d_w31;
+    t.tw4 = raw->tw.tw4; t.tc = raw->tw.tc; t.status = raw->d_status;
+    t.p = p; t.iters = 0; t.ln = raw->L.ln; t.mode = mode; t.span = raw->span;
+    t.carry_threads = raw->carry_threads;
+    t.fuse_middle = o.fused_middle ? 1 : 0;
+    t.gf61_only = gf61 ? 1 : 0;
+    raw->h_test = t;
+    if (cudaMemcpyAsync(raw->d_test, &raw->h_test, sizeof(t), cudaMemcpyHostToDevice, raw->stream) != cudaSuccess) {
+        m2_destroy(c.release());
+        return M2_ECUDA;
     }
     raw->bytes += raw->tw.bytes;
     // shifts, unweighting records and the start state x0, built on the device
@@ -553,10 +562,22 @@ int m2_iterate(m2_ctx* c, uint32_t k) {
     if (k == 0) return M2_OK;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     cudaError_t e = cudaSuccess;
-    if (c->path == M2_PATH_SMALL) {
-        e = launch_one_cta(c, k);
+    if (c->staged) {
+        // the one-launch kernel applies pending carries itself and wants its
+        // tags back; the cluster's starts from digits with none
+        if (c->flow) {
+            e = flow_reset(c);
+        } else {
+            m2k::NormArgs a;
+            int rc = device_canonical(c, a);
+            if (!rc) rc = m2i::load_canon(c, c->iteration);
+            if (rc) return rc;
+        }
+        c->staged = false;
+    }
+    if (c->path == M2_PATH_SMALL || c->cluster) {
+        if (e == cudaSuccess) e = launch_one(c, k);
     } else if (c->flow) {
-        if (c->flow_dirty) e = flow_reset(c);
         for (uint32_t left = k; left > 0 && e == cudaSuccess; left -= c->fargs.k) {
             c->fargs.k = std::min(left, FLOW_ITERS);
             e = m2k::launch_flow(c->L.ln - 1, c->gf61, c->fargs, c->stream);
@@ -692,6 +713,7 @@ int m2_carry_normalize(uint32_t p, const int64_t* digits, const int64_t* seg_car
 
 int m2_test_stall_fused(m2_ctx* c) {
     if (!c) return M2_EINVAL;
+    if (c->cluster) { c->stall = true; return M2_OK; }
     if (!c->flow && (!c->fused || !c->d_flags)) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     if (c->flow) {
@@ -714,7 +736,7 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
     if (!c || stage < 0 || stage > 2) return M2_EINVAL;
     if (c->path != M2_PATH_LARGE) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
-    c->flow_dirty = c->flow;
+    c->staged = c->flow || c->cluster;
     cudaError_t e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
     const size_t h = c->L.h;
     if (e == cudaSuccess && za_out) e = cudaMemcpyAsync(za_out, c->d_za, 16 * h, cudaMemcpyDeviceToHost, c->stream);
@@ -767,13 +789,13 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
     } else {
         for (uint32_t i = 0; i < iters; ++i) for (int st = 0; st < m2k::LARGE_STAGES; ++st) seq.push_back(st);
     }
-    c->flow_dirty = c->flow;
+    c->staged = c->flow || c->cluster;
     std::vector<cudaEvent_t> ev(seq.size() + 1);
     for (auto& e : ev) if (cudaEventCreate(&e) != cudaSuccess) return M2_ECUDA;
     cudaError_t err = cudaEventRecord(ev[0], c->stream);
     for (size_t i = 0; i < seq.size() && err == cudaSuccess; ++i) {
         if (seq[i] < 0)
-            err = launch_one_cta(c, iters);
+            err = launch_one(c, iters);
         else err = m2k::launch_large_stage(c->plan, c->bufs, seq[i], c->stream);
         if (err == cudaSuccess) err = cudaEventRecord(ev[i + 1], c->stream);
     }
@@ -811,7 +833,7 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
 
 uint64_t m2_launches_for(m2_ctx* c, uint32_t k) {
     if (!c || k == 0) return 0;
-    if (c->path == M2_PATH_SMALL) return 1ull;
+    if (c->path == M2_PATH_SMALL || c->cluster) return 1ull;
     if (c->flow) return ((uint64_t)k + FLOW_ITERS - 1) / FLOW_ITERS;
     if (!c->fused) return (uint64_t)m2k::LARGE_STAGES * k;
     // graph replays of GRAPH_ITERS[0] then GRAPH_ITERS[1] squarings, then the

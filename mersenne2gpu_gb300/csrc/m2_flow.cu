@@ -77,32 +77,19 @@ template <u32 TAG> __device__ __forceinline__ u32 off_tag(const X31& v) { return
 __device__ __forceinline__ X61 untag(const X61& v) { return X61{v.a & ~(1ull << 63), v.b & ~(1ull << 63)}; }
 __device__ __forceinline__ X31 untag(const X31& v) { return X31{v.c & P31, v.d & P31}; }
 
-// A bounded wait: after the limit (about a second of polls) the status word
-// gets ST_WAIT_TIMEOUT and this thread waits no more in this launch; every
-// other waiter sees the status word and gives up too.
-struct Wait {
-    int* status;
-    bool dead;
-    __device__ __forceinline__ bool again(u32& it) {   // after an unsuccessful poll
-        if (dead) return false;
-        if ((++it & 255u) == 0) {
-            if (*(volatile int*)status & ST_WAIT_TIMEOUT) { dead = true; return false; }
-            if (it > (1u << 21)) { atomicOr(status, ST_WAIT_TIMEOUT); dead = true; return false; }
-        }
-        if (it > 64) __nanosleep(40);
-        return true;
-    }
-};
+// (the warp's active lanes poll together: diverged loops cost the lone warps of
+// the small shapes their branch latency at every poll)
 template <u32 TAG, class X> __device__ __forceinline__ void take4(X (&x)[4], const X* p, u32 stride, Wait& w) {
     u32 it = 0;
+    const u32 lanes = __activemask();
     do {
         u32 off = 0;
 #pragma unroll
         for (int m = 0; m < 4; ++m) x[m] = ld_relaxed(p + (u64)m * stride);
 #pragma unroll
         for (int m = 0; m < 4; ++m) off |= off_tag<TAG>(x[m]);
-        if ((int)off >= 0) break;
-    } while (w.again(it));
+        if (__all_sync(lanes, (int)off >= 0)) break;
+    } while (__any_sync(lanes, w.again(it)));
 #pragma unroll
     for (int m = 0; m < 4; ++m) x[m] = untag(x[m]);
 }
@@ -135,8 +122,6 @@ template <int LR_, int LB_, int C_> struct Shape {
     // field, n up to 2^15) one barrier for all was faster (n = 2^12 6.6 against 9.4)
     static constexpr bool NARROW = R >= 256;
 };
-
-template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
 // Barrier of the aligned group of at least `d` threads of the field (threads
 // fb, NF in all) that this thread is in: a warp, a quarter, half or all of the

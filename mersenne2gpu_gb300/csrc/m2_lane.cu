@@ -1,4 +1,4 @@
-// m2_lane.cu -- k squarings of one small test (n = 32 ... 1024) in one CTA,
+// m2_lane.cu -- k squarings of one small test (n = 32 ... 256) in one CTA,
 // one element of the transform per thread and field.
 //
 // A lone small transform is all latency: the one-CTA kernel of m2_kernels.cu
@@ -19,67 +19,13 @@
 //
 // What bounds it: the serial chain of one thread (eight steps of one product
 // and two add layers at h = 128, the centre, the row stage), about 3400 cycles
-// at h = 128; at h = 512 the SM's integer pipes (32 warps of 64 registers).
-// Measured, us per squaring, one-CTA kernel -> here: n = 2^8 7.64 -> 1.66,
-// 2^9 7.84 -> 3.17, 2^10 8.61 -> 7.35; n = 2^5 0.94.
-#include "m2_split.cuh"
+// at h = 128.  Measured, us per squaring, one-CTA kernel -> here: n = 2^8 7.64
+// -> 1.57; n = 2^5 0.90.
+#include "m2_lane.cuh"
 
 namespace M2K_NS {
 
 namespace {
-
-// sign-selecting add layers: r = partner + (neg ? -own : own)
-struct Sel61 { u64 mask, add; };   // neg: ~own + (4 P61 + 1)
-__device__ __forceinline__ Sel61 sel61(bool neg) { return neg ? Sel61{~0ull, K4_61 + 1} : Sel61{0ull, 0ull}; }
-
-__device__ __forceinline__ X61 xshx(const X61& v, u32 m) {
-    return X61{__shfl_xor_sync(0xffffffffu, v.a, m), __shfl_xor_sync(0xffffffffu, v.b, m)};
-}
-__device__ __forceinline__ X31 xshx(const X31& v, u32 m) {
-    return X31{__shfl_xor_sync(0xffffffffu, v.c, m), __shfl_xor_sync(0xffffffffu, v.d, m)};
-}
-// one layer, not folded: operands below 4 P61, result below 8 P61
-__device__ __forceinline__ X61 layer(const X61& own, u32 lane_mask, bool neg) {
-    const X61 o = xshx(own, lane_mask);
-    const Sel61 s = sel61(neg);
-    return X61{(own.a ^ s.mask) + s.add + o.a, (own.b ^ s.mask) + s.add + o.b};
-}
-__device__ __forceinline__ X31 layer(const X31& own, u32 lane_mask, bool neg) {
-    const X31 o = xshx(own, lane_mask);
-    const u32 m = neg ? P31 : 0u;   // P31 - v is v ^ P31
-    return X31{add31(own.c ^ m, o.c), add31(own.d ^ m, o.d)};
-}
-// the first layer of a step keeps differences below 3 P61 + 8 (offset 2 P61)
-__device__ __forceinline__ X61 layer_first(const X61& own, u32 lane_mask, bool neg) {
-    const X61 o = xshx(own, lane_mask);
-    const u64 mask = neg ? ~0ull : 0ull, add = neg ? K2_61 + 1 : 0ull;
-    return X61{(own.a ^ mask) + add + o.a, (own.b ^ mask) + add + o.b};
-}
-__device__ __forceinline__ X31 layer_first(const X31& own, u32 lane_mask, bool neg) { return layer(own, lane_mask, neg); }
-__device__ __forceinline__ X61 folded(const X61& v) { return X61{fold61(v.a), fold61(v.b)}; }
-__device__ __forceinline__ X31 folded(const X31& v) { return v; }
-// times i (pos) or -i where `on`; GF(P61) operands below 3 P61 + 8
-__device__ __forceinline__ X61 turn(const X61& v, bool on, bool pos) {
-    const u64 n = K4_61 - (pos ? v.b : v.a);
-    return on ? (pos ? X61{n, v.a} : X61{v.b, n}) : v;
-}
-__device__ __forceinline__ X31 turn(const X31& v, bool on, bool pos) {
-    const u32 n = P31 - (pos ? v.d : v.c);
-    return on ? (pos ? X31{n, v.c} : X31{v.d, n}) : v;
-}
-
-// Radix-4 steps on lane bits lb + 1, lb (m = their value): dif4 and dit4 of
-// m2_field.cuh with one element per lane.
-template <class X> __device__ __forceinline__ X step_fwd(X x, u32 lb, u32 m) {
-    x = layer_first(x, 2u << lb, (m & 2u) != 0);        // v0, v1, v2, v3
-    x = turn(x, m == 3u, true);                         // i v3
-    return folded(layer(x, 1u << lb, (m & 1u) != 0));
-}
-template <class X> __device__ __forceinline__ X step_inv(X x, u32 lb, u32 m) {
-    x = layer_first(x, 1u << lb, (m & 1u) != 0);        // x0 + x1, x0 - x1, x2 + x3, x2 - x3
-    x = turn(x, m == 3u, false);                        // -i (x2 - x3)
-    return folded(layer(x, 2u << lb, (m & 2u) != 0));
-}
 
 template <int A> struct Lane {
     static constexpr u32 H = 1u << A, NF = H < 32 ? 32 : H, NT = kDual ? 2 * NF : NF;
@@ -94,8 +40,6 @@ template <int A> struct Lane {
     // slot of element e: both distributions' accesses on distinct bank groups
     static __device__ __forceinline__ u32 slot(u32 e) { return A > 5 ? e ^ ((e >> SH) & 7u) : e; }
 };
-
-template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
 // the transform of one thread in one field
 template <int A, class X> struct Xform {
@@ -117,15 +61,8 @@ template <int A, class X> struct Xform {
         const u32 k = L::e1(t);
         if (k & 1u) ldtw(tr, tc, k >> 1);
         else tr = xone(tr);
-        // the pair's root is at its even position; positions 0 and 1 (roots 1
-        // and -1) are their own mirrors
-        const u32 mk = mirror(k);
-        ldtw(zeta, tc, ((k & 1u) ? mk : k) >> 1);
-        if (k == 1u) zeta = xminus(zeta);
+        zeta = centre_root<X>(tc, k);
     }
-    static __device__ __forceinline__ X61 xminus(const X61&) { return X61{P61 - 1, 0}; }
-    static __device__ __forceinline__ X31 xminus(const X31&) { return X31{P31 - 1, 0}; }
-    static __device__ __forceinline__ u32 mirror(u32 k) { return k < 2 ? k : (3u << (31 - __clz(k))) - k - 1u; }
     __device__ __forceinline__ void sync() const { bar_field<L::NF>(bar); }
 
     // forward transform, centre square, inverse transform: distribution 0 in and out
@@ -157,12 +94,7 @@ template <int A, class X> struct Xform {
         sync();
         {
             const X o = bufb[L::slot(mirror(k))];
-            const bool odd = (k & 1u) != 0 && k != 1u;
-            const X zk = odd ? o : x, zm = odd ? x : o;
-            const X u0 = xaddconj(zk, zm), u1 = xsubconj(zk, zm);
-            const X v0 = xsub(xsqr(u0), xmul(xsqr(u1), zeta));
-            const X v1 = xmul(u0, xadd(u1, u1));
-            x = odd ? xconjsub(v0, v1) : xadd(v0, v1);
+            x = centre_one(x, o, zeta, k);
         }
         if (L::ODD) {
             x = folded(layer_first(x, 1u, (t & 1u) != 0));
@@ -259,9 +191,9 @@ __global__ void __launch_bounds__(Lane<A>::NT, 1) k_lane(const SmallTest* tests,
 
 }  // namespace
 
-// Up to 512 elements: 1024 threads.  n = 2^11 would need two elements a thread,
-// where one CTA is bound by its SM's pipes either way.
-bool lane_supported(unsigned h, int span, int carry_threads) { return h >= 16 && h <= 512 && span == 2 && carry_threads > 0; }
+// From h = 256 on the transform is spread over a cluster (m2_cluster.cu): here
+// h = 256 took 2.98 us a squaring, h = 512 7.0 (1024 threads of 64 registers).
+bool lane_supported(unsigned h, int span, int carry_threads) { return h >= 16 && h <= 128 && span == 2 && carry_threads > 0; }
 
 cudaError_t launch_lane(const SmallTest* d_tests, int ntests, unsigned h, unsigned iters_override, cudaStream_t s, bool gf61) {
 #if M2_DUAL
@@ -269,7 +201,7 @@ cudaError_t launch_lane(const SmallTest* d_tests, int ntests, unsigned h, unsign
 #endif
     switch (h) {
 #define M2_LANE(A) case 1u << A: k_lane<A><<<ntests, Lane<A>::NT, 0, s>>>(d_tests, iters_override); break;
-        M2_LANE(4) M2_LANE(5) M2_LANE(6) M2_LANE(7) M2_LANE(8) M2_LANE(9)
+        M2_LANE(4) M2_LANE(5) M2_LANE(6) M2_LANE(7)
 #undef M2_LANE
         default: return cudaErrorInvalidValue;
     }

@@ -102,6 +102,25 @@ template <class X> __device__ __forceinline__ Tri<X> ldtri(const DTw* tw4, u32 b
 __device__ __forceinline__ X61 weigh61(i64 d0, i64 d1, u32 s) { return X61{rotl61(digit_to61(d0), s & 0xffu), rotl61(digit_to61(d1), (s >> 8) & 0xffu)}; }
 __device__ __forceinline__ X31 weigh31(i64 d0, i64 d1, u32 s) { return X31{rotl31(digit_to31(d0), s & 0xffu), rotl31(digit_to31(d1), (s >> 8) & 0xffu)}; }
 
+// named barrier of N threads
+template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+
+// A bounded wait: after the limit (about a second of polls) the status word
+// gets ST_WAIT_TIMEOUT and this thread waits no more in this launch; every
+// other waiter sees the status word and gives up too.
+struct Wait {
+    int* status;
+    bool dead;
+    __device__ __forceinline__ bool again(u32& it) {   // after an unsuccessful poll
+        if (dead) return false;
+        if ((++it & 255u) == 0) {
+            if (*(volatile int*)status & ST_WAIT_TIMEOUT) { dead = true; return false; }
+            if (it > (1u << 21)) { atomicOr(status, ST_WAIT_TIMEOUT); dead = true; return false; }
+        }
+        if (it > 64) __nanosleep(40);
+        return true;
+    }
+};
 }  // namespace
 
 }  // namespace M2K_NS
