@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <set>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -154,16 +155,22 @@ struct m2_ctx {
     uint2* d_aux = nullptr;    // per-element unweighting rotations and digit widths (m2k::LargeBufs::aux)
     bool fused = false;        // inverse and next forward column pass as one cooperative launch
     bool gf61 = false;         // GF(P61^2)-only transform (M2_FIELDS_GF61)
-    bool flow = false;         // squarings run in the one-launch kernel (m2_flow.cu)
+    bool flow = false;         // squarings run in a one-launch kernel (m2_flow.cu)
+    bool tide = false;         // the one of large sizes (m2_tide.cu)
+    size_t flow_bytes = 0;     // of d_flow
     bool cluster = false;      // squarings run in one thread-block cluster (m2_cluster.cu)
     bool stall = false;        // its next launch waits for a carry that never comes (m2_test_stall_fused)
     bool staged = false;       // a three-pass stage ran since: pending carries, untagged elements
     m2k::FlowArgs fargs{};
-    char* d_flow = nullptr;    // its tagged carries, then its parity words
+    char* d_flow = nullptr;    // its tagged carries, arrival counter and parity words
+    uint2* d_taux = nullptr;   // the large sizes' row-stage tables and parked digits
+    uint32_t* d_tshift = nullptr;
+    longlong2* d_park = nullptr;
     // GRAPH_ITERS[i] iterations of the three-pass path captured once and replayed
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     bool graph_failed = false;
     void* d_slab = nullptr;    // the allocation that holds the buffers above
+    cudaEvent_t gate_ev = nullptr;   // three-pass contexts with waiting kernels: end of the last enqueued run (Gate)
     // canonical digits and carry-propagation scratch (allocated on first read, in d_read)
     void* d_read = nullptr;
     unsigned long long* d_canon = nullptr;
@@ -248,29 +255,20 @@ bool ensure_graph(m2_ctx* c, int i) {
     return false;
 }
 
-// k squarings of a context whose test one CTA or one cluster runs
-cudaError_t launch_one(m2_ctx* c, uint32_t k) {
-    if (c->cluster) {
-        const bool stall = c->stall;
-        c->stall = false;
-        return m2k::launch_cluster(c->d_test, c->L.ln - 1, k, stall, c->gf61, c->stream);
-    }
-    if (c->lane) return m2k::launch_lane(c->d_test, 1, (unsigned)c->L.h, k, c->stream, c->gf61);
-    return m2k::launch_small(c->d_test, 1, (unsigned)c->L.h, c->threads, k, c->stream, c->h_test.fuse_middle != 0, c->gf61);
-}
-
 // Squarings per launch of the one-launch kernel: long enough that a launch's
 // start is nothing (62 ms at n = 2^20), short enough that other contexts'
 // launches get their turn.
 constexpr uint32_t FLOW_ITERS = 1000;
+constexpr uint32_t TIDE_ITERS = 250;
+
+m2k::TideArgs tide_args(const m2_ctx* c) { return m2k::TideArgs{c->fargs, c->d_taux, c->d_tshift, c->d_park}; }
 
 // the one-launch kernel's tags as every launch expects them: all element tags
 // 1, carries of parity 0
 cudaError_t flow_reset(m2_ctx* c) {
     cudaError_t e = cudaMemsetAsync(c->d_za, 0xff, sizeof(ulonglong2) * c->L.h, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_zb, 0xff, sizeof(uint2) * c->L.h, c->stream);
-    const int lh = c->L.ln - 1;
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flow, 0, 8 * m2k::flow_carry_words(lh) + 4 * m2k::flow_groups(lh), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flow, 0, c->flow_bytes, c->stream);
     return e;
 }
 
@@ -393,6 +391,127 @@ int load_canon(m2_ctx* c, uint32_t iteration) {
 }
 }  // namespace m2i
 
+namespace {
+
+// the context's squarings run in a kernel that loops over them itself: one CTA
+// or cluster, or one cooperative launch of many CTAs
+bool own_kernel(const m2_ctx* c) { return c->path == M2_PATH_SMALL || c->cluster || c->flow; }
+const char* own_kernel_name(const m2_ctx* c) {
+    return c->cluster ? "k_cluster" : c->lane ? "k_lane" : c->tide ? "k_tide" : c->flow ? "k_flow" : "k_small";
+}
+uint32_t iters_per_launch(const m2_ctx* c) { return c->tide ? TIDE_ITERS : c->flow ? FLOW_ITERS : ~0u; }
+
+cudaError_t launch_own(m2_ctx* c, uint32_t k) {
+    cudaError_t e = cudaSuccess;
+    const unsigned h = (unsigned)c->L.h;
+    const int lh = c->L.ln - 1;
+    for (uint32_t left = k, now; left > 0 && e == cudaSuccess; left -= now) {
+        now = std::min(left, iters_per_launch(c));
+        c->fargs.k = now;
+        if (c->cluster) {
+            e = m2k::launch_cluster(c->d_test, lh, now, c->stall, c->gf61, c->stream);
+            c->stall = false;
+        } else if (c->lane) {
+            e = m2k::launch_lane(c->d_test, 1, h, now, c->stream, c->gf61);
+        } else if (c->tide) {
+            e = m2k::launch_tide(lh, c->gf61, tide_args(c), c->stream);
+        } else if (c->flow) {
+            e = m2k::launch_flow(lh, c->gf61, c->fargs, c->stream);
+        } else {
+            e = m2k::launch_small(c->d_test, 1, h, c->threads, now, c->stream, c->h_test.fuse_middle != 0, c->gf61);
+        }
+    }
+    return e;
+}
+
+// After a three-pass stage: the one-launch kernel of mid sizes applies pending
+// carries itself and wants its tags back; the others start from digits with
+// none.
+int unstage(m2_ctx* c) {
+    if (!c->staged) return M2_OK;
+    if (c->flow && !c->tide) {
+        const cudaError_t e = flow_reset(c);
+        if (e != cudaSuccess) return fail_cuda("tags", e);
+    } else {
+        m2k::NormArgs a;
+        int rc = device_canonical(c, a);
+        if (!rc) rc = m2i::load_canon(c, c->iteration);
+        if (rc) return rc;
+    }
+    c->staged = false;
+    return M2_OK;
+}
+
+}  // namespace
+
+namespace {
+
+// ---------------- kernels that wait between their CTAs ----------------
+// The one-launch kernels (cooperative, one CTA to an SM) and the fused column
+// pass of the three-pass path (cooperative or by tickets) spin on one another's
+// words.  The hardware starts a cooperative grid's CTAs as SMs come free; while
+// another context's waiting kernels are squeezed onto the few SMs that are left
+// neither gets on, and waits run out.  So the two kinds take turns: a run of
+// either is enqueued behind the runs of the other kind (one-launch runs also
+// behind each other) that contexts of this process have enqueued on the device
+// before it, by events.  Nothing waits on the host, and a context alone pays
+// one event record a call.
+struct Gate {
+    std::mutex mu;
+    cudaEvent_t one_ev = nullptr;          // end of the last one-launch run
+    cudaStream_t one_stream = nullptr;     // its stream
+    std::set<m2_ctx*> passes;              // contexts with a recorded gate_ev
+};
+std::mutex g_gate_mu;
+std::map<int, std::unique_ptr<Gate>> g_gate;
+Gate& gate_of(int device) {
+    std::lock_guard<std::mutex> lk(g_gate_mu);
+    std::unique_ptr<Gate>& g = g_gate[device];
+    if (!g) g.reset(new Gate());
+    return *g;
+}
+
+// Enqueues a run (`enqueue`) of context c in its turn.  A stream under capture
+// is left alone: its graph's runs are the caller's to order.
+template <class F> cudaError_t in_turn(m2_ctx* c, F&& enqueue) {
+    const bool one = c->flow && !c->staged, passes = !one && c->fused;
+    if (!one && !passes) return enqueue();
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return enqueue();
+    }
+    Gate& g = gate_of(c->device);
+    std::lock_guard<std::mutex> lk(g.mu);
+    cudaError_t e = cudaSuccess;
+    if (g.one_stream && g.one_stream != c->stream) e = cudaStreamWaitEvent(c->stream, g.one_ev, 0);
+    if (one) {
+        for (m2_ctx* o : g.passes)
+            if (e == cudaSuccess && o != c) e = cudaStreamWaitEvent(c->stream, o->gate_ev, 0);
+        if (e == cudaSuccess && !g.one_ev) e = cudaEventCreateWithFlags(&g.one_ev, cudaEventDisableTiming);
+    } else if (e == cudaSuccess && !c->gate_ev) {
+        e = cudaEventCreateWithFlags(&c->gate_ev, cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) e = enqueue();
+    const cudaError_t r = e == cudaSuccess ? cudaEventRecord(one ? g.one_ev : c->gate_ev, c->stream) : e;
+    if (r == cudaSuccess) {
+        if (one) g.one_stream = c->stream;
+        else g.passes.insert(c);
+    }
+    return r;
+}
+// a context that goes away: its enqueued work stays in stream order
+void leave_gate(m2_ctx* c) {
+    if (!c->flow && !c->gate_ev) return;
+    Gate& g = gate_of(c->device);
+    std::lock_guard<std::mutex> lk(g.mu);
+    g.passes.erase(c);
+    if (c->gate_ev) cudaEventDestroy(c->gate_ev);
+    c->gate_ev = nullptr;
+}
+
+}  // namespace
+
 extern "C" {
 
 const char* m2_last_error(void) { return g_last_error; }
@@ -477,14 +596,21 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         // serves the size; M2_PATH_LARGE and a -B hint ask for the three-pass kernels
         const bool lone = o.path == M2_PATH_AUTO && o.carry_pairs == 0;
         raw->cluster = lone && m2k::cluster_supported(lh, raw->span, gf61);
-        raw->flow = lone && !raw->cluster && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 &&
-                    m2k::flow_setup(lh, gf61) == cudaSuccess;
+        raw->tide = lone && m2k::tide_supported(lh, raw->span, gf61);
+        raw->flow = raw->tide || (lone && !raw->cluster && raw->span <= 3 && m2k::flow_carry_words(lh) != 0 &&
+                                  m2k::flow_setup(lh, gf61) == cudaSuccess);
         cudaGetLastError();
         // the inverse column passes' per-element table
         if (m2k::cols_q_supported(P) || raw->flow) mem.add(&raw->d_aux, sizeof(uint2) * h);
         if (raw->flow) {
-            cw = m2k::flow_carry_words(lh);
-            mem.add(&raw->d_flow, 8 * cw + 4 * m2k::flow_groups(lh));
+            cw = raw->tide ? m2k::tide_groups(lh) * raw->plan.R : m2k::flow_carry_words(lh);
+            raw->flow_bytes = 8 * (cw + 1) + 4 * (raw->tide ? m2k::tide_groups(lh) : m2k::flow_groups(lh));
+            mem.add(&raw->d_flow, raw->flow_bytes);
+            if (raw->tide) {
+                mem.add(&raw->d_taux, sizeof(uint2) * m2k::tide_records(lh));
+                mem.add(&raw->d_tshift, sizeof(uint32_t) * m2k::tide_records(lh));
+                mem.add(&raw->d_park, sizeof(longlong2) * m2k::tide_parked(lh));
+            }
         }
     }
     if ((rc = mem.alloc(raw, &raw->d_slab))) { m2_destroy(c.release()); return rc; }
@@ -523,7 +649,8 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         if (raw->flow) {
             raw->fargs = m2k::FlowArgs{raw->d_digits, raw->d_carries, raw->d_za, raw->d_zb, raw->d_w61, raw->d_w31, raw->d_aux,
                                        raw->tw.tw4, raw->tw.tc, reinterpret_cast<unsigned long long*>(raw->d_flow),
-                                       reinterpret_cast<unsigned*>(raw->d_flow + 8 * cw), raw->d_status, 0u, 2u * P.C, raw->span, mode};
+                                       reinterpret_cast<unsigned long long*>(raw->d_flow) + cw,
+                                       reinterpret_cast<unsigned*>(raw->d_flow + 8 * (cw + 1)), raw->d_status, 0u, 2u * P.C, raw->span, mode};
         }
         raw->bufs.ticket = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G);
         raw->bufs.phase = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G + 2);
@@ -547,6 +674,7 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
     const bool host_state = raw->L.q < 4;
     e = m2k::launch_test_init(m2k::TestInit{raw->d_w61, raw->d_w31, raw->d_aux, host_state ? nullptr : raw->d_digits, x0, p, raw->L.ln},
                               raw->stream);
+    if (e == cudaSuccess && raw->tide) e = m2k::tide_tables(lh, tide_args(raw), raw->stream);
     if (e == cudaSuccess) e = reset_sync_words(raw);
     if (e != cudaSuccess) { rc = fail_cuda("test setup", e); m2_destroy(c.release()); return rc; }
     if (host_state) {
@@ -561,33 +689,23 @@ int m2_iterate(m2_ctx* c, uint32_t k) {
     if (!c) return M2_EINVAL;
     if (k == 0) return M2_OK;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
+    int rc = unstage(c);
+    if (rc) return rc;
     cudaError_t e = cudaSuccess;
-    if (c->staged) {
-        // the one-launch kernel applies pending carries itself and wants its
-        // tags back; the cluster's starts from digits with none
-        if (c->flow) {
-            e = flow_reset(c);
-        } else {
-            m2k::NormArgs a;
-            int rc = device_canonical(c, a);
-            if (!rc) rc = m2i::load_canon(c, c->iteration);
-            if (rc) return rc;
-        }
-        c->staged = false;
-    }
-    if (c->path == M2_PATH_SMALL || c->cluster) {
-        if (e == cudaSuccess) e = launch_one(c, k);
-    } else if (c->flow) {
-        for (uint32_t left = k; left > 0 && e == cudaSuccess; left -= c->fargs.k) {
-            c->fargs.k = std::min(left, FLOW_ITERS);
-            e = m2k::launch_flow(c->L.ln - 1, c->gf61, c->fargs, c->stream);
-        }
+    if (own_kernel(c)) {
+        e = in_turn(c, [&] { return launch_own(c, k); });
     } else {
-        uint32_t left = k;
-        for (int i = 0; i < 2; ++i)
-            if (left >= GRAPH_ITERS[i] && ensure_graph(c, i))
-                for (; left >= GRAPH_ITERS[i] && e == cudaSuccess; left -= GRAPH_ITERS[i]) e = cudaGraphLaunch(c->graph[i], c->stream);
-        if (left > 0 && e == cudaSuccess) e = m2k::launch_large_run(c->plan, c->bufs, left, c->fused, c->stream);
+        bool ready[2];   // captured before the turn
+        for (int i = 0; i < 2; ++i) ready[i] = k >= GRAPH_ITERS[i] && (i == 0 || k % GRAPH_ITERS[0] >= GRAPH_ITERS[1] || !ready[0]) && ensure_graph(c, i);
+        e = in_turn(c, [&] {
+            cudaError_t r = cudaSuccess;
+            uint32_t left = k;
+            for (int i = 0; i < 2; ++i)
+                if (ready[i])
+                    for (; left >= GRAPH_ITERS[i] && r == cudaSuccess; left -= GRAPH_ITERS[i]) r = cudaGraphLaunch(c->graph[i], c->stream);
+            if (left > 0 && r == cudaSuccess) r = m2k::launch_large_run(c->plan, c->bufs, left, c->fused, c->stream);
+            return r;
+        });
     }
     if (e != cudaSuccess) return fail_cuda("m2_iterate launch", e);
     c->iteration += k;
@@ -737,7 +855,7 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
     if (c->path != M2_PATH_LARGE) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     c->staged = c->flow || c->cluster;
-    cudaError_t e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
+    cudaError_t e = in_turn(c, [&] { return m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream); });
     const size_t h = c->L.h;
     if (e == cudaSuccess && za_out) e = cudaMemcpyAsync(za_out, c->d_za, 16 * h, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess && zb_out) e = cudaMemcpyAsync(zb_out, c->d_zb, 8 * h, cudaMemcpyDeviceToHost, c->stream);
@@ -766,6 +884,7 @@ int m2_info(m2_ctx* c, m2_info_t* info) {
 void m2_destroy(m2_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
+    leave_gate(c);
     // stream-ordered frees: they follow the context's queued work and do not
     // wait for other streams; its stream is released once that work is done
     if (c->stream)
@@ -781,7 +900,8 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     // the launch sequence m2_iterate issues for `iters` squarings, one event after each
     std::vector<int> seq;
-    if (c->path == M2_PATH_SMALL) seq.push_back(-1);
+    if (const int rc = unstage(c)) return rc;
+    if (own_kernel(c)) seq.push_back(-1);
     else if (c->fused) {
         seq = {0, 1};
         for (uint32_t i = 1; i < iters; ++i) { seq.push_back(m2k::STAGE_MID); seq.push_back(1); }
@@ -789,16 +909,17 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
     } else {
         for (uint32_t i = 0; i < iters; ++i) for (int st = 0; st < m2k::LARGE_STAGES; ++st) seq.push_back(st);
     }
-    c->staged = c->flow || c->cluster;
     std::vector<cudaEvent_t> ev(seq.size() + 1);
     for (auto& e : ev) if (cudaEventCreate(&e) != cudaSuccess) return M2_ECUDA;
-    cudaError_t err = cudaEventRecord(ev[0], c->stream);
-    for (size_t i = 0; i < seq.size() && err == cudaSuccess; ++i) {
-        if (seq[i] < 0)
-            err = launch_one(c, iters);
-        else err = m2k::launch_large_stage(c->plan, c->bufs, seq[i], c->stream);
-        if (err == cudaSuccess) err = cudaEventRecord(ev[i + 1], c->stream);
-    }
+    cudaError_t err = in_turn(c, [&] {
+        cudaError_t r = cudaEventRecord(ev[0], c->stream);
+        for (size_t i = 0; i < seq.size() && r == cudaSuccess; ++i) {
+            if (seq[i] < 0) r = launch_own(c, iters);
+            else r = m2k::launch_large_stage(c->plan, c->bufs, seq[i], c->stream);
+            if (r == cudaSuccess) r = cudaEventRecord(ev[i + 1], c->stream);
+        }
+        return r;
+    });
     if (err == cudaSuccess) err = cudaStreamSynchronize(c->stream);
     // per stage (in order of first appearance): total time and launches
     std::vector<int> order;
@@ -820,12 +941,15 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
         const int st = order[i];
         m2_stage_time& o = out[i];
         std::memset(&o, 0, sizeof(o));
-        const char* nm = (st < 0) ? "k_small" : m2k::large_stage_name(st);
+        const char* nm = (st < 0) ? own_kernel_name(c) : m2k::large_stage_name(st);
         std::strncpy(o.name, nm, sizeof(o.name) - 1);
         o.launches = tot[st].second;
         o.ms_per_launch = tot[st].first / (double)o.launches;
         o.iters_per_launch = (st < 0) ? iters : 1u;
-        o.bytes_per_launch = (st < 0) ? 16ull * c->L.n : m2k::large_stage_bytes(c->plan, st);
+        // on chip between squarings (digits in and out), or both hand-overs of
+        // every squaring through global memory
+        o.bytes_per_launch = (st >= 0) ? m2k::large_stage_bytes(c->plan, st)
+                             : c->flow ? (uint64_t)iters * 2 * m2k::large_stage_bytes(c->plan, 1) : 16ull * c->L.n;
     }
     if (n_stages) *n_stages = k;
     return M2_OK;
@@ -833,8 +957,7 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
 
 uint64_t m2_launches_for(m2_ctx* c, uint32_t k) {
     if (!c || k == 0) return 0;
-    if (c->path == M2_PATH_SMALL || c->cluster) return 1ull;
-    if (c->flow) return ((uint64_t)k + FLOW_ITERS - 1) / FLOW_ITERS;
+    if (own_kernel(c)) return ((uint64_t)k - 1) / iters_per_launch(c) + 1;
     if (!c->fused) return (uint64_t)m2k::LARGE_STAGES * k;
     // graph replays of GRAPH_ITERS[0] then GRAPH_ITERS[1] squarings, then the
     // rest in one sequence

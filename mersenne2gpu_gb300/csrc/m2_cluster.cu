@@ -70,11 +70,6 @@ __device__ __forceinline__ void arm(u32 bar, u32 bytes) {
 // The warp's words of this squaring have arrived.  Bounded: after two seconds
 // the status word gets ST_WAIT_TIMEOUT; a warp that has given up, or sees that
 // another has, neither waits, arms nor sends any more in this launch.
-__device__ __forceinline__ u64 now_ns() {
-    u64 t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
 __device__ __forceinline__ bool arrived(u32 bar, u32 parity) {
     u32 done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"

@@ -73,12 +73,22 @@ struct FlowArgs {
     const DTw* tw4;
     const DTw* tc;
     unsigned long long* fcar;  // flow_carry_words tagged segment carries
+    unsigned long long* arrivals;   // CTAs started, over all launches
     unsigned int* parity;      // flow_groups words: squarings done, modulo 2
     int* status;
     unsigned int k;            // squarings of this launch (>= 1)
     unsigned int seg;          // digits per pending carry segment
     int span;                  // at most 3
     int mode;
+};
+// and of the one of large transforms (m2_tide.cu)
+struct TideArgs {
+    FlowArgs f;
+    // aux and the weighting rotations of column c of group g, row r at
+    // (7 g + c) 1024 + r, and where a CTA leaves a group's digits meanwhile
+    const uint2* taux;
+    const unsigned int* tshift;
+    longlong2* park;
 };
 
 constexpr int LARGE_STAGES = 3;

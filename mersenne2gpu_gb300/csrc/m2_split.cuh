@@ -105,6 +105,12 @@ __device__ __forceinline__ X31 weigh31(i64 d0, i64 d1, u32 s) { return X31{rotl3
 // named barrier of N threads
 template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
+__device__ __forceinline__ u64 now_ns() {
+    u64 t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 // A bounded wait: after the limit (about a second of polls) the status word
 // gets ST_WAIT_TIMEOUT and this thread waits no more in this launch; every
 // other waiter sees the status word and gives up too.
@@ -121,6 +127,28 @@ struct Wait {
         return true;
     }
 };
+// Every CTA of a cooperative launch waits here until all of them have started.
+// The hardware may start some while kernels of other streams hold the other
+// SMs, for as long as those keep coming, so this wait has a limit of its own
+// (100 s); the waits after it are between running CTAs.
+__device__ __forceinline__ void all_started(unsigned long long* arrivals, u32 ctas, Wait& w) {
+    __shared__ int gave_up;
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        const u64 old = atomicAdd(arrivals, 1ull), target = (old / ctas + 1) * ctas, t0 = now_ns();
+        while ((i64)(*(volatile u64*)arrivals - target) < 0) {
+            __nanosleep(200);
+            if (now_ns() - t0 > 100000000000ull || (*(volatile int*)w.status & ST_WAIT_TIMEOUT)) {
+                atomicOr(w.status, ST_WAIT_TIMEOUT);
+                gave_up = 1;
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    w.dead = gave_up != 0;
+}
+
 }  // namespace
 
 }  // namespace M2K_NS
