@@ -987,10 +987,12 @@ namespace {
 // combination of threads per transform (32 ... 256), carry segments (threads,
 // threads / 2, threads / 4, each segment at least span + 1 digits) and the
 // fused or separate transform middle runs a GPU-filling sample of the bucket's
-// own tests for TUNE_ITERS squarings on scratch copies of their state; the
-// highest rate of test-squarings per second wins.  Cached for the process.
+// own tests for TUNE_ITERS squarings on scratch copies of their state, and so
+// does m2_duo.cu's kernel where it serves all of them; the highest rate of
+// test-squarings per second wins.  Cached for the process.
 struct Tuned {
     int threads = 0, carry_shift = 0, fuse = 0;
+    bool duo = false;            // the kernel of m2_duo.cu (its middle is fused, its carry has a segment per thread)
     double ns_per_test_iter = 0.0, ns_default = 0.0;
     int carry_blocks(const m2::Layout& L, int span) const { return small_carry_threads(L, span, threads, carry_shift); }
 };
@@ -999,16 +1001,27 @@ std::map<std::pair<int, u64>, Tuned> g_tune;
 std::map<std::pair<int, u64>, std::pair<int, int>> g_tune_shape;   // (device, h) -> (carry blocks, n) of the choice
 constexpr u32 TUNE_ITERS = 48;
 
+// m2_duo.cu's kernel serves these tests of one size (both fields)
+bool duo_for(const std::vector<m2k::SmallTest>& tests) {
+    for (const m2k::SmallTest& t : tests)
+        if (t.gf61_only || !m2k::duo_supported(1u << (t.ln - 1), t.span, t.carry_threads)) return false;
+    return !tests.empty();
+}
+
 template <class Item>
 int tune_bucket(int device, u64 h, const std::vector<Item>& items, const std::vector<m2k::SmallTest>& tests,
-                const long long* d_dig, int sms, Tuned& out) {
+                const long long* d_dig, int sms, size_t total, Tuned& out) {
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune.find({device, h});
         if (it != g_tune.end()) { out = it->second; return M2_OK; }
     }
     const u64 n = 2 * h;
-    const size_t cap = std::min<size_t>(items.size(), (size_t)std::max(sms, 1) * 8);
+    // A batch of at least a test per SM is timed as a full GPU, the bucket's tests
+    // repeated: a last wave that is not full would count against the kernel with
+    // more tests per SM (n = 4096, 498 tests, m2_duo.cu: 143 ns per test-squaring, 118 in full waves).
+    const size_t full = (size_t)std::max(sms, 1) * std::min<size_t>(32, std::max<size_t>(1, 232448 / (24 * h)));
+    const size_t cap = total >= (size_t)sms ? full : items.size();
     long long* scratch = nullptr;
     m2k::SmallTest* d_t = nullptr;
     int* d_st = nullptr;
@@ -1027,43 +1040,82 @@ int tune_bucket(int device, u64 h, const std::vector<Item>& items, const std::ve
         cleanup();
         return M2_ENOMEM;
     }
+    std::vector<m2k::SmallTest> d;
+    // ns per test-squaring of `ns` tests by `launch` (from the bucket's own states)
+    auto rate = [&](size_t ns, auto launch, double& out_ns) {
+        cudaError_t e = cudaSuccess;
+        for (size_t t = 0; t < ns; t += items.size())
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(scratch + t * n, d_dig, std::min(items.size(), ns - t) * n * sizeof(i64), cudaMemcpyDeviceToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d_t, d.data(), ns * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = launch(2u);   // warm-up
+        if (e == cudaSuccess) e = cudaEventRecord(e0, st);
+        if (e == cudaSuccess) e = launch(TUNE_ITERS);
+        if (e == cudaSuccess) e = cudaEventRecord(e1, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        float ms = 0.f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        out_ns = ms * 1e6 / ((double)ns * TUNE_ITERS);
+        return e;
+    };
+    auto sample = [&](int per_sm) {
+        const size_t ns = std::min(cap, (size_t)std::max(per_sm, 1) * (size_t)std::max(sms, 1));
+        d.clear();
+        for (size_t t = 0; t < ns; ++t) {
+            d.push_back(tests[t % tests.size()]);
+            d[t].digits = scratch + t * n;
+            d[t].status = d_st;
+        }
+        return ns;
+    };
     const int T0 = m2k::small_threads_for((unsigned)h);
     Tuned best;
     best.threads = T0;
-    for (int T = 32; T <= 256; T *= 2) {
+    // one combination of the one-CTA kernel
+    auto small_rate = [&](int T, int shift, int fuse) {
+        const size_t ns = sample(m2k::small_ctas_per_sm((unsigned)h, T, fuse != 0));
+        for (size_t t = 0; t < ns; ++t) {
+            const Item& it = items[t % items.size()];
+            d[t].carry_threads = small_carry_threads(it.L, it.span, T, shift);
+            d[t].fuse_middle = fuse;
+        }
+        double ns_per = 0.0;
+        const cudaError_t e = rate(ns, [&](u32 iters) {
+            return m2k::launch_small(d_t, (int)ns, (unsigned)h, T, iters, st, fuse != 0);
+        }, ns_per);
+        if (T == T0 && shift == 0 && fuse == 0) best.ns_default = ns_per;
+        if (best.ns_per_test_iter == 0.0 || ns_per < best.ns_per_test_iter) {
+            best.threads = T; best.carry_shift = shift; best.fuse = fuse; best.ns_per_test_iter = ns_per;
+        }
+        return e;
+    };
+    cudaError_t e = small_rate(T0, 0, 0);
+    if (e == cudaSuccess && duo_for(tests) && m2k::duo_ctas_per_sm((unsigned)h) > 0) {
+        const size_t ns = sample(m2k::duo_ctas_per_sm((unsigned)h));
+        double ns_per = 0.0;
+        e = rate(ns, [&](u32 iters) { return m2k::launch_duo(d_t, (int)ns, (unsigned)h, iters, st); }, ns_per);
+        if (ns_per < best.ns_per_test_iter) {
+            best.threads = m2k::duo_threads((unsigned)h); best.carry_shift = 0; best.fuse = 1; best.duo = true;
+            best.ns_per_test_iter = ns_per;
+        }
+    }
+    // on a full GPU no other combination comes near m2_duo.cu's kernel; a few
+    // tests of n = 256 or 512 are 5-13% faster in the one-CTA kernel's best
+    for (int T = 32; T <= 256 && !(best.duo && cap == full); T *= 2) {
         for (int shift = 0; shift <= 2; ++shift) {
             // a carry split that the segment length rules out collapses onto a smaller shift: skip repeats
             if (shift > 0 && small_carry_threads(items[0].L, items[0].span, T, shift) ==
                                  small_carry_threads(items[0].L, items[0].span, T, shift - 1))
                 continue;
             for (int fuse = 0; fuse <= 1; ++fuse) {
-                const int per_sm = m2k::small_ctas_per_sm((unsigned)h, T, fuse != 0);
-                const size_t ns = std::min(cap, (size_t)per_sm * (size_t)std::max(sms, 1));
-                std::vector<m2k::SmallTest> d(tests.begin(), tests.begin() + ns);
-                for (size_t t = 0; t < ns; ++t) {
-                    d[t].digits = scratch + t * n;
-                    d[t].status = d_st;
-                    d[t].carry_threads = small_carry_threads(items[t].L, items[t].span, T, shift);
-                    d[t].fuse_middle = fuse;
-                }
-                cudaError_t e = cudaMemcpyAsync(scratch, d_dig, ns * n * sizeof(i64), cudaMemcpyDeviceToDevice, st);
-                if (e == cudaSuccess) e = cudaMemcpyAsync(d_t, d.data(), ns * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, st);
-                if (e == cudaSuccess) e = m2k::launch_small(d_t, (int)ns, (unsigned)h, T, 2, st, fuse != 0);   // warm-up
-                if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-                if (e == cudaSuccess) e = m2k::launch_small(d_t, (int)ns, (unsigned)h, T, TUNE_ITERS, st, fuse != 0);
-                if (e == cudaSuccess) e = cudaEventRecord(e1, st);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-                if (e != cudaSuccess) { cleanup(); return fail_cuda("batch tuning", e); }
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                const double ns_per = ms * 1e6 / ((double)ns * TUNE_ITERS);
-                if (T == T0 && shift == 0 && fuse == 0) best.ns_default = ns_per;
-                if (best.ns_per_test_iter == 0.0 || ns_per < best.ns_per_test_iter) {
-                    best.threads = T; best.carry_shift = shift; best.fuse = fuse; best.ns_per_test_iter = ns_per;
-                }
+                if (T == T0 && shift == 0 && fuse == 0) continue;   // the default, above
+                const double before = best.ns_per_test_iter;
+                if (e == cudaSuccess) e = small_rate(T, shift, fuse);
+                if (best.ns_per_test_iter < before) best.duo = false;
             }
         }
     }
+    if (e != cudaSuccess) { cleanup(); return fail_cuda("batch tuning", e); }
     cleanup();
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[{device, h}] = best;
@@ -1162,7 +1214,7 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         (rc = dmal((void**)&d_res, count * sizeof(u64))) || (rc = dmal((void**)&d_prime, count * sizeof(int))) ||
         (rc = dmal((void**)&d_q, 2 * nb * sizeof(int))))
         return rc;
-    struct Launch { u64 h; int ln, threads, ntests, grid; size_t first; long long* d_dig; std::vector<Item>* items; bool fuse; };
+    struct Launch { u64 h; int ln, threads, ntests, grid; size_t first; long long* d_dig; std::vector<Item>* items; bool fuse, duo; };
     std::vector<Launch> launches;
     std::vector<m2k::SmallTest> tests(count);
     std::vector<m2k::TestInit> init(count);
@@ -1195,7 +1247,7 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
             }
             squarings += it.iters;
         }
-        launches.push_back(Launch{h, items[0].L.ln, 0, (int)nt, 0, first, d_dig, &items, false});
+        launches.push_back(Launch{h, items[0].L.ln, 0, (int)nt, 0, first, d_dig, &items, false, false});
         first += nt;
     }
     cudaError_t e = cudaMemsetAsync(d_q, 0, 2 * nb * sizeof(int), s0);
@@ -1207,25 +1259,28 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         std::vector<Item>& items = *l.items;
         Tuned tn;
         const std::vector<m2k::SmallTest> mine(tests.begin() + l.first, tests.begin() + l.first + l.ntests);
-        if ((rc = tune_bucket(device, l.h, items, mine, l.d_dig, sms, tn))) return rc;
+        if ((rc = tune_bucket(device, l.h, items, mine, l.d_dig, sms, count, tn))) return rc;
         l.threads = tn.threads;
         l.fuse = tn.fuse != 0;
+        // the choice is cached per size: these tests may have one it does not serve
+        l.duo = tn.duo && duo_for(mine);
         for (int t = 0; t < l.ntests; ++t) {
             tests[l.first + t].carry_threads = small_carry_threads(items[t].L, items[t].span, tn.threads, tn.carry_shift);
             tests[l.first + t].fuse_middle = tn.fuse;
         }
-        const int per_sm = m2k::small_ctas_per_sm((unsigned)l.h, l.threads, l.fuse);
+        const int per_sm = l.duo ? m2k::duo_ctas_per_sm((unsigned)l.h) : m2k::small_ctas_per_sm((unsigned)l.h, l.threads, l.fuse);
         l.grid = (int)std::min<size_t>((size_t)l.ntests, (size_t)per_sm * (size_t)std::max(sms, 1));
     }
     if (cudaMemcpyAsync(d_all, tests.data(), count * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, s0) != cudaSuccess) return M2_ECUDA;
     // capture: fork from stream 0 to one stream per bucket, join back
     if (cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return M2_ECUDA;
     cudaEventRecord(dv.events[0], s0);
-    for (size_t b = 0; b < launches.size(); ++b) {
+    for (size_t b = launches.size(); b-- > 0;) {   // the largest size first
         cudaStream_t sb = dv.streams[b + 1];
         cudaStreamWaitEvent(sb, dv.events[0], 0);
         const Launch& l = launches[b];
-        m2k::launch_small_persistent(d_all + l.first, l.ntests, (unsigned)l.h, l.threads, d_q + 2 * b, l.grid, sb, l.fuse);
+        if (l.duo) m2k::launch_duo(d_all + l.first, l.ntests, (unsigned)l.h, 0u, sb, d_q + 2 * b, l.grid);
+        else m2k::launch_small_persistent(d_all + l.first, l.ntests, (unsigned)l.h, l.threads, d_q + 2 * b, l.grid, sb, l.fuse);
         cudaEventRecord(dv.events[b + 3], sb);
         cudaStreamWaitEvent(s0, dv.events[b + 3], 0);
     }
@@ -1417,6 +1472,8 @@ int srv_launch(m2_server* s) {
         }
         const int threads = tuned ? tn.threads : c0->threads;
         const bool fuse = tuned ? tn.fuse != 0 : c0->h_test.fuse_middle != 0;
+        bool duo = !tuned || tn.duo;
+        for (size_t j = 0; j < cnt && duo; ++j) duo = duo_for({s->active[kv.second[j]].ctx->h_test});
         for (size_t j = 0; j < cnt; ++j) {
             SrvItem& it = s->active[kv.second[j]];
             b.ks[j] = std::min(s->quantum, it.total - it.done);
@@ -1431,7 +1488,9 @@ int srv_launch(m2_server* s) {
         if (e == cudaSuccess) e = cudaMemsetAsync(b.d_status, 0, cnt * sizeof(int), b.stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b.d_tests, b.h_tests, cnt * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, b.stream);
         if (e != cudaSuccess) return fail_cuda("server descriptor upload", e);
-        if ((e = m2k::launch_small(b.d_tests, (int)cnt, (unsigned)kv.first, threads, 0u, b.stream, fuse)) != cudaSuccess)
+        e = duo ? m2k::launch_duo(b.d_tests, (int)cnt, (unsigned)kv.first, 0u, b.stream)
+                : m2k::launch_small(b.d_tests, (int)cnt, (unsigned)kv.first, threads, 0u, b.stream, fuse);
+        if (e != cudaSuccess)
             return fail_cuda("server small-test launch", e);
         e = cudaMemcpyAsync(b.h_status, b.d_status, cnt * sizeof(int), cudaMemcpyDeviceToHost, b.stream);
         if (e == cudaSuccess) e = cudaEventRecord(b.ev, b.stream);

@@ -111,6 +111,14 @@ cudaError_t launch_test_init(const TestInit* d_tests, int ntests, cudaStream_t s
 // low 64 bits and verdict of each test's state (n = 2^ln <= 16384 digits)
 cudaError_t launch_results(const SmallTest* d_tests, int ntests, int ln, unsigned long long* res64, int* prime, cudaStream_t s);
 
+// ---- one test per CTA, fields in turn, both fields' layout only (m2_duo.cu) ----
+bool duo_supported(unsigned int h, int span, int carry_threads);
+int duo_threads(unsigned int h);
+int duo_ctas_per_sm(unsigned int h);
+// one CTA per test, or (d_queue) a persistent grid; iters_override as launch_small
+cudaError_t launch_duo(const SmallTest* d_tests, int ntests, unsigned int h, unsigned int iters_override, cudaStream_t s,
+                       int* d_queue = nullptr, int grid = 0);
+
 // Throughput of 32x32->64-bit integer multiplies (mul.wide.u32 / mad.wide.u32)
 // on every SM: independent chains, returns products per second.
 double measure_wide_mul_rate(int device);
