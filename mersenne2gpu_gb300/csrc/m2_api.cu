@@ -30,6 +30,7 @@ namespace {
 // ---------------- device twiddle cache (one table set per device and h) ----------------
 struct TwTables {
     m2k::DTw* tw4 = nullptr;
+    m2k::DTw* tw8 = nullptr;
     m2k::DTw* tc = nullptr;
     size_t bytes = 0;
 };
@@ -53,14 +54,17 @@ int get_twiddles(int device, u64 h, TwTables& out) {
     if (!mp || cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); return M2_ECUDA; }
     cudaError_t e = cudaMallocFromPoolAsync((void**)&t.tw4, b4, mp, s);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void**)&t.tc, bc, mp, s);
+    const size_t b8 = m2k::twiddle8_entries(h) * sizeof(m2k::DTw);
+    if (e == cudaSuccess && b8) e = cudaMallocFromPoolAsync((void**)&t.tw8, b8, mp, s);
     if (e == cudaSuccess) e = m2k::launch_twiddles(t.tw4, t.tc, (unsigned)h, s);
+    if (e == cudaSuccess && b8) e = m2k::launch_twiddles8(t.tw8, (unsigned)h, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaStreamDestroy(s);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return e == cudaErrorMemoryAllocation ? M2_ENOMEM : M2_ECUDA;
     }
-    t.bytes = b4 + bc;
+    t.bytes = b4 + bc + b8;
     g_tw[{device, h}] = t;
     out = t;
     return M2_OK;
@@ -261,7 +265,7 @@ bool ensure_graph(m2_ctx* c, int i) {
 constexpr uint32_t FLOW_ITERS = 1000;
 constexpr uint32_t TIDE_ITERS = 250;
 
-m2k::TideArgs tide_args(const m2_ctx* c) { return m2k::TideArgs{c->fargs, c->d_taux, c->d_tshift, c->d_park}; }
+m2k::TideArgs tide_args(const m2_ctx* c) { return m2k::TideArgs{c->fargs, c->d_taux, c->d_tshift, c->d_park, c->tw.tw8}; }
 
 // the one-launch kernel's tags as every launch expects them: all element tags
 // 1, carries of parity 0

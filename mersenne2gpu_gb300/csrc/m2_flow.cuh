@@ -49,19 +49,19 @@ __device__ __forceinline__ X31 untag(const X31& v) { return X31{v.c & P31, v.d &
 
 // (the warp's active lanes poll together: diverged loops cost the lone warps of
 // the small shapes their branch latency at every poll)
-template <u32 TAG, class X> __device__ __forceinline__ void take4(X (&x)[4], const X* p, u32 stride, Wait& w) {
+template <u32 TAG, int N, class X> __device__ __forceinline__ void take(X (&x)[N], const X* p, u32 stride, Wait& w) {
     u32 it = 0;
     const u32 lanes = __activemask();
     do {
         u32 off = 0;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) x[m] = ld_relaxed(p + (u64)m * stride);
+        for (int m = 0; m < N; ++m) x[m] = ld_relaxed(p + (u64)m * stride);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) off |= off_tag<TAG>(x[m]);
+        for (int m = 0; m < N; ++m) off |= off_tag<TAG>(x[m]);
         if (__all_sync(lanes, (int)off >= 0)) break;
     } while (__any_sync(lanes, w.again(it)));
 #pragma unroll
-    for (int m = 0; m < 4; ++m) x[m] = untag(x[m]);
+    for (int m = 0; m < N; ++m) x[m] = untag(x[m]);
 }
 
 // XOR swizzle of a unit's shared-memory slots (16-byte GF(P61^2) slots, 8-byte
@@ -165,7 +165,7 @@ template <class S, class X> struct Unit {
                   [&](u32 b, X (&x)[4]) {
                       const u32 rho = b / S::C, cc = b % S::C;
                       if (l == NL - 1) {
-                          take4<1>(x, g + (u64)(4 * rho) * S::B + cg * S::C + cc, S::B, w);
+                          take<1>(x, g + (u64)(4 * rho) * S::B + cg * S::C + cc, S::B, w);
                       } else {
                           const u32 s0 = sw((rho / Q * M + rho % Q) * S::C + cc);
 #pragma unroll
@@ -184,17 +184,18 @@ template <class S, class X> struct Unit {
     // ---- row pair (t0, t1), slot s B + i for element i of row t_s ----
     static constexpr bool ODD = (S::LB & 1) != 0;
     static constexpr int NF4 = S::LB / 2 - (ODD ? 0 : 1);    // radix-4 levels outside the tail
-    __device__ __forceinline__ void rows_fwd_level(int l, u32 t0, u32 t1, Wait& w, bool barrier) const {
+    // (the first level: its operands from global memory, or written by another kind of level)
+    __device__ __forceinline__ void rows_fwd_level(int l, u32 t0, u32 t1, Wait& w, bool barrier, bool first) const {
         {
             const u32 M = S::B >> (2 * l), Q = M / 4;
-            level<IR, S::NBR>(!barrier ? 0 : l > 0 ? M : S::NF, [&](u32 b, Tri<X>& t) {
+            level<IR, S::NBR>(!barrier ? 0 : first ? S::NF : M, [&](u32 b, Tri<X>& t) {
                       const u32 rho = b % (S::B / 4), trow = b / (S::B / 4) ? t1 : t0;
                       t = ldtri<X>(tw4, (S::R + trow) * (1u << (2 * l)) + rho / Q);
                   },
                   [&](u32 b, X (&x)[4]) {
                       const u32 rho = b % (S::B / 4), sl = b / (S::B / 4);
                       if (l == 0) {
-                          take4<0>(x, g + (u64)(sl ? t1 : t0) * S::B + rho, Q, w);
+                          take<0>(x, g + (u64)(sl ? t1 : t0) * S::B + rho, Q, w);
                       } else {
                           const u32 s0 = sw(sl * S::B + rho / Q * M + rho % Q);
 #pragma unroll
@@ -337,28 +338,37 @@ template <class S, class... U> __device__ __forceinline__ void run_cols_inv(u32 
         ((u.cols_inv_level(l, cg, w, barrier), barrier = false, asm_fence()), ...);
     }
 }
-template <class S, class... U> __device__ __forceinline__ void run_rows(u32 pi, Wait& w, const U&... u) {
-    constexpr int NF4 = S::LB / 2 - ((S::LB & 1) ? 0 : 1);
-    u32 t0 = 0, t1 = 1;
+// rows of pair pi
+__device__ __forceinline__ void row_pair(u32 pi, u32& t0, u32& t1) {
+    t0 = 0; t1 = 1;
     if (pi) {
         const u32 e = 32u - __clz(pi), a = pi - (1u << (e - 1));
         t0 = (1u << e) + a;
         t1 = (2u << e) - 1u - a;
     }
+}
+// a pair's levels from radix-4 level FIRST on and back
+template <class S, int FIRST, class... U> __device__ __forceinline__ void run_rows_from(u32 pi, u32 t0, u32 t1, Wait& w, const U&... u) {
+    constexpr int NF4 = S::LB / 2 - ((S::LB & 1) ? 0 : 1);
 #pragma unroll
-    for (int l = 0; l < NF4; ++l) {
+    for (int l = FIRST; l < NF4; ++l) {
         bool barrier = true;
-        ((u.rows_fwd_level(l, t0, t1, w, barrier), barrier = false, asm_fence()), ...);
+        ((u.rows_fwd_level(l, t0, t1, w, barrier, l == FIRST), barrier = false, asm_fence()), ...);
     }
     {
         bool barrier = true;
         ((u.rows_tail(pi, t0, t1, barrier), barrier = false, asm_fence()), ...);
     }
 #pragma unroll
-    for (int l = NF4 - 1; l >= 0; --l) {
+    for (int l = NF4 - 1; l >= FIRST; --l) {
         bool barrier = true;
         ((u.rows_inv_level(l, t0, t1, barrier), barrier = false, asm_fence()), ...);
     }
+}
+template <class S, class... U> __device__ __forceinline__ void run_rows(u32 pi, Wait& w, const U&... u) {
+    u32 t0, t1;
+    row_pair(pi, t0, t1);
+    run_rows_from<S, 0>(pi, t0, t1, w, u...);
 }
 
 }  // namespace

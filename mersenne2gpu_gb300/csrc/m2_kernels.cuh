@@ -89,6 +89,7 @@ struct TideArgs {
     const uint2* taux;
     const unsigned int* tshift;
     longlong2* park;
+    const DTw* tw8;            // the radix-8 levels' twiddles (launch_twiddles8)
 };
 
 constexpr int LARGE_STAGES = 3;
@@ -105,6 +106,10 @@ struct TestInit {
     int ln;                    // at most 30
 };
 size_t twiddle_entries(unsigned long long h);   // DTw entries of tw4; tc has h / 2
+// The radix-8 levels' tables (m2_tide.cu): w_{8S}^(a br_S(j)) at 7 (S + j) + a - 1
+// for S = 8, 1024, 8192 blocks before the step, a = 1 ... 7
+size_t twiddle8_entries(unsigned long long h);   // 0 below h = 2^20
+cudaError_t launch_twiddles8(DTw* tw8, unsigned int h, cudaStream_t s);
 cudaError_t launch_twiddles(DTw* tw4, DTw* tc, unsigned int h, cudaStream_t s);   // h >= 4
 cudaError_t launch_test_init(const TestInit& T, cudaStream_t s);
 cudaError_t launch_test_init(const TestInit* d_tests, int ntests, cudaStream_t s);

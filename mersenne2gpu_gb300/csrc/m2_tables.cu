@@ -52,6 +52,19 @@ __global__ void __launch_bounds__(256) k_twiddles(DTw* tw4, DTw* tc, u32 h, int 
     }
 }
 
+__global__ void __launch_bounds__(256) k_twiddles8(DTw* tw8, u32 h, E wh) {
+    const u32 t = blockIdx.x * 256u + threadIdx.x;   // S + j
+    if (t < 8 || t >= 16384) return;
+    const int sb = 31 - __clz(t);
+    if (sb != 3 && sb != 10 && sb != 13) return;
+    const E r = dpow(wh, (u64)(h >> (sb + 3)) * brev(t - (1u << sb), sb));
+    E q = r;
+    for (u32 a = 0; a < 7; ++a) {
+        put_tw(tw8, 7u * t + a, q);
+        q = emul(q, r);
+    }
+}
+
 // w61/w31[j] = n^-1 (n - p j mod n) mod 61 / 31 (shift 0 for j = 0); aux: the
 // rotations by 2^-(s + ln + 1) that unweight an element's two digits, and the
 // digits' widths; digits: the small start value x0
@@ -145,6 +158,12 @@ cudaError_t launch_twiddles(DTw* tw4, DTw* tc, unsigned h, cudaStream_t s) {
     while ((1u << lh) < h) ++lh;
     const unsigned g = (h / 2 + 255) / 256;
     k_twiddles<<<g < 4096 ? g : 4096, 256, 0, s>>>(tw4, tc, h, lh, E{w.a, w.b, w.c, w.d});
+    return cudaGetLastError();
+}
+size_t twiddle8_entries(unsigned long long h) { return h >= (1ull << 20) ? 7 * 16384 : 0; }
+cudaError_t launch_twiddles8(DTw* tw8, unsigned h, cudaStream_t s) {
+    const m2::Dual w = m2::root_of_unity(h);
+    k_twiddles8<<<64, 256, 0, s>>>(tw8, h, E{w.a, w.b, w.c, w.d});
     return cudaGetLastError();
 }
 cudaError_t launch_test_init(const TestInit& T, cudaStream_t s) {

@@ -15,31 +15,113 @@
 // first and parks its digits in the state's buffer, so that no group waits for
 // a carry that its neighbour has not yet begun to make.
 //
+// The first two levels of the columns, and at n = 2^21 of the rows, are
+// radix-8 with a butterfly per thread: 6 twiddle products per element and
+// squaring for 7.5 (the columns' first level has none in either form), a
+// quarter fewer passes over shared memory and barriers.
 //
-// What bounds it: the integer pipes (ALU and multiply-add each a little under
-// 60% busy, issue 0.6 a cycle and scheduler), with the row pairs' 3.37 per SM
-// rounded up to 4.  Measured, us per squaring, three-pass kernels -> here:
-// n = 2^21 128.6 -> 110.2, 2^22 289 -> 235, GF(P61^2) alone at 2^22 204 -> 169
+// What bounds it: the integer pipes (ALU and multiply-add each about 60% busy,
+// issue 0.6 a cycle and scheduler), with the row pairs' 3.37 per SM rounded up
+// to 4.  Measured, us per squaring, three-pass kernels -> here:
+// n = 2^21 128.6 -> 103.4, 2^22 289 -> 233, GF(P61^2) alone at 2^22 204 -> 166
 // (134.3, 299.5 and 208 before the arithmetic steps of m2_field.cuh).  On the
 // way (n = 2^21): the two fields on separate warps 128.6 (the GF(P31) warps
 // finish early and leave half the warps to the rest), both on every warp 117;
-// row-stage tables in row order 110.
+// row-stage tables in row order 110; radix-8 columns 107; four row pairs at a
+// time instead of two 105.7; radix-8 rows 103.4.  At n = 2^22 radix-8 columns
+// took 235 to 233; radix-8 rows there spill and take 241.
 #include "m2_flow.cuh"
 
 namespace M2K_NS {
 
 namespace {
 
-template <int LB_, int UNITS_> struct Shape {
+template <int LB_, int UNITS_, u32 PAIRS_, bool ROWS8_> struct Shape {
     static constexpr int LR = 10, LB = LB_, C = 7, UNITS = UNITS_;
     static constexpr u32 R = 1u << LR, B = 1u << LB, H = R * B;
     static constexpr u32 NBC = R / 4 * C, NBR = 2 * B / 4;   // radix-4 butterflies of a level
-    static constexpr u32 NF = 512, NT = 1024;                // threads of a row pair, of the CTA
-    static constexpr u32 SLOTS = R * C > 4 * B ? R * C : 4 * B, SMEM = 24 * SLOTS;   // a column group, or two row pairs
+    static constexpr u32 PAIRS = PAIRS_;                     // row pairs at a time
+    static constexpr bool ROWS8 = ROWS8_;                    // radix-8 levels in the rows, too
+    static constexpr u32 NT = 1024, NF = NT / PAIRS;         // threads of the CTA, of a row pair
+    static constexpr u32 SLOTS = 2 * B * PAIRS, SMEM = 24 * SLOTS;   // the row pairs, or a column group
     static constexpr u32 SLOT_R = R * C;
-    static constexpr bool NARROW = true;
+    static constexpr bool NARROW = PAIRS == 2;               // 15 barriers: 7 per row pair, or one
+    static constexpr u32 BARS = NARROW ? 7 : 1;
+    static_assert(SLOT_R <= SLOTS, "a column group fits");
+    static_assert(!ROWS8 || NF == 2 * B / 8, "a radix-8 butterfly per thread");
     static_assert(NT == R, "a thread per row in the row stage");
 };
+
+// ---- radix-8 levels ----
+// Three levels of the per-block-twiddle transform at once: with r^8 = c the
+// residues mod X^m - r w^e, w = (1 + i) / sqrt 2, e = 0, 4, 2, 6, 1, 5, 3, 7.
+// sqrt 2 is 2^31 in GF(P61) and 2^16 in GF(P31): a product by w is an
+// addition, a subtraction and two shifts, and 7 products by twiddles do the
+// work of 9 in radix-4 levels.
+//
+// x below 7 2^61 times 2^30 modulo P61, below 2^61 + 2^33
+__device__ __forceinline__ u64 scale61(u64 x) { return ((x & 0x7fffffffull) << 30) + (x >> 31); }
+__device__ __forceinline__ u32 scale31(u32 x) { return rotl31(x, 15); }
+// w (x - y): the difference offset by 2 P61 (below 3 2^61 + 8), the sum and the
+// difference of its coordinates (offset by 4 P61) below 7 2^61 + 16
+__device__ __forceinline__ X61 eighth_of_diff(const X61& x, const X61& y) {
+    const L61 d = lsub(x.a, x.b, y.a, y.b);
+    return X61{scale61(d.a + (K4_61 - d.b)), scale61(d.a + d.b)};
+}
+__device__ __forceinline__ X31 eighth_of_diff(const X31& x, const X31& y) {
+    const X31 d = xsub(x, y);
+    return X31{scale31(sub31(d.c, d.d)), scale31(add31(d.c, d.d))};
+}
+// conj(w) x, x below 2^61 + 8
+__device__ __forceinline__ X61 eighth_conj(const X61& x) { return X61{scale61(x.a + x.b), scale61(x.b + (K2_61 - x.a))}; }
+__device__ __forceinline__ X31 eighth_conj(const X31& x) { return X31{scale31(add31(x.c, x.d)), scale31(sub31(x.d, x.c))}; }
+
+// i x, x below 2 P61
+__device__ __forceinline__ X61 times_i(const X61& x) { return X61{K2_61 - x.b, x.a}; }
+__device__ __forceinline__ X31 times_i(const X31& x) { return xtimes_i(x); }
+
+template <class X> __device__ __forceinline__ void dif8_adds(X (&x)[8]) {
+    X a[4], b[4];
+    a[0] = xadd(x[0], x[4]); b[0] = xsub(x[0], x[4]);
+    a[1] = xadd(x[1], x[5]); b[1] = eighth_of_diff(x[1], x[5]);
+    a[2] = xadd(x[2], x[6]); b[2] = times_i(xsub(x[2], x[6]));
+    a[3] = xadd(x[3], x[7]); b[3] = times_i(eighth_of_diff(x[3], x[7]));
+    dif_adds(a, a[1], a[2], a[3]);
+    dif_adds(b, b[1], b[2], b[3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { x[k] = a[k]; x[4 + k] = b[k]; }
+}
+template <class X> __device__ __forceinline__ void dit8_adds(X (&x)[8]) {
+    X a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { a[k] = x[k]; b[k] = x[4 + k]; }
+    dit_adds(a);
+    dit_adds(b);
+    b[1] = eighth_conj(b[1]);
+    b[2] = times_i(b[2]);                  // its negative: -i b[2] is taken off
+    b[3] = times_i(eighth_conj(b[3]));
+    x[0] = xadd(a[0], b[0]); x[4] = xsub(a[0], b[0]);
+    x[1] = xadd(a[1], b[1]); x[5] = xsub(a[1], b[1]);
+    x[2] = xsub(a[2], b[2]); x[6] = xadd(a[2], b[2]);
+    x[3] = xsub(a[3], b[3]); x[7] = xadd(a[3], b[3]);
+}
+// x[k] times entry k - 1 of t (its conjugate)
+template <class X> __device__ __forceinline__ void twist8(X (&x)[8], const DTw* t) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        X w;
+        ldtw(w, t, k - 1);
+        x[k] = xmul(x[k], w);
+    }
+}
+template <class X> __device__ __forceinline__ void untwist8(X (&x)[8], const DTw* t) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        X w;
+        ldtw(w, t, k - 1);
+        x[k] = xmulc(x[k], w);
+    }
+}
 
 // the column levels: columns c0 ... c0 + nc - 1 (nc <= 7), slot 7 r + c; every
 // thread runs both fields' butterflies threadIdx.x, threadIdx.x + 1024, ...
@@ -47,8 +129,40 @@ template <class S, class X> struct Cols {
     X* z;
     X* g;
     const DTw* tw4;
+    const DTw* tw8;
     u32 c0, nc;
 
+    // radix-8 level l: blocks of R / 8^l rows
+    template <class F> __device__ __forceinline__ void each8(F&& f) const {
+        const u32 rho = threadIdx.x / S::C, cc = threadIdx.x - rho * S::C;
+        if (rho < S::R / 8 && cc < nc) f(rho, cc);
+    }
+    __device__ __forceinline__ void fwd_level8(int l) const {
+        const u32 M = S::R >> (3 * l), Q = M / 8;
+        each8([&](u32 rho, u32 cc) {
+            X* s = z + (rho / Q * M + rho % Q) * S::C + cc;
+            X x[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) x[m] = s[m * Q * S::C];
+            if (l > 0) twist8(x, tw8 + 7 * ((1u << (3 * l)) + rho / Q));
+            dif8_adds(x);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) s[m * Q * S::C] = x[m];
+        });
+    }
+    __device__ __forceinline__ void inv_level8(int l) const {
+        const u32 M = S::R >> (3 * l), Q = M / 8;
+        each8([&](u32 rho, u32 cc) {
+            X* s = z + (rho / Q * M + rho % Q) * S::C + cc;
+            X x[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) x[m] = s[m * Q * S::C];
+            dit8_adds(x);
+            if (l > 0) untwist8(x, tw8 + 7 * ((1u << (3 * l)) + rho / Q));
+#pragma unroll
+            for (int m = 0; m < 8; ++m) s[m * Q * S::C] = x[m];
+        });
+    }
     template <class F> __device__ __forceinline__ void each(F&& f) const {
 #pragma unroll 1
         for (u32 b = threadIdx.x; b < S::NBC; b += S::NT) {
@@ -81,7 +195,7 @@ template <class S, class X> struct Cols {
             X* s = z + (rho / Q * M + rho % Q) * S::C + cc;
             X x[4];
             if (l == S::LR / 2 - 1) {
-                take4<1>(x, g + (u64)(4 * rho) * S::B + c0 + cc, S::B, w);
+                take<1>(x, g + (u64)(4 * rho) * S::B + c0 + cc, S::B, w);
             } else {
 #pragma unroll
                 for (int m = 0; m < 4; ++m) x[m] = s[m * Q * S::C];
@@ -95,16 +209,79 @@ template <class S, class X> struct Cols {
 };
 template <class S, class... F> __device__ __forceinline__ void cols_fwd(const F&... f) {
 #pragma unroll
-    for (int l = 0; l < S::LR / 2; ++l) {
+    for (int l = 0; l < 2; ++l) {
+        __syncthreads();
+        ((f.fwd_level8(l), asm_fence()), ...);
+    }
+#pragma unroll
+    for (int l = 3; l < S::LR / 2; ++l) {
         __syncthreads();
         ((f.fwd_level(l), asm_fence()), ...);
     }
 }
 template <class S, class... F> __device__ __forceinline__ void cols_inv(Wait& w, const F&... f) {
 #pragma unroll
-    for (int l = S::LR / 2 - 1; l >= 0; --l) {
+    for (int l = S::LR / 2 - 1; l >= 3; --l) {
         __syncthreads();
         ((f.inv_level(l, w), asm_fence()), ...);
+    }
+#pragma unroll
+    for (int l = 1; l >= 0; --l) {
+        __syncthreads();
+        ((f.inv_level8(l), asm_fence()), ...);
+    }
+}
+
+// a row pair: two radix-8 levels, then the radix-4 levels and the tail of m2_flow.cuh
+template <class S, class X> __device__ __forceinline__ void rows_fwd_level8(const Unit<S, X>& u, const DTw* tw8, int l, u32 t0, u32 t1, Wait& w) {
+    const u32 M = S::B >> (3 * l), Q = M / 8, rho = u.fb % (S::B / 8), sl = u.fb / (S::B / 8), t = sl ? t1 : t0;
+    const u32 s0 = sw(sl * S::B + rho / Q * M + rho % Q);
+    X x[8];
+    if (l == 0) {
+        take<0>(x, u.g + (u64)t * S::B + rho, Q, w);
+    } else {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) x[m] = u.z[s0 ^ sw(m * Q)];
+    }
+    twist8(x, tw8 + 7 * ((S::R + t) * (1u << (3 * l)) + rho / Q));
+    dif8_adds(x);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) u.z[s0 ^ sw(m * Q)] = x[m];
+}
+template <class S, class X> __device__ __forceinline__ void rows_inv_level8(const Unit<S, X>& u, const DTw* tw8, int l, u32 t0, u32 t1) {
+    const u32 M = S::B >> (3 * l), Q = M / 8, rho = u.fb % (S::B / 8), sl = u.fb / (S::B / 8), t = sl ? t1 : t0;
+    const u32 s0 = sw(sl * S::B + rho / Q * M + rho % Q);
+    X x[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) x[m] = u.z[s0 ^ sw(m * Q)];
+    dit8_adds(x);
+    untwist8(x, tw8 + 7 * ((S::R + t) * (1u << (3 * l)) + rho / Q));
+    if (l > 0) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) u.z[s0 ^ sw(m * Q)] = x[m];
+    } else {
+        X* p = u.g + (u64)t * S::B + rho;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) st_tagged<1>(p + m * Q, x[m]);
+    }
+}
+template <class S, class U0, class... U> __device__ __forceinline__ void rows8(u32 pi, const DTw* tw8, Wait& w, const U0& u0, const U&... u) {
+    u32 t0, t1;
+    row_pair(pi, t0, t1);
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        u0.sync();
+        rows_fwd_level8(u0, tw8, l, t0, t1, w);
+        asm_fence();
+        ((rows_fwd_level8(u, tw8, l, t0, t1, w), asm_fence()), ...);
+    }
+    run_rows_from<S, 3>(pi, t0, t1, w, u0, u...);
+#pragma unroll
+    for (int l = 1; l >= 0; --l) {
+        u0.sync();
+        rows_inv_level8(u0, tw8, l, t0, t1);
+        asm_fence();
+        ((rows_inv_level8(u, tw8, l, t0, t1), asm_fence()), ...);
     }
 }
 
@@ -130,12 +307,11 @@ __global__ void __launch_bounds__(S::NT, 1) k_tide(TideArgs TA) {
     X61* za = reinterpret_cast<X61*>(smem);
     X31* zb = reinterpret_cast<X31*>(smem + 16ull * S::SLOTS);
     const u32 tid = threadIdx.x, cta = blockIdx.x, groups = gridDim.x * S::UNITS;
-    // each half of the threads takes row pairs of its own
-    const u32 half = tid / S::NF;
+    const u32 part = tid / S::NF;        // each part of the threads takes row pairs of its own
     X61* ga = reinterpret_cast<X61*>(A.za);
     X31* gb = reinterpret_cast<X31*>(A.zb);
-    Unit<S, X61> ua{za + half * 2 * S::B, ga, A.tw4, A.tc, tid % S::NF, 1 + 7 * half};
-    Unit<S, X31> ub{zb + half * 2 * S::B, gb, A.tw4, A.tc, tid % S::NF, 1 + 7 * half};
+    Unit<S, X61> ua{za + part * 2 * S::B, ga, A.tw4, A.tc, tid % S::NF, 1 + S::BARS * part};
+    Unit<S, X31> ub{zb + part * 2 * S::B, gb, A.tw4, A.tc, tid % S::NF, 1 + S::BARS * part};
     Wait w{A.status, false};
     all_started(A.arrivals, gridDim.x, w);
     const u32 base = A.parity[cta];      // squarings handed over so far (bit 0); bit 1 never matches a word's tag
@@ -195,14 +371,14 @@ __global__ void __launch_bounds__(S::NT, 1) k_tide(TideArgs TA) {
             za[r * S::C + c] = weigh61(d.x, d.y, s);
             if (kDual) zb[r * S::C + c] = weigh31(d.x, d.y, s >> 16);
         }
-        const Cols<S, X61> fa{za, ga, A.tw4, c0, nc};
-        if (kDual) cols_fwd<S>(fa, Cols<S, X31>{zb, gb, A.tw4, c0, nc});
+        const Cols<S, X61> fa{za, ga, A.tw4, TA.tw8, c0, nc};
+        if (kDual) cols_fwd<S>(fa, Cols<S, X31>{zb, gb, A.tw4, TA.tw8, c0, nc});
         else cols_fwd<S>(fa);
     };
     auto inverse = [&](u32 g, u32 par) { // inverse levels, unweight, CRT, carry chain: digits in the slots
         const u32 c0 = first(g), nc = first(g + 1) - c0;
-        const Cols<S, X61> fa{za, ga, A.tw4, c0, nc};
-        if (kDual) cols_inv<S>(w, fa, Cols<S, X31>{zb, gb, A.tw4, c0, nc});
+        const Cols<S, X61> fa{za, ga, A.tw4, TA.tw8, c0, nc};
+        if (kDual) cols_inv<S>(w, fa, Cols<S, X31>{zb, gb, A.tw4, TA.tw8, c0, nc});
         else cols_inv<S>(w, fa);
         __syncthreads();
         i64 c = 0;
@@ -237,9 +413,14 @@ __global__ void __launch_bounds__(S::NT, 1) k_tide(TideArgs TA) {
         asm volatile("" : "+r"(ua.fb), "+r"(ub.fb));   // addresses and twiddles made anew in every squaring
         __syncthreads();   // the slots' last reads are done
 #pragma unroll 1
-        for (u32 pi = cta + half * gridDim.x; pi < S::R / 2; pi += 2 * gridDim.x) {
-            if (kDual) run_rows<S>(pi, w, ua, ub);
-            else run_rows<S>(pi, w, ua);
+        for (u32 pi = cta + part * gridDim.x; pi < S::R / 2; pi += S::PAIRS * gridDim.x) {
+            if constexpr (S::ROWS8) {
+                if (kDual) rows8<S>(pi, TA.tw8, w, ua, ub);
+                else rows8<S>(pi, TA.tw8, w, ua);
+            } else {
+                if (kDual) run_rows<S>(pi, w, ua, ub);
+                else run_rows<S>(pi, w, ua);
+            }
         }
         const u32 par = (base ^ 1u ^ it) & 1u;
         const bool last = it + 1 == A.k;
@@ -304,11 +485,12 @@ template <class S> cudaError_t tables(const TideArgs& A, cudaStream_t s) {
 
 }  // namespace
 
-// one group of columns per CTA at h = 2^20, two at h = 2^21
-#define M2_TIDE_SHAPES(X) X(20, 10, 1) X(21, 11, 2)
+// one group of columns per CTA at h = 2^20, two at h = 2^21; row pairs at a
+// time (196 KiB of slots) and whether their first levels are radix-8: above
+#define M2_TIDE_SHAPES(X) X(20, 10, 1, 4, true) X(21, 11, 2, 2, false)
 
 size_t tide_groups(int lh) {
-#define M2_TIDE_G(LH, LB, U) if (lh == LH) return (size_t)sm_count() * U;
+#define M2_TIDE_G(LH, LB, U, P, R8) if (lh == LH) return (size_t)sm_count() * U;
     M2_TIDE_SHAPES(M2_TIDE_G)
 #undef M2_TIDE_G
     return 0;
@@ -316,13 +498,13 @@ size_t tide_groups(int lh) {
 // records of the row stage's tables, and of the digits parked meanwhile
 size_t tide_records(int lh) { return tide_groups(lh) * 7 * 1024; }
 size_t tide_parked(int lh) {
-#define M2_TIDE_P(LH, LB, U) if (lh == LH) return (size_t)sm_count() * (U - 1) * 7 * 1024;
+#define M2_TIDE_P(LH, LB, U, P, R8) if (lh == LH) return (size_t)sm_count() * (U - 1) * 7 * 1024;
     M2_TIDE_SHAPES(M2_TIDE_P)
 #undef M2_TIDE_P
     return 0;
 }
 cudaError_t tide_tables(int lh, const TideArgs& A, cudaStream_t s) {
-#define M2_TIDE_T(LH, LB, U) if (lh == LH) return tables<Shape<LB, U>>(A, s);
+#define M2_TIDE_T(LH, LB, U, P, R8) if (lh == LH) return tables<Shape<LB, U, P, R8>>(A, s);
     M2_TIDE_SHAPES(M2_TIDE_T)
 #undef M2_TIDE_T
     return cudaErrorInvalidValue;
@@ -332,7 +514,7 @@ bool tide_supported(int lh, int span, bool gf61) {
     if (gf61) return m2k_g61::tide_supported(lh, span, true);
 #endif
     bool ok = false;
-#define M2_TIDE_F(LH, LB, U) if (lh == LH) ok = fits<Shape<LB, U>>();
+#define M2_TIDE_F(LH, LB, U, P, R8) if (lh == LH) ok = fits<Shape<LB, U, P, R8>>();
     M2_TIDE_SHAPES(M2_TIDE_F)
 #undef M2_TIDE_F
     cudaGetLastError();
@@ -342,7 +524,7 @@ cudaError_t launch_tide(int lh, bool gf61, const TideArgs& A, cudaStream_t s) {
 #if M2_DUAL
     if (gf61) return m2k_g61::launch_tide(lh, true, A, s);
 #endif
-#define M2_TIDE_L(LH, LB, U) if (lh == LH) return launch<Shape<LB, U>>(A, s);
+#define M2_TIDE_L(LH, LB, U, P, R8) if (lh == LH) return launch<Shape<LB, U, P, R8>>(A, s);
     M2_TIDE_SHAPES(M2_TIDE_L)
 #undef M2_TIDE_L
     return cudaErrorInvalidValue;

@@ -72,3 +72,77 @@ def test_gf61_products_range_and_value():
         for got, want in ((mul, (a0 * b0 - a1 * b1, a0 * b1 + a1 * b0)), (conj, (a0 * b0 + a1 * b1, a1 * b0 - a0 * b1)),
                           (sqr, (a0 * a0 - a1 * a1, 2 * a0 * a1))):
             assert all(0 <= g <= top and g % P61 == w % P61 for g, w in zip(got, want))
+
+
+def scale61(x):
+    return u64(((u64(x) & ((1 << 31) - 1)) << 30) + (x >> 31))
+
+
+def radix8(u):
+    """dif8_adds of m2_tide.cu in GF(P61^2), every step as there."""
+    k2, k4 = 2 * P61, 4 * P61
+    add = lambda x, y: tuple(fold61(u64(p + q)) for p, q in zip(x, y))
+    lsub = lambda x, y: tuple(u64(p + u64(k2 - q)) for p, q in zip(x, y))
+    sub = lambda x, y: tuple(fold61(t) for t in lsub(x, y))
+    times_i = lambda x: (u64(k2 - x[1]), x[0])
+
+    def eighth_of_diff(x, y):
+        d = lsub(x, y)
+        return scale61(d[0] + u64(k4 - d[1])), scale61(d[0] + d[1])
+
+    def dif_adds(x, u1, u2, u3):
+        v0, v1 = tuple(u64(p + q) for p, q in zip(x, u2)), tuple(u64(p + q) for p, q in zip(u1, u3))
+        v2, v3 = lsub(x, u2), lsub(u1, u3)
+        fadd, fsub = lambda p, q: fold61(u64(p + q)), lambda p, q: fold61(u64(p + u64(k4 - q)))
+        return [(fadd(v0[0], v1[0]), fadd(v0[1], v1[1])), (fsub(v0[0], v1[0]), fsub(v0[1], v1[1])),
+                (fsub(v2[0], v3[1]), fadd(v2[1], v3[0])), (fadd(v2[0], v3[1]), fsub(v2[1], v3[0]))]
+
+    a = [add(u[m], u[m + 4]) for m in range(4)]
+    b = [sub(u[0], u[4]), eighth_of_diff(u[1], u[5]), times_i(sub(u[2], u[6])), times_i(eighth_of_diff(u[3], u[7]))]
+    return dif_adds(*a) + dif_adds(*b)
+
+
+def unradix8(y):
+    """dit8_adds of m2_tide.cu in GF(P61^2)."""
+    k2, k4 = 2 * P61, 4 * P61
+    add = lambda x, z: tuple(fold61(u64(p + q)) for p, q in zip(x, z))
+    lsub = lambda x, z: tuple(u64(p + u64(k2 - q)) for p, q in zip(x, z))
+    sub = lambda x, z: tuple(fold61(t) for t in lsub(x, z))
+    times_i = lambda x: (u64(k2 - x[1]), x[0])
+    eighth_conj = lambda x: (scale61(x[0] + x[1]), scale61(x[1] + u64(k2 - x[0])))
+
+    def dit_adds(x):
+        v0, v1 = tuple(u64(p + q) for p, q in zip(x[0], x[1])), lsub(x[0], x[1])
+        v2, v3 = tuple(u64(p + q) for p, q in zip(x[2], x[3])), lsub(x[3], x[2])
+        fadd, fsub = lambda p, q: fold61(u64(p + q)), lambda p, q: fold61(u64(p + u64(k4 - q)))
+        return [(fadd(v0[0], v2[0]), fadd(v0[1], v2[1])), (fsub(v1[0], v3[1]), fadd(v1[1], v3[0])),
+                (fsub(v0[0], v2[0]), fsub(v0[1], v2[1])), (fadd(v1[0], v3[1]), fsub(v1[1], v3[0]))]
+
+    a, b = dit_adds(y[:4]), dit_adds(y[4:])
+    b = [b[0], eighth_conj(b[1]), times_i(b[2]), times_i(eighth_conj(b[3]))]
+    return [add(a[0], b[0]), add(a[1], b[1]), sub(a[2], b[2]), sub(a[3], b[3]),
+            sub(a[0], b[0]), sub(a[1], b[1]), add(a[2], b[2]), add(a[3], b[3])]
+
+
+def test_radix8_ranges_and_value():
+    w = [(1, 0)]
+    for _ in range(7):
+        p, q = w[-1]
+        w.append(((p - q << 30) % P61, (p + q << 30) % P61))
+    assert w[2] == (0, 1)
+    rng = random.Random(8)
+    ends = (0, 1, P61, P61 + 8)
+    cases = [[(rng.choice(ends), rng.choice(ends)) for _ in range(8)] for _ in range(4000)]
+    cases += [[(rng.randrange(P61 + 9), rng.randrange(P61 + 9)) for _ in range(8)] for _ in range(1000)]
+    for u in cases:
+        y = radix8(u)
+        for k, e in enumerate((0, 4, 2, 6, 1, 5, 3, 7)):
+            re = sum(u[m][0] * w[m * e % 8][0] - u[m][1] * w[m * e % 8][1] for m in range(8))
+            im = sum(u[m][0] * w[m * e % 8][1] + u[m][1] * w[m * e % 8][0] for m in range(8))
+            assert y[k][0] <= P61 + 8 and y[k][1] <= P61 + 8
+            assert (y[k][0] - re) % P61 == 0 and (y[k][1] - im) % P61 == 0
+        x = unradix8(y)
+        for m in range(8):
+            for c in range(2):
+                assert x[m][c] <= P61 + 8 and (x[m][c] - 8 * u[m][c]) % P61 == 0
+        unradix8(u)                          # ranges alone
