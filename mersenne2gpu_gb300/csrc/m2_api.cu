@@ -1023,7 +1023,7 @@ int tune_bucket(int device, u64 h, const std::vector<Item>& items, const std::ve
     const u64 n = 2 * h;
     // A batch of at least a test per SM is timed as a full GPU, the bucket's tests
     // repeated: a last wave that is not full would count against the kernel with
-    // more tests per SM (n = 4096, 498 tests, m2_duo.cu: 143 ns per test-squaring, 118 in full waves).
+    // more tests per SM (n = 4096, 498 tests, m2_duo.cu: 143 ns per test-squaring for 118 in full waves).
     const size_t full = (size_t)std::max(sms, 1) * std::min<size_t>(32, std::max<size_t>(1, 232448 / (24 * h)));
     const size_t cap = total >= (size_t)sms ? full : items.size();
     long long* scratch = nullptr;

@@ -6,15 +6,18 @@
 // SM.  Here a thread runs a butterfly in GF(P61^2), then the same one in
 // GF(P31^2): 64 registers, 32 warps an SM.  The transform's middle (last
 // forward level, centre square, first inverse level) is one pass over mirror
-// blocks, and a level waits only for the warps that wrote its blocks.
+// blocks, and a radix-4 level waits only for the warps that wrote its blocks.
+// From n = 4096 on the first two levels are radix-8, a butterfly or two per
+// thread (118 -> 111 and 256 -> 238 ns below); at smaller sizes that would
+// halve the threads (n = 2048: 53.7 -> 56.4, 1024 27.7 -> 30.1).
 //
 // What bounds it: the SM's integer pipes (n = 4096: 72% of the cycles, the
 // multiplier another 30%, 23 warps an SM).  Measured, ns per test-squaring of a
 // full GPU, the one-CTA kernel's best combination -> here:
 //   n    256        512          1024         2048         4096       8192
-//        7.5 -> 6.2 15.3 -> 13.0 30.9 -> 27.7 63.4 -> 53.7 138 -> 118 287 -> 256
+//        7.5 -> 6.2 15.3 -> 13.0 30.9 -> 27.7 63.4 -> 53.7 138 -> 111 287 -> 238
 // and us per squaring of a lone test: 5.9 -> 6.6, 6.4 -> 6.8 (n = 256, 512),
-// 12.3 -> 10.3, 24.6 -> 22.2, 51.7 -> 45.0 (n = 2048 ... 8192).
+// 12.3 -> 10.2, 24.6 -> 21.2, 51.7 -> 41.5 (n = 2048 ... 8192).
 #include "m2_flow.cuh"
 
 namespace M2K_NS {
@@ -23,12 +26,18 @@ namespace {
 
 template <int A_> struct Shape {
     static constexpr int A = A_;
-    static constexpr u32 H = 1u << A, NB = H / 4, NF = NB > 256 ? 256 : NB, NT = NF;
+    static constexpr u32 H = 1u << A, NB = H / 4;
+    static constexpr bool R8 = A >= 11, NARROW = true, ODD = (A & 1) != 0;   // R8: the first two levels are radix-8
+    static constexpr u32 NT = NB > 256 ? 256 : NB, NF = NT;
     static constexpr u32 EP = H / NT;                    // consecutive elements of a thread in the row stage
-    static constexpr bool NARROW = true, ODD = (A & 1) != 0;
-    static constexpr int NL = A / 2 - (ODD ? 0 : 1);     // radix-4 levels outside the middle
-    static constexpr u32 SMEM = 24 * H;
+    static constexpr int FIRST = R8 ? 3 : 0;             // radix-4 levels FIRST ... NL - 1 outside the middle
+    static constexpr int NL = A / 2 - (ODD ? 0 : 1);
+    static constexpr u32 SMEM = 24 * H, FIT = 232448 / (SMEM + 8 * NT + 1040), PER = 1024 / NT < FIT ? 1024 / NT : FIT;   // CTAs of an SM
 };
+
+// the radix-8 level's twiddles w_64^(a br_8(j)), at 7 j + a - 1 from here: in the
+// part of the radix-4 table that belongs to no level (32 ... 63 blocks)
+constexpr u32 TW8_AT = 3 * 32;
 
 // XOR swizzle of the slots (as sw, m2_flow.cuh): also for threads 8 elements apart
 __host__ __device__ constexpr u32 swd(u32 e) {
@@ -48,6 +57,26 @@ template <class S, class X> struct Whole {
     template <class F> __device__ __forceinline__ void each(F&& f) const {
 #pragma unroll 1
         for (u32 b = threadIdx.x; b < S::NB; b += S::NT) f(b);
+    }
+    // radix-8 level l = 0, 1: blocks of H / 8^l
+    template <bool FWD> __device__ __forceinline__ void level8(int l) const {
+        const u32 M = S::H >> (3 * l), Q = M / 8;
+#pragma unroll 1
+        for (u32 b = threadIdx.x; b < S::H / 8; b += S::NT) {
+            const u32 s0 = swd(b / Q * M + b % Q);
+            X x[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) x[m] = z[s0 ^ swd(m * Q)];
+            if (!FWD) dit8_adds(x);
+            if (l > 0) {
+                const DTw* t = tw4 + TW8_AT + 7 * (b / Q);
+                if (FWD) twist8(x, t);
+                else untwist8(x, t);
+            }
+            if (FWD) dif8_adds(x);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) z[s0 ^ swd(m * Q)] = x[m];
+        }
     }
     __device__ __forceinline__ void fwd_level(int l) const {
         const u32 M = S::H >> (2 * l), Q = M / 4;
@@ -171,10 +200,20 @@ template <class S> __device__ __forceinline__ void run_duo(const SmallTest& T, u
             zb[p] = weigh31(d.x, d.y, s31);
             zb[q] = weigh31(f.x, f.y, s31 >> 16);
         }
-        __syncthreads();
+        if (S::R8) {
 #pragma unroll
-        for (int l = 0; l < S::NL; ++l) {
-            if (l > 0) sync_group<S>(S::H >> (2 * l), t, 1);
+            for (int l = 0; l < 2; ++l) {
+                __syncthreads();
+                ua.template level8<true>(l);
+                asm_fence();
+                ub.template level8<true>(l);
+                asm_fence();
+            }
+        }
+#pragma unroll
+        for (int l = S::FIRST; l < S::NL; ++l) {
+            if (l == S::FIRST) __syncthreads();
+            else sync_group<S>(S::H >> (2 * l), t, 1);
             ua.fwd_level(l);
             asm_fence();
             ub.fwd_level(l);
@@ -186,12 +225,22 @@ template <class S> __device__ __forceinline__ void run_duo(const SmallTest& T, u
         ub.middle();
         __syncthreads();
 #pragma unroll
-        for (int l = S::NL - 1; l >= 0; --l) {
+        for (int l = S::NL - 1; l >= S::FIRST; --l) {
             if (l < S::NL - 1) sync_group<S>((S::H >> (2 * l)) / 4, t, 1);
             ua.inv_level(l);
             asm_fence();
             ub.inv_level(l);
             asm_fence();
+        }
+        if (S::R8) {
+#pragma unroll
+            for (int l = 1; l >= 0; --l) {
+                if (l == 0 || S::NL > S::FIRST) __syncthreads();
+                ua.template level8<false>(l);
+                asm_fence();
+                ub.template level8<false>(l);
+                asm_fence();
+            }
         }
         __syncthreads();
         // unweight, CRT, carry chain of the thread's digits; the carry to the next thread
@@ -234,7 +283,7 @@ template <class S> __device__ __forceinline__ void run_duo(const SmallTest& T, u
 // One CTA per test (queue == nullptr), or a persistent grid whose CTAs take
 // test indices from *queue until all `ntests` are done (as k_small).
 template <class S>
-__global__ void __launch_bounds__(S::NT, 1024 / S::NT) k_duo(const SmallTest* tests, int ntests, u32 iters_override, int* queue) {
+__global__ void __launch_bounds__(S::NT, S::PER) k_duo(const SmallTest* tests, int ntests, u32 iters_override, int* queue) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ i64 cx[S::NT];
     __shared__ int s_next;
@@ -257,8 +306,13 @@ __global__ void __launch_bounds__(S::NT, 1024 / S::NT) k_duo(const SmallTest* te
     }
 }
 
+// Every size asks for all of the SM's shared memory.  Left to the driver, the
+// sizes of one batch get different splits, an SM keeps its split while a CTA is
+// on it, and the later size's CTAs crowd onto the SMs that have theirs (502
+// tests of n = 512 with 106 of n = 256: 6.95 ms for 2.2 here).
 template <class S> cudaError_t prepare() {
-    return cudaFuncSetAttribute(k_duo<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    const cudaError_t e = cudaFuncSetAttribute(k_duo<S>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_duo<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
 }
 template <class S> int resident() {
     int nb = 0;
@@ -283,7 +337,12 @@ template <class S> cudaError_t launch(const SmallTest* d_tests, int ntests, u32 
 // outgrows a third of an SM's shared memory.  A thread's segment has 8 digits or
 // more: carry spans of up to 7 (the tests of these sizes have 2 or 3).
 bool duo_supported(unsigned h, int span, int carry_threads) { return h >= 128 && h <= 4096 && span <= 7 && carry_threads > 0; }
-int duo_threads(unsigned h) { return (int)(h / 4 > 256 ? 256 : h / 4); }
+int duo_threads(unsigned h) {
+#define M2_DUO_N(A) if (h == 1u << A) return (int)Shape<A>::NT;
+    M2_DUO_SIZES(M2_DUO_N)
+#undef M2_DUO_N
+    return 0;
+}
 int duo_ctas_per_sm(unsigned h) {
 #define M2_DUO_R(A) if (h == 1u << A) return resident<Shape<A>>();
     M2_DUO_SIZES(M2_DUO_R)

@@ -1,5 +1,6 @@
 // m2_split.cuh -- the dual field's arithmetic one field at a time, for kernels
-// that run the two halves on separate warps (m2_flow.cu, m2_lane.cu).
+// that run the two halves on separate warps or in turn (m2_flow.cu, m2_tide.cu,
+// m2_lane.cu, m2_cluster.cu, m2_duo.cu).
 #pragma once
 #include "m2_field.cuh"
 #include "m2_kernels.cuh"
@@ -101,6 +102,77 @@ template <class X> __device__ __forceinline__ Tri<X> ldtri(const DTw* tw4, u32 b
 // the weighted element of digits d0, d1; s: their shifts in bytes 0 and 1
 __device__ __forceinline__ X61 weigh61(i64 d0, i64 d1, u32 s) { return X61{rotl61(digit_to61(d0), s & 0xffu), rotl61(digit_to61(d1), (s >> 8) & 0xffu)}; }
 __device__ __forceinline__ X31 weigh31(i64 d0, i64 d1, u32 s) { return X31{rotl31(digit_to31(d0), s & 0xffu), rotl31(digit_to31(d1), (s >> 8) & 0xffu)}; }
+
+// ---- radix-8 levels ----
+// Three levels of the per-block-twiddle transform at once: with r^8 = c the
+// residues mod X^m - r w^e, w = (1 + i) / sqrt 2, e = 0, 4, 2, 6, 1, 5, 3, 7.
+// sqrt 2 is 2^31 in GF(P61) and 2^16 in GF(P31): a product by w is an
+// addition, a subtraction and two shifts, and 7 products by twiddles do the
+// work of 9 in radix-4 levels.
+//
+// x below 7 2^61 times 2^30 modulo P61, below 2^61 + 2^33
+__device__ __forceinline__ u64 scale61(u64 x) { return ((x & 0x7fffffffull) << 30) + (x >> 31); }
+__device__ __forceinline__ u32 scale31(u32 x) { return rotl31(x, 15); }
+// w (x - y): the difference offset by 2 P61 (below 3 2^61 + 8), the sum and the
+// difference of its coordinates (offset by 4 P61) below 7 2^61 + 16
+__device__ __forceinline__ X61 eighth_of_diff(const X61& x, const X61& y) {
+    const L61 d = lsub(x.a, x.b, y.a, y.b);
+    return X61{scale61(d.a + (K4_61 - d.b)), scale61(d.a + d.b)};
+}
+__device__ __forceinline__ X31 eighth_of_diff(const X31& x, const X31& y) {
+    const X31 d = xsub(x, y);
+    return X31{scale31(sub31(d.c, d.d)), scale31(add31(d.c, d.d))};
+}
+// conj(w) x, x below 2^61 + 8
+__device__ __forceinline__ X61 eighth_conj(const X61& x) { return X61{scale61(x.a + x.b), scale61(x.b + (K2_61 - x.a))}; }
+__device__ __forceinline__ X31 eighth_conj(const X31& x) { return X31{scale31(add31(x.c, x.d)), scale31(sub31(x.d, x.c))}; }
+
+// i x, x below 2 P61
+__device__ __forceinline__ X61 times_i(const X61& x) { return X61{K2_61 - x.b, x.a}; }
+__device__ __forceinline__ X31 times_i(const X31& x) { return xtimes_i(x); }
+
+template <class X> __device__ __forceinline__ void dif8_adds(X (&x)[8]) {
+    X a[4], b[4];
+    a[0] = xadd(x[0], x[4]); b[0] = xsub(x[0], x[4]);
+    a[1] = xadd(x[1], x[5]); b[1] = eighth_of_diff(x[1], x[5]);
+    a[2] = xadd(x[2], x[6]); b[2] = times_i(xsub(x[2], x[6]));
+    a[3] = xadd(x[3], x[7]); b[3] = times_i(eighth_of_diff(x[3], x[7]));
+    dif_adds(a, a[1], a[2], a[3]);
+    dif_adds(b, b[1], b[2], b[3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { x[k] = a[k]; x[4 + k] = b[k]; }
+}
+template <class X> __device__ __forceinline__ void dit8_adds(X (&x)[8]) {
+    X a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { a[k] = x[k]; b[k] = x[4 + k]; }
+    dit_adds(a);
+    dit_adds(b);
+    b[1] = eighth_conj(b[1]);
+    b[2] = times_i(b[2]);                  // its negative: -i b[2] is taken off
+    b[3] = times_i(eighth_conj(b[3]));
+    x[0] = xadd(a[0], b[0]); x[4] = xsub(a[0], b[0]);
+    x[1] = xadd(a[1], b[1]); x[5] = xsub(a[1], b[1]);
+    x[2] = xsub(a[2], b[2]); x[6] = xadd(a[2], b[2]);
+    x[3] = xsub(a[3], b[3]); x[7] = xadd(a[3], b[3]);
+}
+// x[k] times entry k - 1 of t (its conjugate)
+template <class X> __device__ __forceinline__ void twist8(X (&x)[8], const DTw* t) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        X w;
+        ldtw(w, t, k - 1);
+        x[k] = xmul(x[k], w);
+    }
+}
+template <class X> __device__ __forceinline__ void untwist8(X (&x)[8], const DTw* t) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        X w;
+        ldtw(w, t, k - 1);
+        x[k] = xmulc(x[k], w);
+    }
+}
 
 // named barrier of N threads
 template <u32 N> __device__ __forceinline__ void bar_field(u32 id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }

@@ -34,6 +34,8 @@ __device__ __forceinline__ void put_tw(DTw* t, u32 i, const E& v) { t[i] = DTw{f
 // h with per-block twiddles (natural order in, bit-reversed out):
 //   tw4[3*(S+j) + a-1] = r^a, r = w_{4S}^{br_S(j)}, for every radix-4 step with
 //                        S blocks before the step (S = 1, 4, 16, ...)
+//   tw4[96 + 7*j + a-1] = w_64^(a br_8(j)), j < 8, a = 1 ... 7: the radix-8 step
+//                        with 8 blocks before it (m2_duo.cu), for h >= 2048
 //   tc[j]              = w_h^{br_{h/2}(j)}, j < h/2: the centre twiddle of
 //                        position 2j; also the radix-2 step's twiddle when
 //                        log2 h is odd.
@@ -44,6 +46,14 @@ __global__ void __launch_bounds__(256) k_twiddles(DTw* tw4, DTw* tc, u32 h, int 
         if (t == 0) continue;
         const int sb = 31 - __clz(t);
         const u32 S = 1u << sb;
+        if (sb == 3 && h >= 2048u) {
+            const E r = dpow(wh, (u64)(h / 64u) * brev(t - S, 3));
+            E q = r;
+            for (u32 a = 0; a < 7; ++a) {
+                put_tw(tw4, 96u + 7u * (t - S) + a, q);
+                q = emul(q, r);
+            }
+        }
         if ((sb & 1) == 0 && 4u * S <= h) {
             const E r = dpow(wh, (u64)(h / (4u * S)) * brev(t - S, sb));
             const E r2 = esqr(r), r3 = emul(r2, r);

@@ -79,7 +79,7 @@ def scale61(x):
 
 
 def radix8(u):
-    """dif8_adds of m2_tide.cu in GF(P61^2), every step as there."""
+    """dif8_adds of m2_split.cuh in GF(P61^2), every step as there."""
     k2, k4 = 2 * P61, 4 * P61
     add = lambda x, y: tuple(fold61(u64(p + q)) for p, q in zip(x, y))
     lsub = lambda x, y: tuple(u64(p + u64(k2 - q)) for p, q in zip(x, y))
@@ -103,7 +103,7 @@ def radix8(u):
 
 
 def unradix8(y):
-    """dit8_adds of m2_tide.cu in GF(P61^2)."""
+    """dit8_adds of m2_split.cuh in GF(P61^2)."""
     k2, k4 = 2 * P61, 4 * P61
     add = lambda x, z: tuple(fold61(u64(p + q)) for p, q in zip(x, z))
     lsub = lambda x, z: tuple(u64(p + u64(k2 - q)) for p, q in zip(x, z))
