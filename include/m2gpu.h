@@ -347,13 +347,16 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
 
 /* Threads per transform that m2_batch_run chose for transform size 2^ln on
  * `device` (autotuned on the first batch containing that size: every candidate
- * 32 ... 256 times a sample of the batch's own tests; the carry split follows),
+ * 32 ... 256 times a sample of the batch's own tests; the carry split follows;
+ * the fields-in-turn kernel's 512 and 1024 threads at ln = 13, 14 read 256),
  * and the measured nanoseconds per test-squaring.  M2_EINVAL if not tuned yet. */
 int m2_batch_tuned(int device, int ln, int* threads, double* ns_per_test_iter);
 
 /* The full choice of the batch autotuner for transform size 2^ln on `device`
- * (M2_EINVAL if not tuned yet).  The tuner times every valid combination of
- * three knobs on a sample of the batch's own tests:
+ * (M2_EINVAL if not tuned yet).  The tuner times the kernel that runs the two
+ * fields in turn (ln = 8 ... 14; one segment per thread, fused middle) and, where
+ * that does not already win on a full GPU, every valid combination of three
+ * knobs of the kernel that runs them together, on a sample of the batch's own tests:
  *   threads        threads per transform (the reference's -W work-group size,
  *                  mersenne2_gpu.cpp:3668-3672), 32 ... 256;
  *   carry_blocks   segments of the carry, each normalising n / carry_blocks

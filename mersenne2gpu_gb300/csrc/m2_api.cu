@@ -996,7 +996,10 @@ namespace {
 // test-squarings per second wins.  Cached for the process.
 struct Tuned {
     int threads = 0, carry_shift = 0, fuse = 0;
-    bool duo = false;            // the kernel of m2_duo.cu (its middle is fused, its carry has a segment per thread)
+    // the kernel of m2_duo.cu: its middle is fused, its carry has a segment per
+    // thread, and its 512 or 1024 threads at h = 4096, 8192 count as 256, the
+    // most that a caller may ask for
+    bool duo = false;
     double ns_per_test_iter = 0.0, ns_default = 0.0;
     int carry_blocks(const m2::Layout& L, int span) const { return small_carry_threads(L, span, threads, carry_shift); }
 };
@@ -1099,7 +1102,7 @@ int tune_bucket(int device, u64 h, const std::vector<Item>& items, const std::ve
         double ns_per = 0.0;
         e = rate(ns, [&](u32 iters) { return m2k::launch_duo(d_t, (int)ns, (unsigned)h, iters, st); }, ns_per);
         if (ns_per < best.ns_per_test_iter) {
-            best.threads = m2k::duo_threads((unsigned)h); best.carry_shift = 0; best.fuse = 1; best.duo = true;
+            best.threads = std::min(m2k::duo_threads((unsigned)h), 256); best.carry_shift = 0; best.fuse = 1; best.duo = true;
             best.ns_per_test_iter = ns_per;
         }
     }
@@ -1264,10 +1267,10 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         Tuned tn;
         const std::vector<m2k::SmallTest> mine(tests.begin() + l.first, tests.begin() + l.first + l.ntests);
         if ((rc = tune_bucket(device, l.h, items, mine, l.d_dig, sms, count, tn))) return rc;
-        l.threads = tn.threads;
-        l.fuse = tn.fuse != 0;
         // the choice is cached per size: these tests may have one it does not serve
         l.duo = tn.duo && duo_for(mine);
+        l.threads = tn.threads;
+        l.fuse = tn.fuse != 0;
         for (int t = 0; t < l.ntests; ++t) {
             tests[l.first + t].carry_threads = small_carry_threads(items[t].L, items[t].span, tn.threads, tn.carry_shift);
             tests[l.first + t].fuse_middle = tn.fuse;
@@ -1474,10 +1477,10 @@ int srv_launch(m2_server* s) {
             auto f = g_tune.find({s->device, kv.first});
             if (f != g_tune.end()) { tn = f->second; tuned = true; }
         }
-        const int threads = tuned ? tn.threads : c0->threads;
-        const bool fuse = tuned ? tn.fuse != 0 : c0->h_test.fuse_middle != 0;
         bool duo = !tuned || tn.duo;
         for (size_t j = 0; j < cnt && duo; ++j) duo = duo_for({s->active[kv.second[j]].ctx->h_test});
+        const int threads = tuned ? tn.threads : c0->threads;
+        const bool fuse = tuned ? tn.fuse != 0 : c0->h_test.fuse_middle != 0;
         for (size_t j = 0; j < cnt; ++j) {
             SrvItem& it = s->active[kv.second[j]];
             b.ks[j] = std::min(s->quantum, it.total - it.done);

@@ -1,23 +1,24 @@
 // m2_duo.cu -- one test per CTA for the shared launches of batches and the
-// server (n = 256 ... 8192), the two fields one after the other.
+// server (n = 256 ... 16384), the two fields one after the other.
 //
 // The one-CTA kernel of m2_kernels.cu holds an element's four words and a
 // butterfly's twiddles of both fields at once: 106-128 registers, 16 warps an
-// SM.  Here a thread runs a butterfly in GF(P61^2), then the same one in
-// GF(P31^2): 64 registers, 32 warps an SM.  The transform's middle (last
-// forward level, centre square, first inverse level) is one pass over mirror
-// blocks, and a radix-4 level waits only for the warps that wrote its blocks.
-// From n = 4096 on the first two levels are radix-8, a butterfly or two per
-// thread (118 -> 111 and 256 -> 238 ns below); at smaller sizes that would
-// halve the threads (n = 2048: 53.7 -> 56.4, 1024 27.7 -> 30.1).
+// SM (8 at n = 16384).  Here a thread runs a butterfly in GF(P61^2), then the
+// same one in GF(P31^2): 64 registers, 32 warps an SM.  The transform's middle
+// (last forward level, centre square, first inverse level) is one pass over
+// mirror blocks, and a radix-4 level waits only for the warps that wrote its
+// blocks.  From n = 4096 on the first two levels are radix-8, a butterfly per
+// thread (n = 4096 118 -> 111 ns below); at smaller sizes that would halve the
+// threads (n = 2048: 53.7 -> 56.4, 1024 27.7 -> 30.1).
 //
 // What bounds it: the SM's integer pipes (n = 4096: 72% of the cycles, the
 // multiplier another 30%, 23 warps an SM).  Measured, ns per test-squaring of a
 // full GPU, the one-CTA kernel's best combination -> here:
-//   n    256        512          1024         2048         4096       8192
-//        7.5 -> 6.2 15.3 -> 13.0 30.9 -> 27.7 63.4 -> 53.7 138 -> 111 287 -> 238
+//   n    256  512   1024  2048  4096  8192  16384
+//        7.5  15.3  30.9  63.4  138   287   689
+//     -> 6.2  13.0  27.7  53.7  111   229   494
 // and us per squaring of a lone test: 5.9 -> 6.6, 6.4 -> 6.8 (n = 256, 512),
-// 12.3 -> 10.2, 24.6 -> 21.2, 51.7 -> 41.5 (n = 2048 ... 8192).
+// 12.3 -> 10.2, 24.6 -> 21.2, 51.7 -> 36.6, 104 -> 75 (n = 2048 ... 16384).
 #include "m2_flow.cuh"
 
 namespace M2K_NS {
@@ -28,7 +29,7 @@ template <int A_> struct Shape {
     static constexpr int A = A_;
     static constexpr u32 H = 1u << A, NB = H / 4;
     static constexpr bool R8 = A >= 11, NARROW = true, ODD = (A & 1) != 0;   // R8: the first two levels are radix-8
-    static constexpr u32 NT = NB > 256 ? 256 : NB, NF = NT;
+    static constexpr u32 NT = R8 ? H / 8 : NB, NF = NT;
     static constexpr u32 EP = H / NT;                    // consecutive elements of a thread in the row stage
     static constexpr int FIRST = R8 ? 3 : 0;             // radix-4 levels FIRST ... NL - 1 outside the middle
     static constexpr int NL = A / 2 - (ODD ? 0 : 1);
@@ -329,14 +330,14 @@ template <class S> cudaError_t launch(const SmallTest* d_tests, int ntests, u32 
     return cudaGetLastError();
 }
 
-#define M2_DUO_SIZES(X) X(7) X(8) X(9) X(10) X(11) X(12)
+#define M2_DUO_SIZES(X) X(7) X(8) X(9) X(10) X(11) X(12) X(13)
 
 }  // namespace
 
-// h = 128 ... 4096: below, a warp has no block for each lane; above, the state
-// outgrows a third of an SM's shared memory.  A thread's segment has 8 digits or
-// more: carry spans of up to 7 (the tests of these sizes have 2 or 3).
-bool duo_supported(unsigned h, int span, int carry_threads) { return h >= 128 && h <= 4096 && span <= 7 && carry_threads > 0; }
+// h = 128 ... 8192: below, a warp has no block for each lane; above, the state
+// outgrows an SM's shared memory.  A thread's segment has 8 digits or more:
+// carry spans of up to 7 (the tests of these sizes have 2 or 3).
+bool duo_supported(unsigned h, int span, int carry_threads) { return h >= 128 && h <= 8192 && span <= 7 && carry_threads > 0; }
 int duo_threads(unsigned h) {
 #define M2_DUO_N(A) if (h == 1u << A) return (int)Shape<A>::NT;
     M2_DUO_SIZES(M2_DUO_N)

@@ -1,11 +1,12 @@
 """The fields-in-turn kernel of shared launches (m2_duo.cu: batches and the
-server, n = 2^8 ... 2^13) against the same tests run alone."""
+server, n = 2^8 ... 2^14) against the same tests run alone."""
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 # (log2 n, smallest and largest odd exponent of that transform)
-SIZES = [(8, 5377, 10495), (9, 10497, 20991), (10, 20993, 40959), (11, 40961, 81919), (12, 81921, 159743), (13, 159745, 319487)]
+SIZES = [(8, 5377, 10495), (9, 10497, 20991), (10, 20993, 40959), (11, 40961, 81919), (12, 81921, 159743), (13, 159745, 319487),
+         (14, 319489, 622591)]
 
 
 @pytest.mark.parametrize("ln,lo,hi", SIZES)
