@@ -540,7 +540,7 @@ def run_gb300(a, dist: Dist) -> dict | None:
         "warmup": a.warmup, "ms_per_step": dev_ms / a.steps, "higher_is_better": False,
         "scaling": "weak", "vs_baseline": None, "dtype": "u64",
         "data": "synthetic (fixed exponent, state from x0 = 3)",
-        "config": {"workload": WORKLOAD, "iters_per_step": ips, "path": "three-pass",
+        "config": {"workload": WORKLOAD, "iters_per_step": ips, "path": "three-pass" if len(stages) > 1 else "one launch",
                    "plan": {"rows": info.rows, "row_len": info.row_len, "cols_per_cta": info.cols_per_cta,
                             "carry_span": info.span},
                    "l2": f"flushed between steps ({L2_FLUSH_BYTES >> 20} MB write), state stays L2-resident within a step",

@@ -33,7 +33,8 @@ extern "C" {
  * gf61_ntt_prp_opencl_inplace_nobitrev_fused.cpp:508-531. */
 enum { M2_MODE_LL = 0, M2_MODE_PRP = 1, M2_MODE_PRP3 = 2 };
 
-/* execution path selection (0 = automatic) */
+/* execution path selection.  AUTO picks the fastest kernel of a lone test's size;
+ * SMALL asks for the one-CTA kernel, LARGE for the three-pass kernels */
 enum { M2_PATH_AUTO = 0, M2_PATH_SMALL = 1, M2_PATH_LARGE = 2 };
 
 /* fields of the transform: GF(P61^2) x GF(P31^2) recombined by CRT (the
@@ -83,7 +84,8 @@ typedef struct {
     uint64_t n;             /* digits */
     uint32_t iteration;     /* squarings applied so far */
     uint32_t total_iters;   /* p-2 (LL), p (PRP), p-1 (PRP3) (mersenne2_gpu.cpp:4780) */
-    int path;               /* M2_PATH_SMALL or M2_PATH_LARGE */
+    int path;               /* M2_PATH_SMALL or M2_PATH_LARGE: the plan whose buffers and hooks the context has (AUTO
+                               runs faster kernels of its own on either) */
     uint32_t rows, row_len, cols_per_cta, span;   /* large-path plan */
     uint64_t device_bytes;  /* device memory held by the context */
     uint32_t fused_cols;    /* 1: the inverse column pass and the next forward one run as one launch */
