@@ -463,9 +463,11 @@ namespace {
 struct Gate {
     std::mutex mu;
     cudaEvent_t one_ev = nullptr;          // end of the last one-launch run
-    cudaStream_t one_stream = nullptr;     // its stream
+    cudaStream_t one_stream = nullptr;     // its stream; GONE once that context is destroyed (the handle may come back)
     std::set<m2_ctx*> passes;              // contexts with a recorded gate_ev
+    std::vector<cudaEvent_t> left;         // gate_ev of contexts destroyed with work in flight
 };
+const cudaStream_t GONE = reinterpret_cast<cudaStream_t>(~uintptr_t(0));
 std::mutex g_gate_mu;
 std::map<int, std::unique_ptr<Gate>> g_gate;
 Gate& gate_of(int device) {
@@ -492,6 +494,11 @@ template <class F> cudaError_t in_turn(m2_ctx* c, F&& enqueue) {
     if (one) {
         for (m2_ctx* o : g.passes)
             if (e == cudaSuccess && o != c) e = cudaStreamWaitEvent(c->stream, o->gate_ev, 0);
+        for (cudaEvent_t ev : g.left) {
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev, 0);
+            cudaEventDestroy(ev);
+        }
+        g.left.clear();
         if (e == cudaSuccess && !g.one_ev) e = cudaEventCreateWithFlags(&g.one_ev, cudaEventDisableTiming);
     } else if (e == cudaSuccess && !c->gate_ev) {
         e = cudaEventCreateWithFlags(&c->gate_ev, cudaEventDisableTiming);
@@ -510,8 +517,16 @@ void leave_gate(m2_ctx* c) {
     Gate& g = gate_of(c->device);
     std::lock_guard<std::mutex> lk(g.mu);
     g.passes.erase(c);
-    if (c->gate_ev) cudaEventDestroy(c->gate_ev);
+    if (g.one_stream == c->stream) g.one_stream = GONE;
+    if (c->gate_ev) g.left.push_back(c->gate_ev);
     c->gate_ev = nullptr;
+    for (size_t i = 0; i < g.left.size();) {
+        if (cudaEventQuery(g.left[i]) == cudaErrorNotReady) { ++i; continue; }
+        cudaEventDestroy(g.left[i]);
+        g.left[i] = g.left.back();
+        g.left.pop_back();
+    }
+    cudaGetLastError();
 }
 
 }  // namespace
