@@ -21,13 +21,13 @@ CLI = os.path.join(PKG, "mersenne2")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CU_SOURCES = ["m2_kernels.cu", "m2_rows.cu", "m2_cols.cu", "m2_flow.cu", "m2_lane.cu", "m2_cluster.cu", "m2_tide.cu",
-              "m2_duo.cu", "m2_tables.cu", "m2_carry.cu", "m2_api.cu", "m2_peaks.cu", "m2_noalloc.cu",
+              "m2_duo.cu", "m2_pass.cu", "m2_tables.cu", "m2_carry.cu", "m2_api.cu", "m2_peaks.cu", "m2_noalloc.cu",
               "m2_gec.cu"]
 CXX_SOURCES = ["m2_host.cpp"]
 # the transform kernels, built a second time for the GF(P61^2)-only layout
 # (-DM2_DUAL=0: namespace m2k_g61, the GF(P31^2) half compiled away)
 GF61_SOURCES = ["m2_kernels.cu", "m2_rows.cu", "m2_cols.cu", "m2_flow.cu", "m2_lane.cu",
-                "m2_cluster.cu", "m2_tide.cu"]
+                "m2_cluster.cu", "m2_tide.cu", "m2_pass.cu"]
 
 
 def nvcc() -> str:

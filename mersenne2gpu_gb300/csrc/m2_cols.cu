@@ -422,10 +422,10 @@ __global__ void __launch_bounds__(ColShape<CR>::CNT, 65536 / (64 * ColShape<CR>:
     fwd_passes<CR>(z, P, bf, g);
 }
 
-// R = 256 only with rows of 1024 or more: below that (G <= 128 CTAs of 128
-// threads) the generic kernels' larger CTAs measured faster
+// R = 256 only with rows of 1024 or more, and not where passes with the fields
+// in turn are asked for (m2_pass.cu, faster at every R = 256)
 bool cols_q_supported(const LargePlan& P) {
-    return (P.R == 1024u || (P.R == 256u && P.B >= 1024u)) && P.C == (u32)CC && P.span < 2 * CC;
+    return (P.R == 1024u || (P.R == 256u && P.B >= 1024u && !P.in_turn)) && P.C == (u32)CC && P.span < 2 * CC;
 }
 
 namespace {

@@ -51,6 +51,8 @@ template <int LR_, int LB_, int C_> struct Shape {
     static constexpr bool BOTH = NB0 >= 1024;
     static constexpr u32 NF = BOTH ? 1024 : NB0 < 32 ? 32 : NB0;   // threads per field
     static constexpr u32 NT = kDual && !BOTH ? 2 * NF : NF;
+    static constexpr bool EARLY = NT <= 512;                 // registers to spare: twiddles before the barrier
+    static constexpr u32 ROW_TAG = 1;
     static constexpr u32 SEGS = UC / 2;                      // carry segments (2 elements, 4 digits) of a column group
     static constexpr u32 SI = (SEGS + NT - 1) / NT;          // segments per thread
     static constexpr u32 SR = C / 2;                         // segments per row

@@ -105,16 +105,15 @@ template <class S, class X> struct Unit {
     // registers the other warps hide them (h = 2^19: 62.3 -> 60.1 us).
     template <u32 ITERS, u32 NB, class TW, class LD, class OP, class ST>
     __device__ __forceinline__ void level(u32 group, TW&& tw, LD&& ld, OP&& op, ST&& st) const {
-        constexpr bool EARLY = S::NT <= 512;
+        constexpr bool EARLY = S::EARLY;
         Tri<X> t;
         const bool on = NB % S::NF == 0 || fb < NB;
         if (EARLY && on) tw(fb, t);
         if (group) sync_group<S>(group, fb, bar);
         if (!on) return;
-        if (ITERS == 1 && S::NT <= 512) {
+        if (ITERS == 1 && EARLY) {
             X x[4];
             ld(fb, x);
-            if (!EARLY) tw(fb, t);
             op(x, t);
             st(fb, x);
         } else {
@@ -165,7 +164,7 @@ template <class S, class X> struct Unit {
                   [&](u32 b, X (&x)[4]) {
                       const u32 rho = b / S::C, cc = b % S::C;
                       if (l == NL - 1) {
-                          take<1>(x, g + (u64)(4 * rho) * S::B + cg * S::C + cc, S::B, w);
+                          take<S::ROW_TAG>(x, g + (u64)(4 * rho) * S::B + cg * S::C + cc, S::B, w);
                       } else {
                           const u32 s0 = sw((rho / Q * M + rho % Q) * S::C + cc);
 #pragma unroll
@@ -240,7 +239,7 @@ template <class S, class X> struct Unit {
                       } else {
                           X* p = g + (u64)(sl ? t1 : t0) * S::B + rho;
 #pragma unroll
-                          for (int m = 0; m < 4; ++m) st_tagged<1>(p + m * Q, x[m]);
+                          for (int m = 0; m < 4; ++m) st_tagged<S::ROW_TAG>(p + m * Q, x[m]);
                       }
                   });
         }

@@ -675,11 +675,13 @@ cudaError_t launch_large_stage(const LargePlan& P, const LargeBufs& b, int stage
     const size_t sc = large_smem_cols(P), sr = large_smem_rows(P);
     if (stage == STAGE_MID) return b.flags ? launch_cols_mid(P, b, s) : cudaErrorInvalidValue;
     if (stage != 1 && cols_q_supported(P)) return launch_cols_q(P, b, stage == 2, s);
+    if (stage != 1 && col4_supported(P)) return launch_col4(P, b, stage == 2, s);
     if (stage == 0) {
 #define M2_FWD(CC) if (P.C == CC) k_cols_fwd<CC><<<P.G, LTC, sc, s>>>(P, b);
         M2_FOR_C(M2_FWD)
 #undef M2_FWD
     } else if (stage == 1) {
+        if (pair_supported(P)) return launch_pair(P, b, s);
         if (rows_q_supported(P)) return launch_rows_q(P, b, s);
         k_rows<<<P.R / 2, LT, sr, s>>>(P, b);
     } else {

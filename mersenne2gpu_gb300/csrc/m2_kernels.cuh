@@ -38,6 +38,7 @@ struct LargePlan {
     int span;
     unsigned int p;
     int mode;
+    unsigned int in_turn;      // 1: R = 256 runs the passes of m2_pass.cu at every row length, not the fused column kernel
     unsigned int mid_tickets;  // fused column kernel: 0 = cooperative (CTA index = group), 1 = groups by arrival ticket
     unsigned int gf61;         // 1: the GF(P61^2)-only layout; each word is the signed GF(P61) residue (no CRT)
     unsigned int mid_barrier;  // cooperative fused column kernel: 1 = all groups publish before any goes on

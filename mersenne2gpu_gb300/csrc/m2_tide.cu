@@ -45,6 +45,8 @@ template <int LB_, int UNITS_, u32 PAIRS_, bool ROWS8_> struct Shape {
     static constexpr u32 NT = 1024, NF = NT / PAIRS;         // threads of the CTA, of a row pair
     static constexpr u32 SLOTS = 2 * B * PAIRS, SMEM = 24 * SLOTS;   // the row pairs, or a column group
     static constexpr u32 SLOT_R = R * C;
+    static constexpr bool EARLY = false;
+    static constexpr u32 ROW_TAG = 1;
     static constexpr bool NARROW = PAIRS == 2;               // 15 barriers: 7 per row pair, or one
     static constexpr u32 BARS = NARROW ? 7 : 1;
     static_assert(SLOT_R <= SLOTS, "a column group fits");
