@@ -1375,6 +1375,7 @@ struct SrvBucket {
     std::vector<uint64_t> members;       // keys of the tests in the launch in flight
     std::vector<uint32_t> ks;
     bool busy = false;
+    bool whole = false;                  // its CTAs hold whole SMs (srv_launch)
 };
 
 // device memory a test will hold (digits, weights, status, descriptor; the
@@ -1396,6 +1397,8 @@ struct m2_server {
     int device = 0;
     uint64_t budget = 0;
     uint32_t quantum = 1000;
+    int sms = 1;
+    size_t smem_sm = 0;                   // shared memory of an SM
     std::deque<SrvItem> queue;
     std::map<uint64_t, SrvItem> active;   // key: admission order
     uint64_t next_key = 0;
@@ -1437,7 +1440,9 @@ void srv_retire(m2_server* s, SrvItem& it, int status) {
 
 int srv_bucket_reserve(SrvBucket& b, size_t need) {
     cudaError_t e;
-    if (!b.stream && (e = cudaStreamCreateWithFlags(&b.stream, cudaStreamNonBlocking)) != cudaSuccess)
+    int lo = 0, hi = 0;   // before the larger lanes' CTAs (srv_launch)
+    cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    if (!b.stream && (e = cudaStreamCreateWithPriority(&b.stream, cudaStreamNonBlocking, hi)) != cudaSuccess)
         return fail_cuda("server stream", e);
     if (!b.ev && (e = cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming)) != cudaSuccess)
         return fail_cuda("server event", e);
@@ -1459,8 +1464,12 @@ int srv_bucket_reserve(SrvBucket& b, size_t need) {
 // starts a quantum on every idle lane
 int srv_launch(m2_server* s) {
     std::map<u64, std::vector<uint64_t>> small;
+    size_t total = 0;
+    bool waits = false;   // a lane's column CTAs wait for each other
     for (auto& kv : s->active) {
         SrvItem& it = kv.second;
+        if (it.ctx->path == M2_PATH_SMALL) ++total;
+        else if (it.ctx->fused) waits = true;
         if (it.inflight) continue;
         if (it.ctx->path == M2_PATH_SMALL) {
             auto b = s->buckets.find(it.ctx->L.h);
@@ -1468,6 +1477,11 @@ int srv_launch(m2_server* s) {
             continue;
         }
         const uint32_t k = std::min(s->quantum, it.total - it.done);
+        // CTAs that wait for each other need room for all of them
+        if (it.ctx->fused)
+            for (auto& b : s->buckets)
+                if (b.second.busy && b.second.whole && cudaStreamWaitEvent(it.ctx->stream, b.second.ev, 0) != cudaSuccess)
+                    return fail_cuda("server lane order", cudaGetLastError());
         int rc = m2_iterate(it.ctx, k);
         if (rc) return rc;
         cudaError_t e = cudaEventRecord(it.ev, it.ctx->stream);
@@ -1475,6 +1489,15 @@ int srv_launch(m2_server* s) {
         it.inflight = k;
         s->launches += (uint32_t)m2_launches_for(it.ctx, k);
     }
+    // A one-CTA test is one serial chain: among the larger lanes' warps it gets a
+    // warp's share of an SM and a request of a second takes two.  While the
+    // one-CTA tests would fill at most half the SMs, each asks for the shared
+    // memory of a whole one, so that nothing else joins it there; more of them
+    // share in proportion (20 s of a mix: tests of n = 2^8 ... 2^12 12-45k ->
+    // 19-67k squarings/s each, p99 9.5 -> 5.9 s, all tests 227k -> 232k).
+    // Not beside column CTAs that wait for each other (n = 2^21 and up).
+    const size_t per_sm = (2 * total + (size_t)s->sms - 1) / (size_t)s->sms;
+    const size_t min_smem = per_sm && !waits ? s->smem_sm / per_sm : 0;
     for (auto& kv : small) {
         SrvBucket& b = s->buckets[kv.first];
         const size_t cnt = kv.second.size();
@@ -1510,8 +1533,8 @@ int srv_launch(m2_server* s) {
         if (e == cudaSuccess) e = cudaMemsetAsync(b.d_status, 0, cnt * sizeof(int), b.stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b.d_tests, b.h_tests, cnt * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, b.stream);
         if (e != cudaSuccess) return fail_cuda("server descriptor upload", e);
-        e = duo ? m2k::launch_duo(b.d_tests, (int)cnt, (unsigned)kv.first, 0u, b.stream)
-                : m2k::launch_small(b.d_tests, (int)cnt, (unsigned)kv.first, threads, 0u, b.stream, fuse);
+        e = duo ? m2k::launch_duo(b.d_tests, (int)cnt, (unsigned)kv.first, 0u, b.stream, nullptr, 0, min_smem)
+                : m2k::launch_small(b.d_tests, (int)cnt, (unsigned)kv.first, threads, 0u, b.stream, fuse, false, min_smem);
         if (e != cudaSuccess)
             return fail_cuda("server small-test launch", e);
         e = cudaMemcpyAsync(b.h_status, b.d_status, cnt * sizeof(int), cudaMemcpyDeviceToHost, b.stream);
@@ -1519,6 +1542,7 @@ int srv_launch(m2_server* s) {
         if (e != cudaSuccess) return fail_cuda("server status readback", e);
         for (size_t j = 0; j < cnt; ++j) s->active[kv.second[j]].inflight = b.ks[j];
         b.busy = true;
+        b.whole = min_smem != 0;
         s->launches++;
     }
     return M2_OK;
@@ -1578,6 +1602,10 @@ int m2_srv_create(m2_server** out, int device, uint64_t budget_bytes, uint32_t q
     s->device = device;
     s->budget = budget_bytes;
     s->quantum = quantum ? quantum : 1000;
+    int smem = 0;
+    if (cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || s->sms < 1) s->sms = 1;
+    if (cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) == cudaSuccess) s->smem_sm = (size_t)smem;
+    cudaGetLastError();
     if (cudaStreamCreateWithFlags(&s->small_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->small_ready, cudaEventDisableTiming) != cudaSuccess) {
         m2_srv_destroy(s);
@@ -1618,7 +1646,7 @@ int m2_srv_step(m2_server* s) {
         // lanes share the GPU: the passes with the fields in turn, whose CTAs
         // wait for nothing (us a squaring, 8 tests of n = 2^19 25.9 -> 23.6, 4 of
         // 2^20 58.4 -> 52.4, one test alone 44.2 -> 36.6 and 79 -> 66.6)
-        if (rc == M2_OK && it.ctx->path == M2_PATH_LARGE && it.ctx->plan.R == 256u && it.ctx->plan.C == 4u && it.ctx->fused) {
+        if (rc == M2_OK && it.ctx->path == M2_PATH_LARGE && it.ctx->plan.R == 256u && it.ctx->fused) {
             it.ctx->plan.in_turn = 1u;
             it.ctx->fused = false;
         }

@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(ColShape<CR>::CNT, 65536 / (64 * ColShape<CR>:
 }
 
 // R = 256 only with rows of 1024 or more, and not where passes with the fields
-// in turn are asked for (m2_pass.cu, faster at every R = 256)
+// in turn are asked for (m2_pass.cu; with R = 1024 those gain 3% at n = 2^21
+// and lose 4% at 2^22 with several tests on the GPU, and lose 6% with one)
 bool cols_q_supported(const LargePlan& P) {
     return (P.R == 1024u || (P.R == 256u && P.B >= 1024u && !P.in_turn)) && P.C == (u32)CC && P.span < 2 * CC;
 }

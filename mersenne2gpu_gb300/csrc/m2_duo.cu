@@ -19,6 +19,8 @@
 //     -> 6.2  13.0  27.7  53.7  111   229   494
 // and us per squaring of a lone test: 5.9 -> 6.6, 6.4 -> 6.8 (n = 256, 512),
 // 12.3 -> 10.2, 24.6 -> 21.2, 51.7 -> 36.6, 104 -> 75 (n = 2048 ... 16384).
+#include <algorithm>
+
 #include "m2_flow.cuh"
 
 namespace M2K_NS {
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(S::NT, S::PER) k_duo(const SmallTest* tests, i
 // tests of n = 512 with 106 of n = 256: 6.95 ms for 2.2 here).
 template <class S> cudaError_t prepare() {
     const cudaError_t e = cudaFuncSetAttribute(k_duo<S>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_duo<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_duo<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_smem_limit((const void*)k_duo<S>));
 }
 template <class S> int resident() {
     int nb = 0;
@@ -323,10 +325,11 @@ template <class S> int resident() {
     }
     return nb;
 }
-template <class S> cudaError_t launch(const SmallTest* d_tests, int ntests, u32 iters_override, int* d_queue, int grid, cudaStream_t s) {
+template <class S> cudaError_t launch(const SmallTest* d_tests, int ntests, u32 iters_override, int* d_queue, int grid, cudaStream_t s, size_t min_smem) {
     const cudaError_t e = prepare<S>();
     if (e != cudaSuccess) return e;
-    k_duo<S><<<grid, S::NT, S::SMEM, s>>>(d_tests, ntests, iters_override, d_queue);
+    const size_t sm = std::max<size_t>(S::SMEM, std::min<size_t>(min_smem, (size_t)std::max<int>(dyn_smem_limit((const void*)k_duo<S>), 0)));
+    k_duo<S><<<grid, S::NT, sm, s>>>(d_tests, ntests, iters_override, d_queue);
     return cudaGetLastError();
 }
 
@@ -350,8 +353,9 @@ int duo_ctas_per_sm(unsigned h) {
 #undef M2_DUO_R
     return 0;
 }
-cudaError_t launch_duo(const SmallTest* d_tests, int ntests, unsigned h, unsigned iters_override, cudaStream_t s, int* d_queue, int grid) {
-#define M2_DUO_L(A) if (h == 1u << A) return launch<Shape<A>>(d_tests, ntests, iters_override, d_queue, d_queue ? grid : ntests, s);
+cudaError_t launch_duo(const SmallTest* d_tests, int ntests, unsigned h, unsigned iters_override, cudaStream_t s, int* d_queue, int grid,
+                       size_t min_smem) {
+#define M2_DUO_L(A) if (h == 1u << A) return launch<Shape<A>>(d_tests, ntests, iters_override, d_queue, d_queue ? grid : ntests, s, min_smem);
     M2_DUO_SIZES(M2_DUO_L)
 #undef M2_DUO_L
     return cudaErrorInvalidValue;

@@ -23,6 +23,8 @@
 //      k_cols_inv: last inverse levels on the columns, unweight, CRT, carry
 //                  within each row segment of C elements; the segment's carry
 //                  out is applied by the next k_cols_fwd.
+#include <algorithm>
+
 #include "m2_kernels.cuh"
 #include "m2_field.cuh"
 
@@ -391,11 +393,11 @@ const void* small_fn(bool fuse) { return fuse ? (const void*)k_small<true> : (co
 }  // namespace
 
 cudaError_t launch_small(const SmallTest* d_tests, int ntests, unsigned int h, int threads, unsigned int iters_override,
-                         cudaStream_t s, bool fuse, bool gf61) {
+                         cudaStream_t s, bool fuse, bool gf61, size_t min_smem) {
 #if M2_DUAL
-    if (gf61) return m2k_g61::launch_small(d_tests, ntests, h, threads, iters_override, s, fuse, true);
+    if (gf61) return m2k_g61::launch_small(d_tests, ntests, h, threads, iters_override, s, fuse, true, min_smem);
 #endif
-    const size_t sm = small_smem_bytes(h, threads);
+    const size_t sm = std::max(small_smem_bytes(h, threads), std::min(min_smem, (size_t)std::max(dyn_smem_limit(small_fn(fuse)), 0)));
     cudaError_t e = cudaFuncSetAttribute(small_fn(fuse), cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_smem_limit(small_fn(fuse)));
     if (e != cudaSuccess) return e;
     if (fuse) k_small<true><<<ntests, threads, sm, s>>>(d_tests, ntests, h, iters_override, nullptr);

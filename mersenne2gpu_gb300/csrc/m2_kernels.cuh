@@ -121,9 +121,9 @@ cudaError_t launch_results(const SmallTest* d_tests, int ntests, int ln, unsigne
 bool duo_supported(unsigned int h, int span, int carry_threads);
 int duo_threads(unsigned int h);
 int duo_ctas_per_sm(unsigned int h);
-// one CTA per test, or (d_queue) a persistent grid; iters_override as launch_small
+// one CTA per test, or (d_queue) a persistent grid; iters_override and min_smem as launch_small
 cudaError_t launch_duo(const SmallTest* d_tests, int ntests, unsigned int h, unsigned int iters_override, cudaStream_t s,
-                       int* d_queue = nullptr, int grid = 0);
+                       int* d_queue = nullptr, int grid = 0, size_t min_smem = 0);
 
 // Throughput of 32x32->64-bit integer multiplies (mul.wide.u32 / mad.wide.u32)
 // on every SM: independent chains, returns products per second.

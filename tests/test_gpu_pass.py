@@ -29,6 +29,32 @@ def test_server_matches_alone(m2, mode):
             assert got[p].status == 0 and got[p].res64 == e.res64(), (p, mode)
 
 
+def test_server_small_tests_beside_waiting_lanes(m2):
+    """One-CTA tests that hold whole SMs, more of them than that allows, and
+    larger tests whose column CTAs wait for each other."""
+    from mersenne2gpu_gb300.serve import Server
+    small = [20993, 40961, 81929, 159745, 319487] * 9
+    for large in ([], [57885161, 115640321], [57885161] * 2 + small * 3):
+        jobs = small + large
+        got = {}
+        with Server(budget_bytes=8 << 30, quantum=23) as srv:
+            for i, p in enumerate(jobs):
+                srv.submit(i, p, 1, 60)
+            for _ in range(100000):
+                srv.step()
+                for r in srv.poll():
+                    got[r.id] = r
+                if len(got) == len(jobs):
+                    break
+        want = {}
+        for i, p in enumerate(jobs):
+            if p not in want:
+                with m2.Engine(p, 1) as e:
+                    e.iterate(60)
+                    want[p] = e.res64()
+            assert got[i].status == 0 and got[i].res64 == want[p], p
+
+
 @pytest.mark.parametrize("fields", [0, 1])
 @pytest.mark.parametrize("p", [159745, 319487, 622589, 1245183, 2424831, 4849663, 9437183])
 def test_path_large_matches_auto(m2, p, fields):
