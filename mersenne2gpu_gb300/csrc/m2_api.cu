@@ -320,7 +320,7 @@ int read_head(m2_ctx* c, std::vector<u64>& head, unsigned& flags) {
     int rc = device_canonical(c, a);
     if (rc) return rc;
     head.assign(std::min<u64>(c->L.n, HEAD), 0);
-    cudaError_t e = cudaMemcpyAsync(head.data(), c->d_canon, head.size() * sizeof(u64), cudaMemcpyDeviceToHost, c->stream);
+    cudaError_t e = m2i::read_back(head.data(), c->d_canon, head.size() * sizeof(u64), c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, a.flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
     if (e != cudaSuccess) return fail_cuda("digits read", e);
     return m2_sync(c);
@@ -745,7 +745,7 @@ int m2_get_digits(m2_ctx* c, uint64_t* out) {
     m2k::NormArgs a;
     int rc = device_canonical(c, a);
     if (rc) return rc;
-    const cudaError_t e = cudaMemcpyAsync(out, c->d_canon, c->L.n * sizeof(u64), cudaMemcpyDeviceToHost, c->stream);
+    const cudaError_t e = m2i::read_back(out, c->d_canon, c->L.n * sizeof(u64), c->stream);
     if (e != cudaSuccess) return fail_cuda("digits read", e);
     return m2_sync(c);
 }
@@ -841,7 +841,7 @@ int m2_carry_normalize(uint32_t p, const int64_t* digits, const int64_t* seg_car
     int st = 0;
     e = cudaMemsetAsync(a.status, 0, sizeof(int), s);
     if (e == cudaSuccess) e = m2k::launch_normalize(a, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&st, a.status, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = m2i::read_back(&st, a.status, sizeof(int), s);
     if (e == cudaSuccess) e = cudaFreeAsync(scratch, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail_cuda("carry propagation", e);
@@ -861,7 +861,7 @@ int m2_test_stall_fused(m2_ctx* c) {
         return e == cudaSuccess ? M2_OK : fail_cuda("m2_test_stall_fused", e);
     }
     unsigned f0 = 0;
-    cudaError_t e = cudaMemcpyAsync(&f0, c->d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
+    cudaError_t e = m2i::read_back(&f0, c->d_flags, sizeof(unsigned), c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     f0 += 1u << 20;
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_flags, &f0, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream);
@@ -876,8 +876,8 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
     c->staged = c->flow || c->cluster;
     cudaError_t e = in_turn(c, [&] { return m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream); });
     const size_t h = c->L.h;
-    if (e == cudaSuccess && za_out) e = cudaMemcpyAsync(za_out, c->d_za, 16 * h, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && zb_out) e = cudaMemcpyAsync(zb_out, c->d_zb, 8 * h, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && za_out) e = m2i::read_back(za_out, c->d_za, 16 * h, c->stream);
+    if (e == cudaSuccess && zb_out) e = m2i::read_back(zb_out, c->d_zb, 8 * h, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return fail_cuda("m2_test_stage", e);
     if (stage == 2) c->iteration += 1;
@@ -1316,7 +1316,7 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         if (e == cudaSuccess) e = m2k::launch_results(d_all + l.first, l.ntests, l.ln, d_res + l.first, d_prime + l.first, s0);
     std::vector<u64> res(count);
     std::vector<int> prime(count), q(2 * nb);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(res.data(), d_res, count * sizeof(u64), cudaMemcpyDeviceToHost, s0);
+    if (e == cudaSuccess) e = m2i::read_back(res.data(), d_res, count * sizeof(u64), s0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(prime.data(), d_prime, count * sizeof(int), cudaMemcpyDeviceToHost, s0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(q.data(), d_q, 2 * nb * sizeof(int), cudaMemcpyDeviceToHost, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);

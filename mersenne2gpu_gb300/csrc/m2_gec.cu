@@ -158,7 +158,7 @@ int count_diff(m2_gec* g, const ull* a, const ull* b, unsigned* out) {
     if (rc) return rc;
     k_gec_diff<<<grid_for(g->L->n), 256, 0, g->as>>>(a, b, g->L->n, g->count);
     if ((rc = cuda_rc(cudaGetLastError()))) return rc;
-    if ((rc = cuda_rc(cudaMemcpyAsync(out, g->count, sizeof(unsigned), cudaMemcpyDeviceToHost, g->as)))) return rc;
+    if ((rc = cuda_rc(m2i::read_back(out, g->count, sizeof(unsigned), g->as)))) return rc;
     return cuda_rc(cudaStreamSynchronize(g->as));
 }
 

@@ -11,6 +11,19 @@ namespace m2k { struct LargePlan; }
 
 namespace m2i {
 
+// Device-to-host copy behind the stream's work, with that work waited for first
+// where the destination is pageable: the driver then waits for it inside the
+// copy, under a lock that every other thread's allocation, event creation and
+// stream creation needs (a thread beside a batch of 3 s had its first call back
+// after 2.6 s, with the wait here 0.2 ms).
+inline cudaError_t read_back(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    cudaPointerAttributes at{};
+    cudaError_t e = cudaPointerGetAttributes(&at, dst);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e != cudaSuccess || at.type == cudaMemoryTypeUnregistered) e = cudaStreamSynchronize(s);
+    return e == cudaSuccess ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s) : e;
+}
+
 // plan of the three-pass path for exponent layout L (false: no plan fits);
 // carry_pairs is the -B hint (columns per CTA), 0 for the default
 bool plan_large(const m2::Layout& L, int span, uint32_t carry_pairs, m2k::LargePlan& P);

@@ -176,7 +176,7 @@ extern "C" int m2_square_noalloc(uint32_t p, int mode, int64_t* digits, uint32_t
     if (cudaGetLastError() != cudaSuccess) return M2_ECUDA;
 
     int host_status = 0;
-    if (cudaMemcpyAsync(&host_status, status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return M2_ECUDA;
+    if (m2i::read_back(&host_status, status, sizeof(int), st) != cudaSuccess) return M2_ECUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return M2_ECUDA;
     return host_status ? M2_ESTATE : M2_OK;
 }
