@@ -100,7 +100,18 @@ typedef struct {
 int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts);
 
 /* Replaces k rounds of enqueue_plan(iter_plan); enqueue_plan(post_plan);
- * (mersenne2_gpu.cpp:4812-4822).  Asynchronous on the context's stream. */
+ * (mersenne2_gpu.cpp:4812-4822).  Asynchronous on the context's stream.
+ * From n = 2^14 on a context alone on the device runs kernels that need 64 to
+ * 152 SMs at once.  Beside other contexts, servers and batches of this process
+ * that have work in flight on the device it takes the three-pass kernels where
+ * either would keep the other from getting on, and launches it has queued give
+ * way to such work within the one that runs; their squarings then run in the
+ * next m2_sync, m2_get_digits, m2_res64, m2_verdict or m2_test_stage
+ * call, which waits for them.  Kernels that this library does not know of (the
+ * caller's own, m2_square_noalloc, replays of graphs that the caller captured)
+ * may delay such a launch until there is room for all of it.  Replays of graphs
+ * captured from contexts whose info says fused_cols are the caller's to order
+ * behind other contexts' work. */
 int m2_iterate(m2_ctx* ctx, uint32_t k);
 
 /* Replaces clFinish at a report point (mersenne2_gpu.cpp:4788); also reports

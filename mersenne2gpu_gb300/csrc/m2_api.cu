@@ -1,6 +1,7 @@
 // m2_api.cu -- the C ABI of include/m2gpu.h on top of the kernels.
 #include "../../include/m2gpu.h"
 #include "m2_host.hpp"
+#include "m2_board.hpp"
 #include "m2_internal.hpp"
 #include "m2_kernels.cuh"
 
@@ -10,7 +11,6 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
-#include <set>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -141,7 +141,9 @@ struct m2_ctx {
     unsigned char* d_w61 = nullptr;
     unsigned char* d_w31 = nullptr;
     TwTables tw;
-    int* d_status = nullptr;
+    m2k::StateWords* d_words = nullptr;
+    unsigned* yield = nullptr; // host word that calls its queued one-launch kernels off
+    int* d_status = nullptr;   // d_words->status
     long long* d_digits = nullptr;
     // small path
     m2k::SmallTest* d_test = nullptr;
@@ -170,11 +172,14 @@ struct m2_ctx {
     uint2* d_taux = nullptr;   // the large sizes' row-stage tables and parked digits
     uint32_t* d_tshift = nullptr;
     longlong2* d_park = nullptr;
-    // GRAPH_ITERS[i] iterations of the three-pass path captured once and replayed
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    // contexts whose kernels wait for each other: the plan of passes that do not
+    m2k::LargePlan free_plan{};
+    // GRAPH_ITERS[i] iterations of the three-pass path captured once and replayed, by plan and by free_plan
+    cudaGraphExec_t graph[2][2] = {};
     bool graph_failed = false;
     void* d_slab = nullptr;    // the allocation that holds the buffers above
-    cudaEvent_t gate_ev = nullptr;   // three-pass contexts with waiting kernels: end of the last enqueued run (Gate)
+    std::shared_ptr<m2b::Run> run;   // its work in flight, as other contexts see it
+    bool may_owe = false;      // a launch that may be called off was enqueued since the last settle
     // canonical digits and carry-propagation scratch (allocated on first read, in d_read)
     void* d_read = nullptr;
     unsigned long long* d_canon = nullptr;
@@ -227,12 +232,18 @@ size_t flags_bytes(const m2k::LargePlan& P) { return sizeof(unsigned) * ((size_t
 // less on those two passes per squaring.
 constexpr uint32_t GRAPH_ITERS[2] = {500, 50};
 
+// k squarings by the three-pass kernels; free: by those of them that wait for nothing
+cudaError_t launch_passes(m2_ctx* c, uint32_t k, bool free) {
+    return m2k::launch_large_run(free ? c->free_plan : c->plan, c->bufs, k, c->fused && !free, c->stream);
+}
+
 // Captures GRAPH_ITERS[i] iterations on the context's stream into an executable
 // graph (once); replays cost one launch instead of 2 or 3 per iteration.  Not done
 // while the caller is capturing the stream itself, or if capture is refused
 // (the legacy default stream): launches are then issued one by one.
-bool ensure_graph(m2_ctx* c, int i) {
-    if (c->graph[i]) return true;
+bool ensure_graph(m2_ctx* c, int i, bool free) {
+    cudaGraphExec_t& exec = c->graph[free][i];
+    if (exec) return true;
     if (c->graph_failed) return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
@@ -246,24 +257,25 @@ bool ensure_graph(m2_ctx* c, int i) {
         return false;
     }
     cudaError_t e = cudaSuccess;
-    e = m2k::launch_large_run(c->plan, c->bufs, GRAPH_ITERS[i], c->fused, c->stream);
+    e = launch_passes(c, GRAPH_ITERS[i], free);
     const cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
-    if (e == cudaSuccess && ee == cudaSuccess && g && cudaGraphInstantiate(&c->graph[i], g, 0) == cudaSuccess) {
+    if (e == cudaSuccess && ee == cudaSuccess && g && cudaGraphInstantiate(&exec, g, 0) == cudaSuccess) {
         cudaGraphDestroy(g);
         return true;
     }
     if (g) cudaGraphDestroy(g);
     cudaGetLastError();
-    c->graph[i] = nullptr;
+    exec = nullptr;
     c->graph_failed = true;
     return false;
 }
 
 // Squarings per launch of the one-launch kernel: long enough that a launch's
-// start is nothing (62 ms at n = 2^20), short enough that other contexts'
-// launches get their turn.
+// start is nothing (58 ms at n = 2^20), short enough that other contexts'
+// launches get their turn; and by passes between two looks at what is in flight.
 constexpr uint32_t FLOW_ITERS = 1000;
 constexpr uint32_t TIDE_ITERS = 250;
+constexpr uint32_t FREE_ITERS = 1000;
 
 m2k::TideArgs tide_args(const m2_ctx* c) { return m2k::TideArgs{c->fargs, c->d_taux, c->d_tshift, c->d_park, c->tw.tw8}; }
 
@@ -277,7 +289,7 @@ cudaError_t flow_reset(m2_ctx* c) {
 }
 
 // what a new state needs beside its digits: no pending carries, epoch flags
-// and tags as at creation
+// and tags as at creation (a good status and nothing owed are clear_words')
 cudaError_t reset_sync_words(m2_ctx* c) {
     cudaError_t e = cudaSuccess;
     if (c->path == M2_PATH_LARGE) e = cudaMemsetAsync(c->d_carries, 0, sizeof(i64) * (size_t)c->plan.R * c->plan.G, c->stream);
@@ -286,6 +298,38 @@ cudaError_t reset_sync_words(m2_ctx* c) {
     if (e == cudaSuccess) c->staged = false;
     return e;
 }
+
+cudaError_t clear_words(m2_ctx* c) { return cudaMemsetAsync(c->d_words, 0, offsetof(m2k::StateWords, yield), c->stream); }
+
+// Words of pinned host memory that call queued launches off, one per one-launch
+// context: 64 bytes apart, in pages kept for the process (a launch of a context
+// that is gone may still look at its word).
+std::mutex g_yield_mu;
+std::vector<unsigned*> g_yield;
+unsigned* yield_word() {
+    std::lock_guard<std::mutex> lk(g_yield_mu);
+    if (g_yield.empty()) {
+        unsigned* page = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // another thread may be capturing
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaHostAlloc((void**)&page, 4096, cudaHostAllocPortable | cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        for (int i = 0; i < 64; ++i) g_yield.push_back(page + 16 * i);
+    }
+    unsigned* w = g_yield.back();
+    g_yield.pop_back();
+    *w = 0;
+    return w;
+}
+
+// waits for the context's stream and reads its words
+int read_words(m2_ctx* c, m2k::StateWords& w) {
+    cudaError_t e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = cudaMemcpy(&w, c->d_words, sizeof(w), cudaMemcpyDeviceToHost);
+    return e == cudaSuccess ? M2_OK : M2_ECUDA;
+}
+int status_code(int st) { return (st & m2k::ST_WAIT_TIMEOUT) ? M2_ETIMEOUT : st ? M2_ESTATE : M2_OK; }
 
 int cuda_err(cudaError_t e) { return e == cudaSuccess ? M2_OK : (e == cudaErrorMemoryAllocation ? M2_ENOMEM : M2_ECUDA); }
 
@@ -312,18 +356,6 @@ int device_canonical(m2_ctx* c, m2k::NormArgs& a) {
     m2k::norm_bind_scratch(a, c->d_norm);
     const cudaError_t e = m2k::launch_normalize(a, c->stream);
     return e == cudaSuccess ? M2_OK : fail_cuda("carry propagation launch", e);
-}
-
-// the first digits (enough for 64 bits) and the summary flags of the canonical state
-int read_head(m2_ctx* c, std::vector<u64>& head, unsigned& flags) {
-    m2k::NormArgs a;
-    int rc = device_canonical(c, a);
-    if (rc) return rc;
-    head.assign(std::min<u64>(c->L.n, HEAD), 0);
-    cudaError_t e = m2i::read_back(head.data(), c->d_canon, head.size() * sizeof(u64), c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, a.flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
-    if (e != cudaSuccess) return fail_cuda("digits read", e);
-    return m2_sync(c);
 }
 
 }  // namespace
@@ -388,7 +420,7 @@ int load_canon(m2_ctx* c, uint32_t iteration) {
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     cudaError_t e = m2k::launch_balance(c->d_canon, c->d_digits, c->L.p, c->L.ln, c->L.n, nullptr, c->stream);
     if (e == cudaSuccess) e = reset_sync_words(c);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
+    if (e == cudaSuccess) e = clear_words(c);
     if (e != cudaSuccess) return fail_cuda("state load", e);
     c->iteration = iteration;
     return M2_OK;
@@ -405,8 +437,10 @@ const char* own_kernel_name(const m2_ctx* c) {
 }
 uint32_t iters_per_launch(const m2_ctx* c) { return c->tide ? TIDE_ITERS : c->flow ? FLOW_ITERS : ~0u; }
 
-cudaError_t launch_own(m2_ctx* c, uint32_t k) {
+// (ask: the launches look first whether they are called off)
+cudaError_t launch_own(m2_ctx* c, uint32_t k, bool ask) {
     cudaError_t e = cudaSuccess;
+    c->fargs.ask = ask;
     const unsigned h = (unsigned)c->L.h;
     const int lh = c->L.ln - 1;
     for (uint32_t left = k, now; left > 0 && e == cudaSuccess; left -= now) {
@@ -428,108 +462,145 @@ cudaError_t launch_own(m2_ctx* c, uint32_t k) {
     return e;
 }
 
-// After a three-pass stage: the one-launch kernel of mid sizes applies pending
+// After three-pass kernels: the one-launch kernel of mid sizes applies pending
 // carries itself and wants its tags back; the others start from digits with
 // none.
 int unstage(m2_ctx* c) {
     if (!c->staged) return M2_OK;
+    cudaError_t e = cudaSuccess;
     if (c->flow && !c->tide) {
-        const cudaError_t e = flow_reset(c);
-        if (e != cudaSuccess) return fail_cuda("tags", e);
+        e = flow_reset(c);
     } else {
         m2k::NormArgs a;
-        int rc = device_canonical(c, a);
-        if (!rc) rc = m2i::load_canon(c, c->iteration);
+        const int rc = device_canonical(c, a);
         if (rc) return rc;
+        e = m2k::launch_balance(c->d_canon, c->d_digits, c->L.p, c->L.ln, c->L.n, nullptr, c->stream);
+        if (e == cudaSuccess) e = reset_sync_words(c);
     }
+    if (e != cudaSuccess) return fail_cuda("state after three-pass kernels", e);
     c->staged = false;
     return M2_OK;
 }
 
-}  // namespace
-
-namespace {
-
-// ---------------- kernels that wait between their CTAs ----------------
-// The one-launch kernels (cooperative, one CTA to an SM) and the fused column
-// pass of the three-pass path (cooperative or by tickets) spin on one another's
-// words.  The hardware starts a cooperative grid's CTAs as SMs come free; while
-// another context's waiting kernels are squeezed onto the few SMs that are left
-// neither gets on, and waits run out.  So the two kinds take turns: a run of
-// either is enqueued behind the runs of the other kind (one-launch runs also
-// behind each other) that contexts of this process have enqueued on the device
-// before it, by events.  Nothing waits on the host, and a context alone pays
-// one event record a call.
-struct Gate {
-    std::mutex mu;
-    cudaEvent_t one_ev = nullptr;          // end of the last one-launch run
-    cudaStream_t one_stream = nullptr;     // its stream; GONE once that context is destroyed (the handle may come back)
-    std::set<m2_ctx*> passes;              // contexts with a recorded gate_ev
-    std::vector<cudaEvent_t> left;         // gate_ev of contexts destroyed with work in flight
-};
-const cudaStream_t GONE = reinterpret_cast<cudaStream_t>(~uintptr_t(0));
-std::mutex g_gate_mu;
-std::map<int, std::unique_ptr<Gate>> g_gate;
-Gate& gate_of(int device) {
-    std::lock_guard<std::mutex> lk(g_gate_mu);
-    std::unique_ptr<Gate>& g = g_gate[device];
-    if (!g) g.reset(new Gate());
-    return *g;
+// k squarings by the three-pass kernels; free: by those of them that wait for nothing
+int run_passes(m2_ctx* c, uint64_t k, bool free) {
+    bool ready[2];
+    for (int i = 0; i < 2; ++i)
+        ready[i] = k >= GRAPH_ITERS[i] && (i == 0 || k % GRAPH_ITERS[0] >= GRAPH_ITERS[1] || !ready[0]) && ensure_graph(c, i, free);
+    cudaError_t e = cudaSuccess;
+    if (c->flow) c->staged = true;
+    for (int i = 0; i < 2; ++i)
+        if (ready[i])
+            for (; k >= GRAPH_ITERS[i] && e == cudaSuccess; k -= GRAPH_ITERS[i]) e = cudaGraphLaunch(c->graph[free][i], c->stream);
+    if (k > 0 && e == cudaSuccess) e = launch_passes(c, (uint32_t)k, free);
+    return e == cudaSuccess ? M2_OK : fail_cuda("three-pass launch", e);
 }
 
-// Enqueues a run (`enqueue`) of context c in its turn.  A stream under capture
-// is left alone: its graph's runs are the caller's to order.
-template <class F> cudaError_t in_turn(m2_ctx* c, F&& enqueue) {
-    const bool one = c->flow && !c->staged, passes = !one && c->fused;
-    if (!one && !passes) return enqueue();
+m2b::Kind alone(const m2_ctx* c) { return c->flow ? m2b::ONE : c->fused ? m2b::FUSED : m2b::FREE; }
+
+// k squarings on the context's stream, by the kernels of its size (at most
+// `most`) or by those that what else is in flight on the device calls for
+// (m2_board.hpp).  A one-launch context is left as its own kernel leaves it:
+// graphs that its caller captured may run that next.
+int advance(m2_ctx* c, uint32_t k, m2b::Kind most) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        // recorded for the caller to replay: the kernels of a context alone
         cudaGetLastError();
-        return enqueue();
+        int rc = unstage(c);
+        if (rc) return rc;
+        const cudaError_t e = own_kernel(c) ? launch_own(c, k, false) : launch_passes(c, k, false);
+        return e == cudaSuccess ? M2_OK : fail_cuda("m2_iterate launch", e);
     }
-    Gate& g = gate_of(c->device);
-    std::lock_guard<std::mutex> lk(g.mu);
-    cudaError_t e = cudaSuccess;
-    if (g.one_stream && g.one_stream != c->stream) e = cudaStreamWaitEvent(c->stream, g.one_ev, 0);
-    if (one) {
-        for (m2_ctx* o : g.passes)
-            if (e == cudaSuccess && o != c) e = cudaStreamWaitEvent(c->stream, o->gate_ev, 0);
-        for (cudaEvent_t ev : g.left) {
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, ev, 0);
-            cudaEventDestroy(ev);
+    m2b::Board& board = m2b::Board::of(c->device);
+    m2b::Kind kind = board.begin(*c->run, most);
+    bool ask = c->tide;   // the queued launches of a long call; every one of those that take the whole GPU
+    int rc = M2_OK;
+    for (uint32_t left = k, now; left > 0 && !rc; left -= now) {
+        if (left != k) kind = board.again(*c->run, most);
+        if (c->flow && kind == m2b::FREE) {
+            now = std::min(left, FREE_ITERS);
+            rc = run_passes(c, now, true);
+        } else if (own_kernel(c)) {
+            now = std::min(left, iters_per_launch(c));
+            if ((rc = unstage(c))) break;
+            const cudaError_t e = launch_own(c, now, ask);
+            if (e != cudaSuccess) rc = fail_cuda("m2_iterate launch", e);
+            c->may_owe |= ask && c->flow;
+            ask = true;
+        } else {
+            now = left;
+            rc = run_passes(c, now, kind == m2b::FREE && c->fused);
         }
-        g.left.clear();
-        if (e == cudaSuccess && !g.one_ev) e = cudaEventCreateWithFlags(&g.one_ev, cudaEventDisableTiming);
-    } else if (e == cudaSuccess && !c->gate_ev) {
-        e = cudaEventCreateWithFlags(&c->gate_ev, cudaEventDisableTiming);
     }
-    if (e == cudaSuccess) e = enqueue();
-    const cudaError_t r = e == cudaSuccess ? cudaEventRecord(one ? g.one_ev : c->gate_ev, c->stream) : e;
-    if (r == cudaSuccess) {
-        if (one) g.one_stream = c->stream;
-        else g.passes.insert(c);
-    }
-    return r;
+    if (!rc && c->flow) rc = unstage(c);
+    const cudaError_t e = board.end(*c->run);
+    return rc ? rc : e == cudaSuccess ? M2_OK : fail_cuda("end of run", e);
 }
-// a context that goes away: its enqueued work stays in stream order
-void leave_gate(m2_ctx* c) {
-    if (!c->flow && !c->gate_ev) return;
-    Gate& g = gate_of(c->device);
-    std::lock_guard<std::mutex> lk(g.mu);
-    g.passes.erase(c);
-    if (g.one_stream == c->stream) g.one_stream = GONE;
-    if (c->gate_ev) g.left.push_back(c->gate_ev);
-    c->gate_ev = nullptr;
-    for (size_t i = 0; i < g.left.size();) {
-        if (cudaEventQuery(g.left[i]) == cudaErrorNotReady) { ++i; continue; }
-        cudaEventDestroy(g.left[i]);
-        g.left[i] = g.left.back();
-        g.left.pop_back();
+
+// Waits for the context's work, runs the squarings of launches that were called
+// off, and returns the state's code; *more (may be null): there were any.
+int settle(m2_ctx* c, bool* more = nullptr) {
+    if (more) *more = false;
+    for (uint64_t owed = 0;;) {
+        m2k::StateWords w{};
+        int rc = read_words(c, w);
+        if (rc) return rc;
+        if ((rc = status_code(w.status))) return rc;
+        owed += w.owed;
+        if (owed == 0) {
+            c->may_owe = false;
+            return M2_OK;
+        }
+        if (more) *more = true;
+        if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
+        const cudaError_t e = cudaMemsetAsync(&c->d_words->owed, 0, sizeof(w.owed), c->stream);
+        if (e != cudaSuccess) return fail_cuda("state words", e);
+        // in parts, each by what is in flight then; the part after a launch that
+        // was called off in kernels that always start
+        const uint32_t now = (uint32_t)std::min<uint64_t>(owed, w.owed ? FREE_ITERS : iters_per_launch(c));
+        if ((rc = advance(c, now, w.owed ? m2b::FREE : alone(c)))) return rc;
+        owed -= now;
     }
-    cudaGetLastError();
+}
+
+// Reads of the state: `enqueue` puts canonicalisation and copies on the
+// context's stream, again if squarings were still owed at their end.
+template <class F> int read_settled(m2_ctx* c, F&& enqueue) {
+    for (bool more = true; more;) {
+        int rc = enqueue();
+        if (!rc) rc = settle(c, &more);
+        if (rc) return rc;
+    }
+    return M2_OK;
+}
+
+// the first digits (enough for 64 bits) and the summary flags of the canonical state
+int read_head(m2_ctx* c, std::vector<u64>& head, unsigned& flags) {
+    return read_settled(c, [&] {
+        m2k::NormArgs a;
+        const int rc = device_canonical(c, a);
+        if (rc) return rc;
+        head.assign(std::min<u64>(c->L.n, HEAD), 0);
+        cudaError_t e = m2i::read_back(head.data(), c->d_canon, head.size() * sizeof(u64), c->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, a.flags, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
+        return e == cudaSuccess ? M2_OK : fail_cuda("digits read", e);
+    });
 }
 
 }  // namespace
+
+namespace m2i {
+int settle(m2_ctx* c) { return c->may_owe ? ::settle(c) : M2_OK; }
+int iterate_unowed(m2_ctx* c, uint32_t k) {
+    if (!c->tide) return m2_iterate(c, k);
+    if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
+    const int rc = run_passes(c, k, true);
+    if (!rc) c->iteration += k;
+    return rc;
+}
+void share_turns(m2_ctx* a, m2_ctx* b) { m2b::Board::of(a->device).group(*a->run, *b->run, a); }
+}  // namespace m2i
 
 extern "C" {
 
@@ -600,7 +671,7 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
     Slab mem;
     mem.add(&raw->d_w61, n);
     mem.add(&raw->d_w31, n);
-    mem.add(&raw->d_status, sizeof(int));
+    mem.add(&raw->d_words, sizeof(m2k::StateWords));
     mem.add(&raw->d_digits, n * sizeof(i64));
     const int lh = raw->L.ln - 1;
     size_t cw = 0;
@@ -633,7 +704,22 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
         }
     }
     if ((rc = mem.alloc(raw, &raw->d_slab))) { m2_destroy(c.release()); return rc; }
-    cudaError_t e = cudaMemsetAsync(raw->d_status, 0, sizeof(int), raw->stream);
+    raw->d_status = &raw->d_words->status;
+    m2k::StateWords words{};
+    if (raw->flow) words.yield = raw->yield = yield_word();
+    try {
+        raw->run = std::make_shared<m2b::Run>();
+        m2b::Board::of(raw->device).add(raw->run);
+    } catch (const std::bad_alloc&) {
+        m2_destroy(c.release());
+        return M2_ENOMEM;
+    }
+    raw->run->stream = raw->stream;
+    raw->run->large = path == M2_PATH_LARGE && !raw->cluster;
+    raw->run->whole = raw->tide;
+    raw->run->crowds = raw->L.ln <= 18;
+    raw->run->yield = raw->yield;
+    cudaError_t e = cudaMemcpyAsync(raw->d_words, &words, sizeof(words), cudaMemcpyHostToDevice, raw->stream);
     if (e != cudaSuccess) { m2_destroy(c.release()); return M2_ECUDA; }
     if (path == M2_PATH_SMALL) {
         raw->threads = m2k::small_threads_for((unsigned)h);
@@ -669,8 +755,14 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts) {
             raw->fargs = m2k::FlowArgs{raw->d_digits, raw->d_carries, raw->d_za, raw->d_zb, raw->d_w61, raw->d_w31, raw->d_aux,
                                        raw->tw.tw4, raw->tw.tc, reinterpret_cast<unsigned long long*>(raw->d_flow),
                                        reinterpret_cast<unsigned long long*>(raw->d_flow) + cw,
-                                       reinterpret_cast<unsigned*>(raw->d_flow + 8 * (cw + 1)), raw->d_status, 0u, 2u * P.C, raw->span, mode};
+                                       reinterpret_cast<unsigned*>(raw->d_flow + 8 * (cw + 1)), raw->d_status, 0u,
+                                       (unsigned short)(2u * P.C), (unsigned short)0, raw->span, mode};
         }
+        // without the fused column kernel; with the fields in turn where those serve the size (m2_pass.cu)
+        raw->free_plan = raw->plan;
+        raw->free_plan.mid_tickets = raw->free_plan.mid_barrier = 0u;
+        raw->free_plan.in_turn = P.R == 256u ? 1u : 0u;
+        if (((raw->flow || raw->fused) && m2k::pass_setup(raw->free_plan) != cudaSuccess) || (raw->tide && m2k::normalize_setup() != cudaSuccess)) { m2_destroy(c.release()); return M2_EUNSUPPORTED; }
         raw->bufs.ticket = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G);
         raw->bufs.phase = reinterpret_cast<unsigned long long*>(raw->d_flags + P.G + 2);
     }
@@ -708,51 +800,30 @@ int m2_iterate(m2_ctx* c, uint32_t k) {
     if (!c) return M2_EINVAL;
     if (k == 0) return M2_OK;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
-    int rc = unstage(c);
-    if (rc) return rc;
-    cudaError_t e = cudaSuccess;
-    if (own_kernel(c)) {
-        e = in_turn(c, [&] { return launch_own(c, k); });
-    } else {
-        bool ready[2];   // captured before the turn
-        for (int i = 0; i < 2; ++i) ready[i] = k >= GRAPH_ITERS[i] && (i == 0 || k % GRAPH_ITERS[0] >= GRAPH_ITERS[1] || !ready[0]) && ensure_graph(c, i);
-        e = in_turn(c, [&] {
-            cudaError_t r = cudaSuccess;
-            uint32_t left = k;
-            for (int i = 0; i < 2; ++i)
-                if (ready[i])
-                    for (; left >= GRAPH_ITERS[i] && r == cudaSuccess; left -= GRAPH_ITERS[i]) r = cudaGraphLaunch(c->graph[i], c->stream);
-            if (left > 0 && r == cudaSuccess) r = m2k::launch_large_run(c->plan, c->bufs, left, c->fused, c->stream);
-            return r;
-        });
-    }
-    if (e != cudaSuccess) return fail_cuda("m2_iterate launch", e);
-    c->iteration += k;
-    return M2_OK;
+    const int rc = advance(c, k, alone(c));
+    if (!rc) c->iteration += k;
+    return rc;
 }
 
 int m2_sync(m2_ctx* c) {
     if (!c) return M2_EINVAL;
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return M2_ECUDA;
-    int st = 0;
-    if (cudaMemcpy(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return M2_ECUDA;
-    if (st & m2k::ST_WAIT_TIMEOUT) return M2_ETIMEOUT;
-    return st ? M2_ESTATE : M2_OK;
+    return settle(c);
 }
 
 int m2_get_digits(m2_ctx* c, uint64_t* out) {
     if (!c || !out) return M2_EINVAL;
-    m2k::NormArgs a;
-    int rc = device_canonical(c, a);
-    if (rc) return rc;
-    const cudaError_t e = m2i::read_back(out, c->d_canon, c->L.n * sizeof(u64), c->stream);
-    if (e != cudaSuccess) return fail_cuda("digits read", e);
-    return m2_sync(c);
+    return read_settled(c, [&] {
+        m2k::NormArgs a;
+        const int rc = device_canonical(c, a);
+        if (rc) return rc;
+        const cudaError_t e = m2i::read_back(out, c->d_canon, c->L.n * sizeof(u64), c->stream);
+        return e == cudaSuccess ? M2_OK : fail_cuda("digits read", e);
+    });
 }
 
 int m2_set_digits(m2_ctx* c, const uint64_t* digits, uint32_t iteration) {
     if (!c || !digits) return M2_EINVAL;
-    if (m2_sync(c) == M2_ECUDA) return M2_ECUDA;
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return M2_ECUDA;   // (the old state's owed squarings go with it)
     // canonical input (every digit below 2^width), the usual case: uploaded and
     // balanced on the device, which also checks that it is canonical; anything
     // else is reduced on the host first
@@ -765,7 +836,7 @@ int m2_set_digits(m2_ctx* c, const uint64_t* digits, uint32_t iteration) {
     if (e == cudaSuccess) e = m2k::launch_balance(c->d_canon, c->d_digits, c->L.p, c->L.ln, c->L.n, d_bad, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, d_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = reset_sync_words(c);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
+    if (e == cudaSuccess) e = clear_words(c);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return fail_cuda("state upload", e);
     if (bad) {
@@ -873,8 +944,9 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
     if (!c || stage < 0 || stage > 2) return M2_EINVAL;
     if (c->path != M2_PATH_LARGE) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
+    if (const int rc = c->flow ? settle(c) : M2_OK) return rc;
     c->staged = c->flow || c->cluster;
-    cudaError_t e = in_turn(c, [&] { return m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream); });
+    cudaError_t e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
     const size_t h = c->L.h;
     if (e == cudaSuccess && za_out) e = m2i::read_back(za_out, c->d_za, 16 * h, c->stream);
     if (e == cudaSuccess && zb_out) e = m2i::read_back(zb_out, c->d_zb, 8 * h, c->stream);
@@ -903,13 +975,18 @@ int m2_info(m2_ctx* c, m2_info_t* info) {
 void m2_destroy(m2_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
-    leave_gate(c);
+    if (c->run) m2b::Board::of(c->device).remove(c->run);
+    if (c->yield) {
+        std::lock_guard<std::mutex> lk(g_yield_mu);
+        g_yield.push_back(c->yield);
+    }
     // stream-ordered frees: they follow the context's queued work and do not
     // wait for other streams; its stream is released once that work is done
     if (c->stream)
         for (void* b : {c->d_slab, c->d_read}) if (b) cudaFreeAsync(b, c->stream);
-    for (cudaGraphExec_t g : c->graph)
-        if (g) cudaGraphExecDestroy(g);
+    for (auto& set : c->graph)
+        for (cudaGraphExec_t g : set)
+            if (g) cudaGraphExecDestroy(g);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -920,8 +997,11 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
     // the launch sequence m2_iterate issues for `iters` squarings, one event after each
     std::vector<int> seq;
     if (const int rc = unstage(c)) return rc;
-    if (own_kernel(c)) seq.push_back(-1);
-    else if (c->fused) {
+    m2b::Board& board = m2b::Board::of(c->device);
+    const m2b::Kind kind = board.begin(*c->run, alone(c));
+    const bool free = kind == m2b::FREE && kind != alone(c);
+    if (own_kernel(c) && !free) seq.push_back(-1);
+    else if (kind == m2b::FUSED) {
         seq = {0, 1};
         for (uint32_t i = 1; i < iters; ++i) { seq.push_back(m2k::STAGE_MID); seq.push_back(1); }
         seq.push_back(2);
@@ -929,17 +1009,17 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
         for (uint32_t i = 0; i < iters; ++i) for (int st = 0; st < m2k::LARGE_STAGES; ++st) seq.push_back(st);
     }
     std::vector<cudaEvent_t> ev(seq.size() + 1);
-    for (auto& e : ev) if (cudaEventCreate(&e) != cudaSuccess) return M2_ECUDA;
-    cudaError_t err = in_turn(c, [&] {
-        cudaError_t r = cudaEventRecord(ev[0], c->stream);
-        for (size_t i = 0; i < seq.size() && r == cudaSuccess; ++i) {
-            if (seq[i] < 0) r = launch_own(c, iters);
-            else r = m2k::launch_large_stage(c->plan, c->bufs, seq[i], c->stream);
-            if (r == cudaSuccess) r = cudaEventRecord(ev[i + 1], c->stream);
-        }
-        return r;
-    });
+    cudaError_t err = cudaSuccess;
+    for (auto& e : ev) if (err == cudaSuccess) err = cudaEventCreate(&e);
+    if (err == cudaSuccess) err = cudaEventRecord(ev[0], c->stream);
+    if (free && c->flow) c->staged = true;
+    for (size_t i = 0; i < seq.size() && err == cudaSuccess; ++i) {
+        if (seq[i] < 0) err = launch_own(c, iters, false);
+        else err = m2k::launch_large_stage(free ? c->free_plan : c->plan, c->bufs, seq[i], c->stream);
+        if (err == cudaSuccess) err = cudaEventRecord(ev[i + 1], c->stream);
+    }
     if (err == cudaSuccess) err = cudaStreamSynchronize(c->stream);
+    board.done(*c->run);
     // per stage (in order of first appearance): total time and launches
     std::vector<int> order;
     std::map<int, std::pair<double, uint64_t>> tot;
@@ -952,9 +1032,10 @@ int m2_profile(m2_ctx* c, uint32_t iters, m2_stage_time* out, int max_stages, in
             tot[seq[i]].second += 1;
         }
     }
-    for (auto& e : ev) cudaEventDestroy(e);
+    for (auto& e : ev) if (e) cudaEventDestroy(e);
     if (err != cudaSuccess) return fail_cuda("m2_profile", err);
     c->iteration += iters;
+    if (const int rc = unstage(c)) return rc;
     const int k = std::min((int)order.size(), max_stages);
     for (int i = 0; i < k; ++i) {
         const int st = order[i];
@@ -1218,6 +1299,18 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         }
     } dv;
     const size_t nb = buckets.size();
+    struct Turn {   // in flight from here to the end of the call
+        m2b::Board& board;
+        std::shared_ptr<m2b::Run> run = std::make_shared<m2b::Run>();
+        explicit Turn(int device) : board(m2b::Board::of(device)) {
+            board.add(run);
+            board.begin(*run, m2b::BATCH);
+        }
+        ~Turn() {
+            board.done(*run);
+            board.remove(run);
+        }
+    } turn(device);
     dv.streams.resize(nb + 1, nullptr);
     for (auto& s : dv.streams) if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return M2_ECUDA;
     dv.events.resize(nb + 3, nullptr);
@@ -1374,6 +1467,7 @@ struct SrvBucket {
     cudaEvent_t ev = nullptr;
     std::vector<uint64_t> members;       // keys of the tests in the launch in flight
     std::vector<uint32_t> ks;
+    std::shared_ptr<m2b::Run> run;
     bool busy = false;
     bool whole = false;                  // its CTAs hold whole SMs (srv_launch)
 };
@@ -1533,8 +1627,17 @@ int srv_launch(m2_server* s) {
         if (e == cudaSuccess) e = cudaMemsetAsync(b.d_status, 0, cnt * sizeof(int), b.stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b.d_tests, b.h_tests, cnt * sizeof(m2k::SmallTest), cudaMemcpyHostToDevice, b.stream);
         if (e != cudaSuccess) return fail_cuda("server descriptor upload", e);
+        m2b::Board& board = m2b::Board::of(s->device);
+        if (!b.run) {
+            b.run = std::make_shared<m2b::Run>();
+            b.run->stream = b.stream;
+            board.add(b.run);
+        }
+        board.begin(*b.run, m2b::FREE);
         e = duo ? m2k::launch_duo(b.d_tests, (int)cnt, (unsigned)kv.first, 0u, b.stream, nullptr, 0, min_smem)
                 : m2k::launch_small(b.d_tests, (int)cnt, (unsigned)kv.first, threads, 0u, b.stream, fuse, false, min_smem);
+        const cudaError_t er = board.end(*b.run);
+        if (e == cudaSuccess) e = er;
         if (e != cudaSuccess)
             return fail_cuda("server small-test launch", e);
         e = cudaMemcpyAsync(b.h_status, b.d_status, cnt * sizeof(int), cudaMemcpyDeviceToHost, b.stream);
@@ -1733,6 +1836,7 @@ void m2_srv_destroy(m2_server* s) {
     }
     for (auto& kv : s->buckets) {
         SrvBucket& b = kv.second;
+        if (b.run) m2b::Board::of(s->device).remove(b.run);
         cudaFree(b.d_tests); cudaFree(b.d_status); cudaFreeHost(b.h_tests); cudaFreeHost(b.h_status);
         if (b.ev) cudaEventDestroy(b.ev);
         if (b.stream) cudaStreamDestroy(b.stream);

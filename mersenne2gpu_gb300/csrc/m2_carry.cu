@@ -347,6 +347,15 @@ cudaError_t launch_normalize(const NormArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+cudaError_t normalize_setup() {
+    cudaFuncAttributes at;
+    cudaError_t e = cudaSuccess;
+    for (const void* f : {(const void*)k_norm_init, (const void*)k_norm_blocks, (const void*)k_norm_scan, (const void*)k_norm_apply,
+                          (const void*)k_norm_ones, (const void*)k_balance})
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, f);
+    return e;
+}
+
 cudaError_t launch_balance(const u64* canon, i64* digits, u64 p, int ln, u64 n, unsigned* bad, cudaStream_t s) {
     const unsigned g = (unsigned)((n + 255) / 256 < 2048 ? (n + 255) / 256 : 2048);
     k_balance<<<g, 256, 0, s>>>(canon, digits, p, ln, n, bad);

@@ -77,9 +77,10 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
     Unit<S, X31> ub{zb, reinterpret_cast<X31*>(A.zb), A.tw4, A.tc, fb, 8};
     const bool has_cols = S::G == S::CTAS || x < S::G, has_rows = S::R / 2 == S::CTAS || x < S::R / 2;
     Wait w{A.status, false};
-    all_started(A.arrivals, S::CTAS, w);
+    if (!all_started(A.arrivals, S::CTAS, A.status, A.k, A.ask)) return;
     const u32 base = has_cols ? A.parity[x] : 0u;  // squarings handed over so far (bit 0); bit 1 never matches a word's tag
 
+    const u32 seg = A.seg;
     // this thread's carry segments: segment s holds elements 2s, 2s+1 of the
     // column group's slots (row 2s / C)
     u32 w61[S::SI], w31[S::SI];
@@ -99,8 +100,8 @@ __global__ void __launch_bounds__(S::NT, 1) k_flow(FlowArgs A) {
         const longlong2* src = reinterpret_cast<const longlong2*>(A.digits + 2ull * e0[q]);
         const longlong2 v0 = src[0], v1 = src[1];
         d[q][0] = v0.x; d[q][1] = v0.y; d[q][2] = v1.x; d[q][3] = v1.y;
-        if ((2 * e0[q]) % A.seg == 0) {
-            const u32 idx = 2 * e0[q] / A.seg, prev = idx ? idx - 1 : 2 * S::H / A.seg - 1;
+        if ((2 * e0[q]) % seg == 0) {
+            const u32 idx = 2 * e0[q] / seg, prev = idx ? idx - 1 : 2 * S::H / seg - 1;
             i64 c = A.carries[prev];
             A.carries[prev] = 0;
 #pragma unroll

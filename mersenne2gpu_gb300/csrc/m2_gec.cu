@@ -14,9 +14,10 @@
 //   D_t = Z 4^((t-1)(1 - 2^B)),  Z = 4 x_k0 D_(t-1)^(2^B),
 // where Z is formed by the same product and the power of two is a rotation of
 // the p-bit residue (2^p == 1), applied once per verification (k_gec_rotate).
-// The block products are enqueued without a host wait: the context's stream
-// hands the boundary state to the second context's stream through an event,
-// and waits for the product through another before its next squaring.
+// The block products are enqueued without a host wait (but where launches of the
+// block may have been called off, m2i::settle): the context's stream hands the
+// boundary state to the second context's stream through an event, and waits for
+// the product through another before its next squaring.
 #include "m2_internal.hpp"
 
 #include <cuda_runtime.h>
@@ -114,6 +115,13 @@ int cuda_rc(cudaError_t e) {
     return e == cudaErrorMemoryAllocation ? M2_ENOMEM : M2_ECUDA;
 }
 
+// c's squarings have run.  A state that its kernels reported as wrong is no error
+// here: the check finds it and rolls back.
+int settled(m2_ctx* c) {
+    const int rc = m2i::settle(c);
+    return rc == M2_ESTATE || rc == M2_ETIMEOUT ? M2_OK : rc;
+}
+
 // aux's state <- a +/- b (canonical vectors in device memory), canonical
 // digits of the result left in aux's canonical buffer
 int combine_into_aux(m2_gec* g, const ull* a, const ull* b, bool subtract, const ull** canon) {
@@ -133,8 +141,10 @@ int square_k(m2_gec* g, const ull* v, u32 k, const ull** canon) {
     if (rc) return rc;
     if (v != buf && (rc = cuda_rc(cudaMemcpyAsync(buf, v, g->L->n * sizeof(ull), cudaMemcpyDeviceToDevice, g->as)))) return rc;
     if ((rc = m2i::load_canon(g->aux, 0))) return rc;
-    if ((rc = m2_iterate(g->aux, k))) return rc;
-    return m2i::canonical(g->aux, canon);
+    // the one squaring of a product is not waited for
+    if (k == 1) rc = m2i::iterate_unowed(g->aux, 1);
+    else if (!(rc = m2_iterate(g->aux, k))) rc = settled(g->aux);
+    return rc ? rc : m2i::canonical(g->aux, canon);
 }
 
 // out = 4 a b mod 2^p - 1: canonical a, b, out in device memory, out distinct
@@ -165,7 +175,8 @@ int count_diff(m2_gec* g, const ull* a, const ull* b, unsigned* out) {
 // ctx's current canonical state copied to dst (ctx's stream, then waited for)
 int ctx_state(m2_gec* g, ull* dst) {
     const ull* c = nullptr;
-    int rc = m2i::canonical(g->ctx, &c);
+    int rc = settled(g->ctx);
+    if (!rc) rc = m2i::canonical(g->ctx, &c);
     if (!rc) rc = cuda_rc(cudaMemcpyAsync(dst, c, g->L->n * sizeof(ull), cudaMemcpyDeviceToDevice, g->cs));
     if (!rc) rc = cuda_rc(cudaStreamSynchronize(g->cs));
     return rc;
@@ -214,6 +225,7 @@ int m2_gec_create(m2_gec** out, m2_ctx* ctx, uint32_t block) {
     const m2_opts o = m2i::creation_opts(ctx);
     if ((rc = m2_create(&g->aux, info.p, M2_MODE_PRP, &o))) { delete g; return rc; }
     g->as = m2i::stream(g->aux);
+    m2i::share_turns(ctx, g->aux);
     const size_t bytes = g->L->n * sizeof(ull);
     // one allocation: the six vectors, then the counter
     rc = set_device(g);
@@ -250,6 +262,7 @@ int m2_gec_iterate(m2_gec* g, uint32_t k) {
         // the boundary state to the check's stream, D_(t+1) = 4 D_t x_(k0+(t+1)B),
         // and the chain's next squaring after the product
         const ull* c = nullptr;
+        if ((rc = settled(g->ctx))) break;
         if ((rc = m2i::canonical(g->ctx, &c))) break;
         if ((rc = cuda_rc(cudaMemcpyAsync(g->xb, c, bytes, cudaMemcpyDeviceToDevice, g->cs)))) break;
         if ((rc = cuda_rc(cudaEventRecord(g->to_aux, g->cs)))) break;

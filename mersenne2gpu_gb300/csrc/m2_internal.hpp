@@ -44,6 +44,16 @@ int canonical(m2_ctx* c, const unsigned long long** out);
 int raw_state(m2_ctx* c, long long** digits);
 // the context's canonical buffer (device memory, n words), allocated if needed
 int canon_buffer(m2_ctx* c, unsigned long long** buf);
+// where launches may have been called off (m2_board.hpp): waits for the context's
+// work and runs their squarings.  A read on the device, like canonical(), comes
+// after it.  The state's code
+int settle(m2_ctx* c);
+// m2_iterate by launches that are not called off; after it the state is read by
+// canonical() or replaced by load_canon()
+int iterate_unowed(m2_ctx* c, uint32_t k);
+// the runs of these contexts are ordered by events: neither keeps the other off
+// the device
+void share_turns(m2_ctx* a, m2_ctx* b);
 // state <- the canonical digits in the canonical buffer (balanced on the
 // device), with the iteration counter set
 int load_canon(m2_ctx* c, uint32_t iteration);

@@ -13,6 +13,15 @@ enum Mode : int { LL = 0, PRP = 1, PRP3 = 2 };
 // Status word written by kernels (0 = ok).
 enum Status : int { ST_OK = 0, ST_CARRY_RANGE = 1, ST_NORMALIZE = 2, ST_WAIT_TIMEOUT = 4 };
 
+// A context's words for its host: the status, and the squarings that one-launch
+// kernels (m2_flow.cu, m2_tide.cu) were to run but did not start on.
+struct StateWords {
+    int status;
+    int pad;
+    unsigned long long owed;
+    const unsigned* yield;   // host word, not 0: launches that ask are called off (or null)
+};
+
 // One independent test for the whole-iteration-in-one-CTA kernel.
 struct SmallTest {
     long long* digits;        // n balanced digits (in/out)
@@ -74,11 +83,12 @@ struct FlowArgs {
     const DTw* tw4;
     const DTw* tc;
     unsigned long long* fcar;  // flow_carry_words tagged segment carries
-    unsigned long long* arrivals;   // CTAs started, over all launches
+    unsigned long long* arrivals;   // CTAs started, over all launches, and the marks of launches that did not run
     unsigned int* parity;      // flow_groups words: squarings done, modulo 2
-    int* status;
+    int* status;               // of the context's StateWords
     unsigned int k;            // squarings of this launch (>= 1)
-    unsigned int seg;          // digits per pending carry segment
+    unsigned short seg;        // digits per pending carry segment
+    unsigned short ask;        // 1: the launch looks at StateWords::yield first
     int span;                  // at most 3
     int mode;
 };
@@ -146,6 +156,7 @@ struct NormArgs {
 size_t norm_scratch_bytes(unsigned long long n);
 void norm_bind_scratch(NormArgs& a, void* scratch);
 cudaError_t launch_normalize(const NormArgs& a, cudaStream_t s);
+cudaError_t normalize_setup();   // loads its kernels and launch_balance's (see pass_setup)
 // canonical digits -> balanced digits with no pending carries; *bad |= 1 when
 // an input digit is not canonical (bad may be null)
 cudaError_t launch_balance(const unsigned long long* canon, long long* digits, unsigned long long p, int ln,

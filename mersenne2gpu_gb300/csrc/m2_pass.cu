@@ -117,6 +117,29 @@ template <int LR_, int LB_> struct ColShape {
 
 }  // namespace
 
+cudaError_t pass_setup(const LargePlan& P) {
+#if M2_DUAL
+    if (P.gf61) return m2k_g61::pass_setup(P);
+#endif
+    cudaFuncAttributes at;
+    cudaError_t e = cudaSuccess;
+    if (pair_supported(P)) {
+#define M2_PAIR_A(LR, LB) if (P.R == 1u << LR && P.B == 1u << LB) e = cudaFuncGetAttributes(&at, k_pair<Shape<LR, LB>>);
+        M2_PAIR_SHAPES(M2_PAIR_A)
+#undef M2_PAIR_A
+    }
+    if (col4_supported(P)) {
+#define M2_COL4_A(LR, LB)                                                                        \
+    if (P.R == 1u << LR && P.B == 1u << LB) {                                                    \
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, k_col4_fwd<ColShape<LR, LB>>);      \
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, k_col4_inv<ColShape<LR, LB>>);      \
+    }
+        M2_COL4_SHAPES(M2_COL4_A)
+#undef M2_COL4_A
+    }
+    return e;
+}
+
 // rows of 1024 and 2048 elements where the plan asks for them
 bool pair_supported(const LargePlan& P) {
     if (P.B >= 1024u && !P.in_turn) return false;

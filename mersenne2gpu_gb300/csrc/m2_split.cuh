@@ -199,26 +199,52 @@ struct Wait {
         return true;
     }
 };
-// Every CTA of a cooperative launch waits here until all of them have started.
-// The hardware may start some while kernels of other streams hold the other
-// SMs, for as long as those keep coming, so this wait has a limit of its own
-// (100 s); the waits after it are between running CTAs.
-__device__ __forceinline__ void all_started(unsigned long long* arrivals, u32 ctas, Wait& w) {
-    __shared__ int gave_up;
+// Every CTA of a cooperative launch waits here until all of them have started;
+// false: the launch is called off, for all of them.  The state stays as it was
+// then, and the k squarings are added to those that the host still has to run
+// (StateWords::owed).  A launch that asks (`ask`) is called off by its first CTA
+// when the context's host word says that other work waits: queued launches give
+// way within the one that runs.  CTAs whose grid does not start whole would call
+// it off after 20 ms; on a GB300 all CTAs of a cooperative grid start at one
+// instant (measured beside kernels that came free one by one).
+//
+// arrivals: the low 48 bits count the CTAs of all launches, bits 62 and 63 mark a
+// launch of even and odd index as called off.  A mark is set while the count is
+// short of the launch's last CTA (by the first CTA before it counts itself, by
+// others with compare-and-swap), so a CTA that sees the full count without the
+// mark sees what all the others see; the first CTA to arrive of the next launch
+// takes it away, when every CTA of this one has read it.
+__device__ __forceinline__ bool all_started(unsigned long long* arrivals, u32 ctas, int* status, u32 k, u32 ask) {
+    __shared__ int runs;
     if (threadIdx.x == 0) {
-        gave_up = 0;
-        const u64 old = atomicAdd(arrivals, 1ull), target = (old / ctas + 1) * ctas, t0 = now_ns();
-        while ((i64)(*(volatile u64*)arrivals - target) < 0) {
-            __nanosleep(200);
-            if (now_ns() - t0 > 100000000000ull || (*(volatile int*)w.status & ST_WAIT_TIMEOUT)) {
-                atomicOr(w.status, ST_WAIT_TIMEOUT);
-                gave_up = 1;
-                break;
-            }
+        StateWords* words = reinterpret_cast<StateWords*>(status);
+        constexpr u64 COUNT = (1ull << 48) - 1;
+        const volatile unsigned* yield = ask && blockIdx.x == 0 ? words->yield : nullptr;
+        const bool give_way = yield && *yield;
+        const u64 t0 = now_ns();
+        u64 v = *(volatile u64*)arrivals;
+        if (!give_way) v = atomicAdd(arrivals, 1ull);
+        // (other CTAs of this launch may arrive meanwhile, but not its last)
+        const u64 launch = (v & COUNT) / ctas, full = (launch + 1) * ctas, off = 1ull << (62 + (launch & 1));
+        if (give_way) {
+            if (!(atomicOr(arrivals, off) & off)) atomicAdd(&words->owed, (unsigned long long)k);
+            v = atomicAdd(arrivals, 1ull);
         }
+        if ((v & COUNT) == launch * ctas) atomicAnd(arrivals, ~(1ull << (63 - (launch & 1))));   // the mark of the launch before
+        do {
+            v = *(volatile u64*)arrivals;
+            if ((v & off) || (v & COUNT) >= full) break;
+            if (now_ns() - t0 < 20000000ull) {
+                __nanosleep(200);
+            } else if (atomicCAS(arrivals, v, v | off) == v) {
+                atomicAdd(&words->owed, (unsigned long long)k);
+                v |= off;
+            }
+        } while (!(v & off));
+        runs = !(v & off);
     }
     __syncthreads();
-    w.dead = gave_up != 0;
+    return runs != 0;
 }
 
 }  // namespace

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(S::NT, 1) k_tide(TideArgs TA) {
     Unit<S, X61> ua{za + part * 2 * S::B, ga, A.tw4, A.tc, tid % S::NF, 1 + S::BARS * part};
     Unit<S, X31> ub{zb + part * 2 * S::B, gb, A.tw4, A.tc, tid % S::NF, 1 + S::BARS * part};
     Wait w{A.status, false};
-    all_started(A.arrivals, gridDim.x, w);
+    if (!all_started(A.arrivals, gridDim.x, A.status, A.k, A.ask)) return;
     const u32 base = A.parity[cta];      // squarings handed over so far (bit 0); bit 1 never matches a word's tag
     const u32 r = tid;                   // this thread's row in the row stage
     const u32 mul = (A.mode == PRP3) ? 3u : 1u;
