@@ -197,6 +197,12 @@ struct Slab {
     std::vector<Part> parts;
     template <class T> void add(T** p, size_t bytes) { parts.push_back(Part{(void**)p, bytes}); }
     int alloc(m2_ctx* c, void** base) {
+        // (recorded by a capture, the memory would be the graph's, not the context's)
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return fail_cuda("allocation", cudaErrorStreamCaptureUnsupported);
+        }
         cudaMemPool_t mp = ctx_pool(c->device);
         if (!mp) return M2_ECUDA;
         size_t total = 0;
@@ -507,7 +513,9 @@ int advance(m2_ctx* c, uint32_t k, m2b::Kind most) {
     if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         // recorded for the caller to replay: the kernels of a context alone
         cudaGetLastError();
+        const bool staged = c->staged;
         int rc = unstage(c);
+        c->staged = staged;   // the state's, which changes when the graph is replayed
         if (rc) return rc;
         const cudaError_t e = own_kernel(c) ? launch_own(c, k, false) : launch_passes(c, k, false);
         return e == cudaSuccess ? M2_OK : fail_cuda("m2_iterate launch", e);
@@ -945,7 +953,11 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
     if (c->path != M2_PATH_LARGE) return M2_EUNSUPPORTED;
     if (cudaSetDevice(c->device) != cudaSuccess) return M2_ECUDA;
     if (const int rc = c->flow ? settle(c) : M2_OK) return rc;
-    c->staged = c->flow || c->cluster;
+    if (c->flow || c->cluster) {
+        // what unstage needs, also under a capture
+        if (const int rc = canon_alloc(c)) return rc;
+        c->staged = true;
+    }
     cudaError_t e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
     const size_t h = c->L.h;
     if (e == cudaSuccess && za_out) e = m2i::read_back(za_out, c->d_za, 16 * h, c->stream);

@@ -44,3 +44,48 @@ def test_contexts_destroyed_with_work_in_flight(m2):
                     e.iterate(40)
                     got.append(e.res64())
             assert got == want
+
+
+@pytest.mark.parametrize("p", [9941, 216091, 1257787, 57885161])
+def test_nothing_is_created_under_capture(m2, p):
+    """A context on a stream that is being captured is refused, as is a read that
+    has no buffer yet: their memory would be the graph's.  The capture goes on."""
+    import torch
+    s = torch.cuda.Stream()
+    with m2.Engine(p, 1, stream=s.cuda_stream) as e, m2.Engine(p, 1) as ref:
+        e.iterate(3)
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            with pytest.raises(m2.M2Error, match=r"\(-3\)"):
+                m2.Engine(p, 1, stream=s.cuda_stream)
+            with pytest.raises(m2.M2Error, match=r"\(-3\)"):
+                e.digits()
+            e.iterate(4)
+        with torch.cuda.stream(s):
+            g.replay()
+        s.synchronize()
+        ref.iterate(7)
+        assert np.array_equal(e.digits(), ref.digits())
+
+
+@pytest.mark.parametrize("p", [216091, 1257787, 57885161])
+def test_capture_after_three_pass_stages(m2, p):
+    """Squarings recorded while the state is as three-pass stages left it: for the
+    replays, and for calls that come before any."""
+    import torch
+    s = torch.cuda.Stream()
+    with m2.Engine(p, 1, stream=s.cuda_stream) as e, m2.Engine(p, 1) as ref:
+        for stage in (0, 1, 2):
+            e.test_stage(stage)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            e.iterate(2)
+        e.iterate(3)
+        for _ in range(2):
+            with torch.cuda.stream(s):
+                g.replay()
+        s.synchronize()
+        e.iterate(1)
+        ref.iterate(1 + 3 + 2 * 2 + 1)
+        assert np.array_equal(e.digits(), ref.digits())
