@@ -167,6 +167,7 @@ struct m2_ctx {
     bool cluster = false;      // squarings run in one thread-block cluster (m2_cluster.cu)
     bool stall = false;        // its next launch waits for a carry that never comes (m2_test_stall_fused)
     bool staged = false;       // a three-pass stage ran since: pending carries, untagged elements
+    bool untagged = false;     // three-pass kernels wrote the elements last
     m2k::FlowArgs fargs{};
     char* d_flow = nullptr;    // its tagged carries, arrival counter and parity words
     uint2* d_taux = nullptr;   // the large sizes' row-stage tables and parked digits
@@ -291,6 +292,7 @@ cudaError_t flow_reset(m2_ctx* c) {
     cudaError_t e = cudaMemsetAsync(c->d_za, 0xff, sizeof(ulonglong2) * c->L.h, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_zb, 0xff, sizeof(uint2) * c->L.h, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flow, 0, c->flow_bytes, c->stream);
+    c->untagged = false;
     return e;
 }
 
@@ -494,6 +496,7 @@ int run_passes(m2_ctx* c, uint64_t k, bool free) {
     for (int i = 0; i < 2; ++i)
         ready[i] = k >= GRAPH_ITERS[i] && (i == 0 || k % GRAPH_ITERS[0] >= GRAPH_ITERS[1] || !ready[0]) && ensure_graph(c, i, free);
     cudaError_t e = cudaSuccess;
+    c->untagged = true;
     if (c->flow) c->staged = true;
     for (int i = 0; i < 2; ++i)
         if (ready[i])
@@ -958,8 +961,15 @@ int m2_test_stage(m2_ctx* c, int stage, void* za_out, void* zb_out) {
         if (const int rc = canon_alloc(c)) return rc;
         c->staged = true;
     }
-    cudaError_t e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
     const size_t h = c->L.h;
+    cudaError_t e = cudaSuccess;
+    // a stage out of order: its kernels poll for elements without tags (m2_pass.cu)
+    if (stage != 0 && !c->untagged) {
+        e = cudaMemsetAsync(c->d_za, 0, 16 * h, c->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->d_zb, 0, 8 * h, c->stream);
+    }
+    c->untagged = true;
+    if (e == cudaSuccess) e = m2k::launch_large_stage(c->plan, c->bufs, stage, c->stream);
     if (e == cudaSuccess && za_out) e = m2i::read_back(za_out, c->d_za, 16 * h, c->stream);
     if (e == cudaSuccess && zb_out) e = m2i::read_back(zb_out, c->d_zb, 8 * h, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);

@@ -51,3 +51,20 @@ def test_stage_model_catches_a_planted_fault(oracle_mod):
     bad[13] = ((bad[13][0] + 1) % S.P31, bad[13][1])
     with pytest.raises(AssertionError, match="row 1 of 8, column 5"):
         _first_diff(bad, res, 8, 8, "planted")
+
+
+@pytest.mark.parametrize("p", [216091, 1257787, 24036583])
+@pytest.mark.parametrize("path", [0, 2])
+def test_stage_out_of_order_waits_for_nothing(m2, p, path):
+    """The row or inverse column pass without a pass before it: meaningless, but no
+    error, also on a context whose kernel tags its elements."""
+    for stage in (1, 2):
+        with m2.Engine(p, 1, path=path) as e, m2.Engine(p, 1, path=path) as ref:
+            start = e.digits()
+            if stage == 2:
+                e.iterate(2)
+            e.test_stage(stage)
+            e.set_digits(start, 0)
+            e.iterate(3)
+            ref.iterate(3)
+            assert (e.digits() == ref.digits()).all()
