@@ -152,7 +152,8 @@ void m2_destroy(m2_ctx* ctx);
  * are shared by every test of that size and cached for the process, outside
  * the budget).  Shared one-CTA launches take the batch autotuner's launch
  * shape for their transform size when m2_batch_run has tuned it in this
- * process, else the default shape.
+ * process for as many tests (fewer than the device's SMs, or more), else the
+ * default shape.
  * Results of a test are identical to running it alone (m2_create/m2_iterate).
  * Times are seconds since m2_srv_create (host steady clock). */
 typedef struct m2_server m2_server;
@@ -362,7 +363,9 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
  * `device` (autotuned on the first batch containing that size: every candidate
  * 32 ... 256 times a sample of the batch's own tests; the carry split follows;
  * the fields-in-turn kernel's 512 and 1024 threads at ln = 13, 14 read 256),
- * and the measured nanoseconds per test-squaring.  M2_EINVAL if not tuned yet. */
+ * and the measured nanoseconds per test-squaring.  M2_EINVAL if not tuned yet.
+ * Batches of fewer tests than the device has SMs are tuned for themselves; this
+ * and m2_batch_tuning report the choice for the larger ones where there is one. */
 int m2_batch_tuned(int device, int ln, int* threads, double* ns_per_test_iter);
 
 /* The full choice of the batch autotuner for transform size 2^ln on `device`
@@ -393,6 +396,9 @@ typedef struct {
     double ns_default;        /* the same for the untuned default (h/4 threads, one segment per thread, unfused) */
 } m2_batch_tuning_t;
 int m2_batch_tuning(int device, int ln, m2_batch_tuning_t* out);
+/* The kernel of that choice: "k_duo" (the two fields in turn) or "k_small" (both
+ * together, by the three knobs); NULL if not tuned yet. */
+const char* m2_batch_kernel(int device, int ln);
 
 #ifdef __cplusplus
 }

@@ -27,7 +27,7 @@ EXPORTS = (
     "m2_profile", "m2_launches_for", "m2_measure_mul_peak", "m2_square_noalloc",
     "m2_srv_create", "m2_srv_submit", "m2_srv_step", "m2_srv_poll", "m2_srv_stats_get", "m2_srv_active_get",
     "m2_srv_destroy",
-    "m2_last_error", "m2_carry_normalize", "m2_batch_tuned", "m2_batch_tuning", "m2_layout_fields", "m2_test_stall_fused",
+    "m2_last_error", "m2_carry_normalize", "m2_batch_tuned", "m2_batch_tuning", "m2_batch_kernel", "m2_layout_fields", "m2_test_stall_fused",
     "m2_test_stage",
     "m2_gec_create", "m2_gec_iterate", "m2_gec_check", "m2_gec_verified", "m2_gec_stats_get", "m2_gec_destroy",
 )
@@ -110,6 +110,8 @@ def _lib() -> ctypes.CDLL:
         L.m2_test_stage.argtypes = [vp, i, vp, vp]
         L.m2_batch_tuned.argtypes = [i, i, ctypes.POINTER(i), ctypes.POINTER(ctypes.c_double)]
         L.m2_batch_tuning.argtypes = [i, i, ctypes.POINTER(_BatchTuning)]
+        L.m2_batch_kernel.argtypes = [i, i]
+        L.m2_batch_kernel.restype = ctypes.c_char_p
         L.m2_last_error.argtypes = []
         L.m2_gec_create.argtypes = [ctypes.POINTER(vp), vp, u32]
         L.m2_gec_iterate.argtypes = [vp, u32]
@@ -119,7 +121,8 @@ def _lib() -> ctypes.CDLL:
         L.m2_gec_destroy.argtypes = [vp]
         L.m2_last_error.restype = ctypes.c_char_p
         for name in EXPORTS:
-            if name not in ("m2_destroy", "m2_strerror", "m2_launches_for", "m2_last_error", "m2_gec_destroy") \
+            if name not in ("m2_destroy", "m2_strerror", "m2_launches_for", "m2_last_error", "m2_gec_destroy",
+                            "m2_batch_kernel") \
                     and not name.startswith("m2_srv"):
                 getattr(L, name).restype = i
         _LIB = L
@@ -377,11 +380,11 @@ def batch_tuned(ln: int, device: int = 0) -> tuple[int, float] | None:
 def batch_tuning(ln: int, device: int = 0) -> dict | None:
     """The batch autotuner's choice for transform size 2^ln (None if not tuned):
     threads per transform, carry blocks and their length in digit pairs (-B),
-    fused or separate transform middle, and the measured ns per test-squaring
-    of the choice and of the untuned default."""
+    fused or separate transform middle, the kernel, and the measured ns per
+    test-squaring of the choice and of the untuned default."""
     t = _BatchTuning()
     if _lib().m2_batch_tuning(device, ln, ctypes.byref(t)) != 0:
         return None
     return {"threads": t.threads, "carry_blocks": t.carry_blocks, "carry_pairs": t.carry_pairs,
             "fused_middle": t.fused_middle, "ns_per_test_squaring": t.ns_per_test_iter,
-            "ns_default": t.ns_default}
+            "ns_default": t.ns_default, "kernel": _lib().m2_batch_kernel(device, ln).decode()}

@@ -20,6 +20,7 @@
 #include <chrono>
 #include <deque>
 #include <thread>
+#include <tuple>
 
 using m2::i64;
 using m2::u32;
@@ -1119,11 +1120,21 @@ struct Tuned {
     // most that a caller may ask for
     bool duo = false;
     double ns_per_test_iter = 0.0, ns_default = 0.0;
-    int carry_blocks(const m2::Layout& L, int span) const { return small_carry_threads(L, span, threads, carry_shift); }
+    int blocks = 0;            // carry segments of the choice, and digits
+    int n = 0;
 };
 std::mutex g_tune_mu;
-std::map<std::pair<int, u64>, Tuned> g_tune;
-std::map<std::pair<int, u64>, std::pair<int, int>> g_tune_shape;   // (device, h) -> (carry blocks, n) of the choice
+// per device, size and whether the tests in flight fill the GPU (a test per SM and
+// more): a few tests of n = 512 are faster in the one-CTA kernel, a full GPU of
+// them in m2_duo.cu's, so neither's choice is the other's
+std::map<std::tuple<int, u64, bool>, Tuned> g_tune;
+bool find_tuned(int device, u64 h, bool full, Tuned& out) {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tune.find({device, h, full});
+    if (it == g_tune.end()) return false;
+    out = it->second;
+    return true;
+}
 constexpr u32 TUNE_ITERS = 48;
 
 // m2_duo.cu's kernel serves these tests of one size (both fields)
@@ -1136,17 +1147,14 @@ bool duo_for(const std::vector<m2k::SmallTest>& tests) {
 template <class Item>
 int tune_bucket(int device, u64 h, const std::vector<Item>& items, const std::vector<m2k::SmallTest>& tests,
                 const long long* d_dig, int sms, size_t total, Tuned& out) {
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune.find({device, h});
-        if (it != g_tune.end()) { out = it->second; return M2_OK; }
-    }
+    const bool fills = total >= (size_t)sms;
+    if (find_tuned(device, h, fills, out)) return M2_OK;
     const u64 n = 2 * h;
     // A batch of at least a test per SM is timed as a full GPU, the bucket's tests
     // repeated: a last wave that is not full would count against the kernel with
     // more tests per SM (n = 4096, 498 tests, m2_duo.cu: 143 ns per test-squaring for 118 in full waves).
     const size_t full = (size_t)std::max(sms, 1) * std::min<size_t>(32, std::max<size_t>(1, 232448 / (24 * h)));
-    const size_t cap = total >= (size_t)sms ? full : items.size();
+    const size_t cap = fills ? full : items.size();
     long long* scratch = nullptr;
     m2k::SmallTest* d_t = nullptr;
     int* d_st = nullptr;
@@ -1242,41 +1250,47 @@ int tune_bucket(int device, u64 h, const std::vector<Item>& items, const std::ve
     }
     if (e != cudaSuccess) { cleanup(); return fail_cuda("batch tuning", e); }
     cleanup();
+    best.blocks = small_carry_threads(items[0].L, items[0].span, best.threads, best.carry_shift);
+    best.n = (int)n;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[{device, h}] = best;
-    g_tune_shape[{device, h}] = {best.carry_blocks(items[0].L, items[0].span), (int)n};
+    g_tune[{device, h, fills}] = best;
     out = best;
     return M2_OK;
 }
 
 }  // namespace
 
+// the choice on a full GPU, else the one for fewer tests
+static bool tuned_for(int device, int ln, Tuned& t) {
+    const u64 h = u64(1) << (ln - 1);
+    return find_tuned(device, h, true, t) || find_tuned(device, h, false, t);
+}
+
 extern "C" {
 
 int m2_batch_tuned(int device, int ln, int* threads, double* ns_per_test_iter) {
-    if (ln < 3 || ln > 14) return M2_EINVAL;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune.find({device, u64(1) << (ln - 1)});
-    if (it == g_tune.end()) return M2_EINVAL;
-    if (threads) *threads = it->second.threads;
-    if (ns_per_test_iter) *ns_per_test_iter = it->second.ns_per_test_iter;
+    Tuned t;
+    if (ln < 3 || ln > 14 || !tuned_for(device, ln, t)) return M2_EINVAL;
+    if (threads) *threads = t.threads;
+    if (ns_per_test_iter) *ns_per_test_iter = t.ns_per_test_iter;
     return M2_OK;
 }
 
 int m2_batch_tuning(int device, int ln, m2_batch_tuning_t* out) {
-    if (ln < 3 || ln > 14 || !out) return M2_EINVAL;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    const u64 h = u64(1) << (ln - 1);
-    auto it = g_tune.find({device, h});
-    auto sh = g_tune_shape.find({device, h});
-    if (it == g_tune.end() || sh == g_tune_shape.end()) return M2_EINVAL;
-    out->threads = it->second.threads;
-    out->carry_blocks = sh->second.first;
-    out->carry_pairs = sh->second.first ? sh->second.second / (2 * sh->second.first) : 0;
-    out->fused_middle = it->second.fuse;
-    out->ns_per_test_iter = it->second.ns_per_test_iter;
-    out->ns_default = it->second.ns_default;
+    Tuned t;
+    if (ln < 3 || ln > 14 || !out || !tuned_for(device, ln, t)) return M2_EINVAL;
+    out->threads = t.threads;
+    out->carry_blocks = t.blocks;
+    out->carry_pairs = t.blocks ? t.n / (2 * t.blocks) : 0;
+    out->fused_middle = t.fuse;
+    out->ns_per_test_iter = t.ns_per_test_iter;
+    out->ns_default = t.ns_default;
     return M2_OK;
+}
+const char* m2_batch_kernel(int device, int ln) {
+    Tuned t;
+    if (ln < 3 || ln > 14 || !tuned_for(device, ln, t)) return nullptr;
+    return t.duo ? "k_duo" : "k_small";
 }
 
 // Tests are bucketed by transform length h; every bucket is one persistent
@@ -1625,12 +1639,7 @@ int srv_launch(m2_server* s) {
         // cached, else the first member's; every member gets the launch's variant
         const m2_ctx* c0 = s->active[kv.second[0]].ctx;
         Tuned tn;
-        bool tuned = false;
-        {
-            std::lock_guard<std::mutex> lk(g_tune_mu);
-            auto f = g_tune.find({s->device, kv.first});
-            if (f != g_tune.end()) { tn = f->second; tuned = true; }
-        }
+        const bool tuned = find_tuned(s->device, kv.first, total >= (size_t)s->sms, tn);
         bool duo = !tuned || tn.duo;
         for (size_t j = 0; j < cnt && duo; ++j) duo = duo_for({s->active[kv.second[j]].ctx->h_test});
         const int threads = tuned ? tn.threads : c0->threads;
