@@ -20,6 +20,10 @@ using i64 = int64_t;
 constexpr u64 P61 = (u64(1) << 61) - 1;
 constexpr u32 P31 = (u32(1) << 31) - 1;
 
+// The IBDWT shift lr x modulo m = 61 or 31 (lr < m): the factor x, up to n, is
+// reduced first, so that the product fits 32 bits at every n.
+constexpr u32 weight_shift(u32 lr, u32 x, u32 m) { return lr * (x % m) % m; }
+
 // Dual-field element as stored in the twiddle tables: GF(P61^2) pair + GF(P31^2) pair.
 struct alignas(8) Dual {
     u64 a, b;   // GF(P61^2): a + b i

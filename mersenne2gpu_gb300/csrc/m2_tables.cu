@@ -85,8 +85,8 @@ __device__ __forceinline__ void init_element(const TestInit& T, u32 k) {
 #pragma unroll
     for (u32 c = 0; c < 2; ++c) {
         const u32 j = 2 * k + c, r = (u32)((u64)T.p * j) & (n - 1);
-        s61[c] = j ? (lr61 * (n - r)) % 61u : 0u;
-        s31[c] = j ? (lr31 * (n - r)) % 31u : 0u;
+        s61[c] = j ? m2::weight_shift(lr61, n - r, 61u) : 0u;
+        s31[c] = j ? m2::weight_shift(lr31, n - r, 31u) : 0u;
         const u32 a = (s61[c] + (u32)T.ln + 1u) % 61u, b = (s31[c] + (u32)T.ln + 1u) % 31u;
         u61[c] = a ? 61u - a : 0u;
         u31[c] = b ? 31u - b : 0u;

@@ -146,3 +146,29 @@ def test_radix8_ranges_and_value():
             for c in range(2):
                 assert x[m][c] <= P61 + 8 and (x[m][c] - 8 * u[m][c]) % P61 == 0
         unradix8(u)                          # ranges alone
+
+
+def test_weight_shift_at_every_transform_size(tmp_path):
+    """The device's shifts n^-1 (n - p j mod n) mod 61 and 31 up to n = 2^30, from
+    the header that the table kernel includes, against whole numbers."""
+    import os
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mersenne2gpu_gb300", "csrc")
+    src = tmp_path / "s.cpp"
+    src.write_text('#include "m2_host.hpp"\n#include <cstdio>\nint main() { unsigned lr, x, m;\n'
+                   'while (std::scanf("%u %u %u", &lr, &x, &m) == 3) std::printf("%u\\n", m2::weight_shift(lr, x, m)); }\n')
+    exe = tmp_path / "s"
+    subprocess.run(["g++", "-std=c++17", "-I", csrc, "-o", str(exe), str(src)], check=True)
+    rng = random.Random(61)
+    cases = []
+    for ln in range(3, 31):
+        n = 1 << ln
+        for m in (61, 31):
+            lr = (1 << (m - 1 - ln)) % m
+            assert lr * n % m == 1
+            cases += [(lr, x, m) for x in [1, 2, n // 2, n - 1, n] + [rng.randrange(1, n + 1) for _ in range(40)]]
+    out = subprocess.run([str(exe)], input="\n".join("%d %d %d" % c for c in cases), capture_output=True, text=True, check=True).stdout
+    assert [int(v) for v in out.split()] == [lr * x % m for lr, x, m in cases]
+    # the product as it was, in 32 bits, is wrong from n = 2^27 on
+    wrong = min(x for lr, x, m in cases if lr * x % (1 << 32) % m != lr * x % m)
+    assert wrong > 1 << 26
