@@ -852,14 +852,15 @@ int m2_set_digits(m2_ctx* c, const uint64_t* digits, uint32_t iteration) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return fail_cuda("state upload", e);
     if (bad) {
-        std::vector<u64> canon;
-        const m2::Layout L = m2::make_layout(c->L.p, c->gf61 ? 61 : 92);
         try {
-            canon = m2::canonical_from_unsigned(L, digits);
+            const m2::Layout L = m2::make_layout(c->L.p, c->gf61 ? 61 : 92);
+            rc = upload_state(c, L, m2::canonical_from_unsigned(L, digits));
+        } catch (const std::bad_alloc&) {
+            rc = M2_ENOMEM;
         } catch (const std::exception&) {
-            return M2_EINVAL;
+            rc = M2_EINVAL;
         }
-        if ((rc = upload_state(c, L, canon))) return rc;
+        if (rc) return rc;
         cudaMemset(c->d_status, 0, sizeof(int));
     }
     c->iteration = iteration;
