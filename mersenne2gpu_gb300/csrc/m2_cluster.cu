@@ -282,6 +282,10 @@ __global__ void __launch_bounds__(S::NT, 1) k_cluster(const SmallTest* test, u32
         T.digits[2 * k] = d0; T.digits[2 * k + 1] = d1;
     }
     cluster_sync();   // no CTA leaves while another may still write to it
+    // words for a warp that has given up are not waited for: the last of them were
+    // sent before the barrier, and its CTA stays for far longer than one takes
+    if (w.dead)
+        for (const u64 t0 = now_ns(); now_ns() - t0 < 20000ull;) {}
 }
 
 template <class S> cudaError_t config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, cudaStream_t s) {
