@@ -1317,9 +1317,24 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     // device memory from the stream-ordered pool: a call neither waits for nor
-    // holds up other work on the device
+    // holds up other work on the device.  What the pool grew by goes back at the
+    // end, but for 256 MiB that the next call finds ready (the tests of a full GPU
+    // take 10 to 50 MB).
     cudaMemPool_t mp = ctx_pool(device);
     if (!mp) return M2_ECUDA;
+    struct Trim {
+        cudaMemPool_t mp;
+        uint64_t keep = 0;
+        explicit Trim(cudaMemPool_t pool) : mp(pool) {
+            if (cudaMemPoolGetAttribute(mp, cudaMemPoolAttrReservedMemCurrent, &keep) != cudaSuccess) cudaGetLastError();
+            keep = std::max<uint64_t>(keep, 256ull << 20);
+        }
+        ~Trim() {
+            uint64_t now = 0;
+            if (cudaMemPoolGetAttribute(mp, cudaMemPoolAttrReservedMemCurrent, &now) != cudaSuccess) cudaGetLastError();
+            if (now > keep && cudaMemPoolTrimTo(mp, keep) != cudaSuccess) cudaGetLastError();
+        }
+    } trim(mp);
     struct Dev {
         std::vector<void*> allocs;
         std::vector<cudaStream_t> streams;
@@ -1327,8 +1342,10 @@ int m2_batch_run(const uint32_t* p, const int* modes, const uint32_t* iters, siz
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         ~Dev() {
-            if (!streams.empty() && streams[0])
+            if (!streams.empty() && streams[0]) {
                 for (auto a : allocs) cudaFreeAsync(a, streams[0]);
+                cudaStreamSynchronize(streams[0]);
+            }
             if (exec) cudaGraphExecDestroy(exec);
             if (graph) cudaGraphDestroy(graph);
             for (auto e : events) if (e) cudaEventDestroy(e);
