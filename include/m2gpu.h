@@ -109,9 +109,10 @@ int m2_create(m2_ctx** out, uint32_t p, int mode, const m2_opts* opts);
  * next m2_sync, m2_get_digits, m2_res64, m2_verdict or m2_test_stage
  * call, which waits for them.  Kernels that this library does not know of (the
  * caller's own, m2_square_noalloc, replays of graphs that the caller captured)
- * may delay such a launch until there is room for all of it.  Replays of graphs
- * captured from contexts whose info says fused_cols are the caller's to order
- * behind other contexts' work. */
+ * may delay such a launch until there is room for all of it.  A call on a stream
+ * under capture records the kernels of a context alone: replays that run beside
+ * other work are the caller's to order where those are the fused column passes
+ * (M2_PATH_LARGE from n = 2^19 on, and n = 2^23), whose waits have a limit. */
 int m2_iterate(m2_ctx* ctx, uint32_t k);
 
 /* Replaces clFinish at a report point (mersenne2_gpu.cpp:4788); also reports
@@ -261,12 +262,14 @@ int m2_square_noalloc(uint32_t p, int mode, int64_t* digits, uint32_t iters, voi
 int m2_carry_normalize(uint32_t p, const int64_t* digits, const int64_t* seg_carries, uint32_t seg_digits,
                        uint64_t* out, void* stream);
 
-/* Test hook of the fused column kernel's bounded wait (no GPU fault): raises
- * the epoch flag of column CTA 0 by 2^20, so in the next fused launch CTA 0
- * waits for a flag value that its predecessor never writes; the wait gives up
+/* Test hook of the bounded waits between CTAs (no GPU fault): in the next launch
+ * of the context's kernel a wait is for a value that never comes -- the one-launch
+ * kernels of n = 2^14 ... 2^22 for a segment carry of a tag that no word has, the
+ * cluster kernel of n = 2^9 ... 2^13 for one carry more than there are, the fused
+ * column kernel for an epoch flag 2^20 above its predecessor's.  The wait gives up
  * after its limit, the launch completes, and m2_sync reports M2_ETIMEOUT.  The
  * state is then meaningless until m2_set_digits reloads it (which also resets
- * the flags).  M2_EUNSUPPORTED when the context has no fused column pass. */
+ * tags and flags).  M2_EUNSUPPORTED for contexts whose kernels wait for nothing. */
 int m2_test_stall_fused(m2_ctx* ctx);
 
 /* Test hook for stage-by-stage checks of the three-pass path: runs one stage
