@@ -53,6 +53,7 @@ def test_stage_model_catches_a_planted_fault(oracle_mod):
         _first_diff(bad, res, 8, 8, "planted")
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("p", [216091, 1257787, 24036583])
 @pytest.mark.parametrize("path", [0, 2])
 def test_stage_out_of_order_waits_for_nothing(m2, p, path):
